@@ -757,6 +757,11 @@ size_t woq_b200_workspace_bytes(const woq_b200_ctx* c, int64_t m) {
   n_tok = (n_tok + 15) / 16 * 16;
   if (n_tok < 16) n_tok = 16;
   size_t tc = woq::tc_partial_bytes(c->num_sms, n_tok);
+  if (m > 16) {
+    // (a workspace made for m tokens serves any smaller call as well)
+    n_tok = m > 256 ? 256 : static_cast<int>((m + 31) / 32 * 32);
+    tc = woq::pair_partial_bytes(c->num_sms, n_tok);
+  }
   return kWsHeaderBytes + (decode > tc ? decode : tc);
 }
 
@@ -855,6 +860,60 @@ static int make_kmajor_map(CUtensorMap* map, const void* base, int64_t rows, int
   return WOQ_B200_OK;
 }
 
+// More than 16 tokens: one launch on CTA pairs, whatever the token count.
+// The activations as [K / 64][rows][64] with 128-byte swizzle: one box is `kbs` k-blocks of `box_rows` rows.
+static int make_kblock_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_rows,
+                           int kbs) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return fail(WOQ_B200_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+  cuuint64_t dims[3] = {64, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(cols / 64)};
+  cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld) * 2, 128};
+  cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(kbs)};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(WOQ_B200_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
+  return WOQ_B200_OK;
+}
+
+static int run_pair(const woq_b200_ctx* c, const void* x, int64_t m, int64_t ldx, int32_t fusion, const void* o0,
+                    const void* o1, const int32_t* row_idx, const void* row_w, void* y, int64_t ldy, uint8_t* w8,
+                    cudaStream_t stream) {
+  woq::PairParams p{};
+  p.wq = c->wq_tc;
+  p.sz = c->sz_tc;
+  p.bias = c->bias;
+  p.y = static_cast<__nv_bfloat16*>(y);
+  p.other0 = static_cast<const __nv_bfloat16*>(o0);
+  p.other1 = static_cast<const __nv_bfloat16*>(o1);
+  p.row_idx = row_idx;
+  p.row_w = static_cast<const __nv_bfloat16*>(row_w);
+  p.status = reinterpret_cast<int*>(w8);
+  p.counters = reinterpret_cast<uint32_t*>(w8 + 256);
+  p.partials = reinterpret_cast<float*>(w8 + kWsHeaderBytes);
+  p.ldy = ldy;
+  p.m = (int)m;
+  p.n = (int)c->desc.n;
+  p.n_out = fusion == WOQ_B200_FUSE_SILU_MUL ? (int)(c->desc.n / 2) : (int)c->desc.n;
+  woq::pair_token_tiles(m, &p.n_tok, &p.tok_tiles);
+  p.tiles = c->tiles_tc;
+  p.w_tiles = (c->tiles_tc + 1) / 2;
+  p.kb_per_tile = c->kb_per_tile;
+  p.kbpg_shift = c->kbpg_shift;
+  p.groups = c->groups;
+  p.fusion = fusion;
+  p.gate_up = c->gate_up;
+  p.vec = ldy % 8 == 0 && aligned16(y) && (!o0 || aligned16(o0)) && (!o1 || aligned16(o1));
+  p.in_place = c->plain_scales;
+  if (woq::pair_plan(p) == 0) return fail(WOQ_B200_ERR_UNSUPPORTED, "no pipeline shape for %d token columns", p.n_tok);
+  CUtensorMap xmap;
+  if (int rc = make_kblock_map(&xmap, x, m, c->desc.k, ldx, p.n_tok / 2, p.kbs)) return rc;
+  CUDA_TRY(woq::launch_int4_pair(p, xmap, c->num_sms, stream));
+  woq::count_launch();
+  return WOQ_B200_OK;
+}
+
 static int run_tc(const woq_b200_ctx* c, const void* x, int64_t m, int64_t ldx, int32_t fusion,
                   const void* o0, const void* o1, const int32_t* row_idx, const void* row_w,
                   void* y, int64_t ldy, void* ws, size_t ws_bytes, cudaStream_t stream) {
@@ -864,6 +923,8 @@ static int run_tc(const woq_b200_ctx* c, const void* x, int64_t m, int64_t ldx, 
   if (c->tiles_tc > kMaxCounterTiles)
     return fail(WOQ_B200_ERR_UNSUPPORTED, "N too large for the workspace header");
   if (int rc = settle_prepack_flag(c)) return rc;
+  if (m > 16)
+    return run_pair(c, x, m, ldx, fusion, o0, o1, row_idx, row_w, y, ldy, static_cast<uint8_t*>(ws), stream);
   CUtensorMap xmap;
   const int64_t mt = m < 256 ? m : 256;
   int n_tok = static_cast<int>((mt + 15) / 16 * 16);

@@ -1,5 +1,6 @@
-// INT4 weight-only-quantised GEMM on the 5th-generation tensor cores (tcgen05 + TMEM), for
-// any token count up to 256 per launch.
+// INT4 weight-only-quantised GEMM on the 5th-generation tensor cores (tcgen05 + TMEM), one CTA per
+// tile.  Calls of more than 16 tokens run on CTA pairs (woq_pair_tc.cu); this kernel serves contexts
+// that ask for the tensor cores, or hold only the tensor-core tiling, at 16 tokens and fewer.
 //
 // Orientation: the weight is the A operand (128 output rows = the 128 TMEM lanes), the
 // activations are the B operand (N = tokens, 16..256), so one CTA tile is y^T[128 rows x

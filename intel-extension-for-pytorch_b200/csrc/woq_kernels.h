@@ -132,6 +132,35 @@ size_t tc_partial_bytes(int grid, int n_tok);
 size_t tc_plan(TcParams& p);  // fills a_col0, kbs, stages, w_ring from n_tok; returns the dynamic shared memory (0: none)
 cudaError_t launch_int4_tc(TcParams p, const CUtensorMap& xmap, int grid, cudaStream_t stream);
 
+// ---- tensor-core path on CTA pairs (more than 16 tokens) ---------------------------------
+struct PairParams {
+  const uint8_t* wq;   // row layout, as TcParams
+  const uint32_t* sz;
+  const float* bias;
+  __nv_bfloat16* y;
+  const __nv_bfloat16* other0;
+  const __nv_bfloat16* other1;
+  const int32_t* row_idx;
+  const __nv_bfloat16* row_w;
+  float* partials;     // [CTAs][2][n_tok][128]
+  uint32_t* counters;  // [CTAs], zero between calls
+  int* status;
+  int64_t ldy;
+  int m, n, n_out;
+  int n_tok, tok_tiles;         // token columns of a tile (a multiple of 32, <= 256); tiles of tokens
+  int tiles, w_tiles;           // 128-row tiles; pairs of them (rounded up)
+  int kb_per_tile, kbpg_shift, groups;
+  int kbs, stages, w_ring;      // k-blocks per stage; slots of the two rings
+  int unit;                     // shares are multiples of this many k-blocks
+  int fusion, gate_up;
+  int in_place;  // every scale normal and below 0.5, every zero point below 16
+  int vec;  // y and the extra operands can be accessed 16 bytes at a time
+};
+void pair_token_tiles(int64_t m, int* n_tok, int* tok_tiles);
+size_t pair_plan(PairParams& p);  // fills kbs, stages, w_ring, unit; dynamic shared memory (0: none)
+size_t pair_partial_bytes(int num_sms, int n_tok);
+cudaError_t launch_int4_pair(PairParams p, const CUtensorMap& xmap, int num_sms, cudaStream_t stream);
+
 __host__ __device__ inline int tc_tile_row_to_n(int n_total, int gate_up, int tile, int row) {
   if (gate_up) return row < 64 ? tile * 64 + row : n_total / 2 + tile * 64 + (row - 64);
   return tile * kTcTileN + row;

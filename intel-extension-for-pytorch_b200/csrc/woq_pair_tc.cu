@@ -1,0 +1,655 @@
+// Weight-only-quantised GEMM on CTA pairs (tcgen05 cta_group::2 + TMEM) for more than 16 tokens.
+//
+// A pair of CTAs on neighbouring SMs owns 256 output rows x up to 256 tokens: each CTA dequantises
+// its own 128 weight rows into its tensor memory (the A operand), each loads half of the
+// activation tile into its shared memory (the B operand), and the leader's MMAs (M = 256) read both
+// halves.  Against one CTA per tile that halves the activation bytes an SM takes from L2 and writes
+// to shared memory per FLOP: 20 KB per 128 rows x 256 tokens x 64 k instead of 36 KB.
+//
+//   warp 0      producer: bulk copies of packed weights + group scales of this CTA's rows
+//   warp 1      producer: TMA loads of this CTA's half of the activation tile; both CTAs' loads
+//               complete on the leader's barrier
+//   warp 2      (leader) issues the MMAs, one commit per stage frees the stage in both CTAs
+//   warp 3      tensor-memory allocation
+//   warps 4-11  epilogue: accumulators -> bias -> bf16 tile in shared memory -> fused post-op -> y.
+//               The accumulators are free again once the bf16 tile is written; the copy to global
+//               memory runs beside the next tile's MMAs.
+//   warps 12-27 dequantise: thread = output row, one k-block of a stage per warpgroup
+//
+// Work split: the sequence of (256-row tile, token tile, k-block), token tiles innermost but
+// for k, is cut into equal contiguous shares, one per pair ("stream-K").  A tile that several
+// pairs share is summed in k order: whoever arrives last adds the others' fp32 partial tiles from
+// the workspace (the pair that holds the beginning of the tile reaches it at the end of its own
+// share, when the others are normally done, and then adds its accumulators straight from TMEM).
+// Nobody waits for an arrival, and the order of the sum does not depend on timing.
+//
+// What bounds it: at 256 token columns the tensor cores under the power limit (57344 x 8192, 512
+// tokens: 339 us, 1420 TFLOP/s, against 501 us for one CTA per tile and 256 tokens per launch); at 32
+// columns the dequantiser's issue slots and the hand-overs between roles (91 us, 2.7 TB/s of weights,
+// was 125 us).  A lone thread beside sixteen dequantising warps gets an instruction issued every ten
+// cycles or so, so the roles' work per stage is what has to be small: one activation copy per stage,
+// several k-blocks per stage, no wait or fence that is not needed.
+#include "woq_kernels.h"
+#include "woq_pair_common.cuh"
+
+namespace woq {
+
+namespace {
+
+constexpr int kRoleWarps = 4, kEpiWarps = 8, kDeqGroups = 4;
+constexpr int kDeqWarp0 = kRoleWarps + kEpiWarps;
+constexpr int kPairThreads = (kDeqWarp0 + 4 * kDeqGroups) * 32;
+constexpr int kEpiThreads = kEpiWarps * 32;
+constexpr int kPairTmemCols = 512;
+constexpr int kMaxXRing = 8, kMaxPairWRing = 24;
+constexpr int kPairHeaderBytes = 1024;
+constexpr int kOutPitch = kTcTileN * 2 + 16;  // bytes of one token's row of the bf16 tile (+16: bank spread)
+constexpr int kEpiBar = 1;
+
+struct PairHeader {
+  uint64_t w_full[kMaxPairWRing];  // packed weights + scales of the slot have landed
+  uint64_t w_free[kMaxPairWRing];  // the dequantising warps have read the slot
+  uint64_t full[kMaxXRing];        // leader: the A halves of both CTAs written, both x halves landed
+  uint64_t free_[kMaxXRing];       // the stage's MMAs have completed
+  uint64_t d_full, d_empty;        // accumulators complete / (leader) read by all epilogue warps of the pair
+  uint32_t tmem_base;
+  int abort_flag;
+  int decision;
+};
+static_assert(sizeof(PairHeader) <= kPairHeaderBytes, "header too large");
+
+__device__ __forceinline__ int pair_owner_of(int64_t b, int64_t total, int64_t pairs) {
+  return static_cast<int>(((b + 1) * pairs - 1) / total);
+}
+
+__device__ __forceinline__ float bf_lo(uint32_t v) { return __uint_as_float(v << 16); }
+__device__ __forceinline__ float bf_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
+__device__ __forceinline__ uint32_t bf_pack(float lo, float hi) {
+  uint32_t r;
+  asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+  return r;
+}
+__device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    f[2 * i] = bf_lo(w[i]);
+    f[2 * i + 1] = bf_hi(w[i]);
+  }
+}
+
+// Eight neighbouring columns from column n of row `o` (element offset) that may be unaligned or run
+// past the limit.
+__device__ __forceinline__ uint4 load8(const __nv_bfloat16* p, size_t o, int valid, bool vec) {
+  if (vec && valid >= 8) return *reinterpret_cast<const uint4*>(p + o);
+  const unsigned short* s = reinterpret_cast<const unsigned short*>(p) + o;
+  uint32_t w[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    w[i] = 0u;
+    if (2 * i < valid) w[i] = s[2 * i];
+    if (2 * i + 1 < valid) w[i] |= static_cast<uint32_t>(s[2 * i + 1]) << 16;
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+__device__ __forceinline__ void store8(__nv_bfloat16* p, size_t o, const float (&f)[8], int valid, bool vec) {
+  const uint4 v = make_uint4(bf_pack(f[0], f[1]), bf_pack(f[2], f[3]), bf_pack(f[4], f[5]), bf_pack(f[6], f[7]));
+  if (vec && valid >= 8) {
+    *reinterpret_cast<uint4*>(p + o) = v;
+    return;
+  }
+  unsigned short* s = reinterpret_cast<unsigned short*>(p) + o;
+  const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    if (i < valid) s[i] = static_cast<unsigned short>(w[i >> 1] >> (16 * (i & 1)));
+}
+
+// The finished bf16 tile S[token][128 rows] -> fused post-op -> y, by the epilogue warps.  A thread
+// takes eight neighbouring columns of a token at a time, two such pieces together, so that the
+// operand loads of both are in flight before the first is used.
+__device__ __forceinline__ void pair_copy_out(const PairParams& p, const uint8_t* S, int tile, int tok0, int mv, int tid) {
+  constexpr int kBatch = 2;
+  const bool silu_mul = p.fusion == FUSE_SILU_MUL;
+  const int sh = silu_mul ? 3 : 4;  // pieces per token: 8 or 16
+  const int items = mv << sh;
+  const bool vec = p.vec != 0;
+  const int fusion = p.fusion;
+  for (int base = tid; base < items; base += kBatch * kEpiThreads) {
+    uint4 f0[kBatch], f1[kBatch];
+    size_t off[kBatch];
+    int valid[kBatch];
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      const int idx = base + u * kEpiThreads;
+      valid[u] = 0;
+      if (idx >= items) continue;
+      const int tok = idx >> sh, c = idx & ((1 << sh) - 1);
+      int n0, limit;
+      if (silu_mul) {
+        n0 = tile * 64 + c * 8;
+        limit = p.n_out;
+      } else if (p.gate_up) {
+        n0 = (c < 8 ? 0 : p.n / 2 - 64) + tile * 64 + c * 8;
+        limit = c < 8 ? p.n / 2 : p.n;
+      } else {
+        n0 = tile * kTcTileN + c * 8;
+        limit = p.n;
+      }
+      valid[u] = limit - n0 < 8 ? limit - n0 : 8;
+      const int64_t row = fusion == FUSE_SCALED_SCATTER_ADD ? p.row_idx[tok0 + tok] : tok0 + tok;
+      off[u] = static_cast<size_t>(row) * p.ldy + n0;
+      if (valid[u] > 0) {
+        if (fusion == FUSE_ADD || fusion == FUSE_ADD_ADD || fusion == FUSE_MUL) f0[u] = load8(p.other0, off[u], valid[u], vec);
+        if (fusion == FUSE_ADD_ADD) f1[u] = load8(p.other1, off[u], valid[u], vec);
+        if (fusion == FUSE_SCALED_SCATTER_ADD) f0[u] = load8(p.y, off[u], valid[u], vec);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kBatch; ++u) {
+      if (valid[u] <= 0) continue;
+      const int idx = base + u * kEpiThreads;
+      const int tok = idx >> sh, c = idx & ((1 << sh) - 1);
+      const uint8_t* src = S + tok * kOutPitch + c * 16;
+      float r[8];
+      unpack8(*reinterpret_cast<const uint4*>(src), r);
+      if (silu_mul) {
+        float up[8];
+        unpack8(*reinterpret_cast<const uint4*>(src + 128), up);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) r[e] = up[e] * silu_bf16(r[e]);
+      } else if (fusion == FUSE_ADD || fusion == FUSE_ADD_ADD) {
+        float a[8];
+        unpack8(f0[u], a);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) r[e] += a[e];
+        if (fusion == FUSE_ADD_ADD) {
+          unpack8(f1[u], a);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) r[e] = bf16_round(r[e]) + a[e];
+        }
+      } else if (fusion == FUSE_MUL) {
+        float a[8];
+        unpack8(f0[u], a);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) r[e] *= a[e];
+      } else if (fusion == FUSE_SCALED_SCATTER_ADD) {
+        float a[8];
+        unpack8(f0[u], a);
+        const float w = __bfloat162float(p.row_w[tok0 + tok]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) r[e] = a[e] + r[e] * w;
+      } else if (fusion != FUSE_NONE) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) r[e] = unary_post_op(r[e], fusion);
+      }
+      store8(p.y, off[u], r, valid[u], vec);
+    }
+  }
+}
+
+// IN_PLACE: every scale is normal and below 0.5 and every zero point below 16, so nibbles at bits 4..7
+// of a half-word can be used where they are: masked, the half-word read as bf16 is 16 q 2^-133 exactly
+// (the encoding is linear below 2^-125); subtract 16 zp 2^-133, multiply by scale * 2^129.  13 instead
+// of 15 instructions per eight weights, bit for bit the same results.
+template <bool IN_PLACE>
+__device__ __forceinline__ void pair_dequant(const uint4& v0, const uint4& v1, uint32_t szw, uint32_t (&r)[32]) {
+  const uint32_t z0 = __byte_perm(szw, 0, 0x1010), s0 = __byte_perm(szw, 0, 0x3232);
+  const uint32_t z1 = IN_PLACE ? (szw & 0xfu) * 0x00100010u : z0;
+  const uint32_t s1 = IN_PLACE ? s0 + 0x40804080u : s0;
+  const uint32_t words[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const uint32_t w = words[j], u = w >> 8;
+    r[j * 4] = bf16x2_mul(bf16x2_sub(lop3_and_or(w, 0x000f000fu, kBf16Magic), z0), s0);
+    r[j * 4 + 2] = bf16x2_mul(bf16x2_sub(lop3_and_or(u, 0x000f000fu, kBf16Magic), z0), s0);
+    if (IN_PLACE) {
+      r[j * 4 + 1] = bf16x2_mul(bf16x2_sub(w & 0x00f000f0u, z1), s1);
+      r[j * 4 + 3] = bf16x2_mul(bf16x2_sub(u & 0x00f000f0u, z1), s1);
+    } else {
+      r[j * 4 + 1] = bf16x2_mul(bf16x2_sub(lop3_and_or(w >> 4, 0x000f000fu, kBf16Magic), z0), s0);
+      r[j * 4 + 3] = bf16x2_mul(bf16x2_sub(lop3_and_or(u >> 4, 0x000f000fu, kBf16Magic), z0), s0);
+    }
+  }
+}
+
+template <bool IN_PLACE>
+__global__ void __launch_bounds__(kPairThreads, 1)
+    woq_int4_pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtensorMap xmap) {
+  extern __shared__ __align__(1024) uint8_t smem[];
+  PairHeader* hdr = reinterpret_cast<PairHeader*>(smem);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (smem_u32(smem) & 1023u) {  // swizzled tiles need a 1024-byte aligned base (the same in both CTAs)
+    if (tid == 0) atomicCAS(p.status, 0, 99);
+    return;
+  }
+  const int half_tok = p.n_tok >> 1;
+  const int x_blk = half_tok * 128;
+  const int x_stage_bytes = p.kbs * x_blk;
+  const int w_stage_bytes = p.kbs * (kTcBlockBytes + 512);
+  uint8_t* x_stages = smem + kPairHeaderBytes;
+  uint8_t* w_stages = x_stages + static_cast<size_t>(p.stages) * x_stage_bytes;
+  uint8_t* out_tile = w_stages + static_cast<size_t>(p.w_ring) * w_stage_bytes;
+
+  const uint32_t rank = pair_cta_rank();
+  const int pair = blockIdx.x >> 1;
+  const int64_t pairs = gridDim.x >> 1;
+  const int kbpt = p.kb_per_tile, kbs = p.kbs, n_stages = p.stages, n_wring = p.w_ring;
+  // shares are dealt in units of p.unit k-blocks
+  const int64_t units = static_cast<int64_t>(p.w_tiles) * p.tok_tiles * kbpt / p.unit;
+  const int64_t b_begin = pair * units / pairs * p.unit, b_end = (pair + 1) * units / pairs * p.unit;
+  const int item0 = static_cast<int>(b_begin / kbpt);       // item = weight tile * tok_tiles + token tile
+  const int kb00 = static_cast<int>(b_begin % kbpt);
+  const int rem0 = static_cast<int>(b_end - b_begin);
+
+  if (tid == 0) {
+    for (int s = 0; s < n_stages; ++s) {
+      mbar_init(&hdr->full[s], 8 * kbs + 1);  // four warps per k-block and CTA, the leader's x producer
+      mbar_init(&hdr->free_[s], 1);
+    }
+    for (int s = 0; s < n_wring; ++s) {
+      mbar_init(&hdr->w_full[s], 1);
+      mbar_init(&hdr->w_free[s], 4 * kbs);
+    }
+    mbar_init(&hdr->d_full, 1);
+    mbar_init(&hdr->d_empty, 2 * kEpiWarps);
+    hdr->abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 3) {
+    pair_tmem_alloc(&hdr->tmem_base, kPairTmemCols);
+    pair_tmem_relinquish();
+    tc_fence_before_sync();
+  }
+  __syncthreads();
+  pair_sync();
+  tc_fence_after_sync();
+  grid_launch_dependents();
+  const uint32_t tmem_base = hdr->tmem_base;
+  volatile int* abort_flag = &hdr->abort_flag;
+
+  if (warp == 0) {
+    // ---- packed weights and their group scales (never written by an earlier launch) ----
+    if (lane == 0) {
+      int item = item0, kb0 = kb00, rem = rem0, wslot = 0;
+      uint32_t wphase = 0;
+      while (rem > 0) {
+        int tile = item / p.tok_tiles * 2 + static_cast<int>(rank);
+        if (tile >= p.tiles) tile = p.tiles - 1;  // odd tile count: the last pair's second half repeats it
+        const uint8_t* wsrc = p.wq + (static_cast<size_t>(tile) * kbpt + kb0) * kTcBlockBytes;
+        const uint32_t* ssrc = p.sz + static_cast<size_t>(tile) * p.groups * kTcTileN;
+        int seg = kbpt - kb0 < rem ? kbpt - kb0 : rem;
+        rem -= seg;
+        while (seg > 0) {
+          const int nkb = seg < kbs ? seg : kbs;
+          uint8_t* ws = w_stages + static_cast<size_t>(wslot) * w_stage_bytes;
+          const int g0 = kb0 >> p.kbpg_shift;
+          const int ng = ((kb0 + nkb - 1) >> p.kbpg_shift) - g0 + 1;
+          mbar_wait(&hdr->w_free[wslot], wphase ^ 1, abort_flag, p.status, 31);
+          mbar_arrive_expect_tx(&hdr->w_full[wslot], nkb * kTcBlockBytes + ng * 512);
+          bulk_g2s(ws, wsrc, nkb * kTcBlockBytes, &hdr->w_full[wslot]);
+          bulk_g2s(ws + kbs * kTcBlockBytes, ssrc + static_cast<size_t>(g0) * kTcTileN, ng * 512, &hdr->w_full[wslot]);
+          wsrc += nkb * kTcBlockBytes;
+          kb0 += nkb;
+          seg -= nkb;
+          if (++wslot == n_wring) {
+            wslot = 0;
+            wphase ^= 1;
+          }
+        }
+        if (kb0 == kbpt) {
+          kb0 = 0;
+          ++item;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ---- this CTA's half of the activation tile, one copy per stage (a stage cut short by the end of
+    // ---- the share still loads whole: its last k-blocks are not used) ----
+    if (lane == 0) {
+      grid_dependency_wait();
+      int item = item0, kb0 = kb00, rem = rem0, slot = 0;
+      uint32_t phase = 0;
+      const uint32_t full0 = pair_map(&hdr->full[0], 0);
+      while (rem > 0) {
+        const int row = item % p.tok_tiles * p.n_tok + static_cast<int>(rank) * half_tok;
+        int seg = kbpt - kb0 < rem ? kbpt - kb0 : rem;
+        rem -= seg;
+        for (; seg > 0; seg -= kbs) {
+          mbar_wait(&hdr->free_[slot], phase ^ 1, abort_flag, p.status, 32);
+          if (rank == 0) mbar_arrive_expect_tx(&hdr->full[slot], 2 * x_stage_bytes);
+          pair_tma_load_3d(x_stages + slot * x_stage_bytes, &xmap, 0, row, kb0, full0 + slot * 8);
+          kb0 += kbs;
+          if (++slot == n_stages) {
+            slot = 0;
+            phase ^= 1;
+          }
+        }
+        kb0 = 0;
+        ++item;
+      }
+    }
+  } else if (warp == 2) {
+    if (rank == 0) {
+      // ---- the whole warp walks the stages, one elected lane issues ----
+      const uint32_t idesc = pair_idesc(p.n_tok, /*bf16*/ 1, /*bf16*/ 1, /*f32*/ 1);
+      const uint64_t desc0 = umma_desc_k128(smem_u32(x_stages));
+      const uint32_t a_base = tmem_base + p.n_tok;
+      const uint32_t x_blk16 = static_cast<uint32_t>(x_blk >> 4);
+      int kb0 = kb00, rem = rem0, slot = 0;
+      uint32_t phase = 0, seg_no = 0;
+      while (rem > 0) {
+        int seg = kbpt - kb0 < rem ? kbpt - kb0 : rem;
+        rem -= seg;
+        kb0 = 0;
+        uint32_t accumulate = 0;
+        mbar_wait(&hdr->d_empty, (seg_no & 1) ^ 1, abort_flag, p.status, 33);
+        for (; seg > 0; seg -= kbs) {
+          mbar_wait(&hdr->full[slot], phase, abort_flag, p.status, 34);
+          tc_fence_after_sync();
+          if (elect_one()) {
+            const int nkb = seg < kbs ? seg : kbs;
+            uint32_t a = a_base + slot * (kbs * 32);
+            uint64_t b = desc0 + static_cast<uint32_t>(slot * kbs) * x_blk16;
+            for (int j = 0; j < nkb; ++j) {
+#pragma unroll
+              for (int ks = 0; ks < 4; ++ks) {
+                pair_mma_f16_ts(tmem_base, a + ks * 8, b + ks * 2, idesc, accumulate);
+                accumulate = 1;
+              }
+              a += 32;
+              b += x_blk16;
+            }
+            pair_commit(&hdr->free_[slot]);
+            if (seg <= kbs) pair_commit(&hdr->d_full);
+          }
+          __syncwarp();
+          accumulate = 1;
+          if (++slot == n_stages) {
+            slot = 0;
+            phase ^= 1;
+          }
+        }
+        ++seg_no;
+      }
+    }
+  } else if (warp >= kDeqWarp0) {
+    // ---- dequantise: one k-block of a stage per warpgroup.  Stages of four k-blocks involve all four
+    // ---- warpgroups, stages of two alternate between two halves of them. ----
+    const int wg = (warp - kDeqWarp0) >> 2, q = warp & 3;
+    const int row = q * 32 + lane;
+    const int step = kDeqGroups / kbs;  // 1 or 2
+    const int j = wg & (kbs - 1);       // k-block within the stage
+    const uint32_t a_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + p.n_tok + j * 32;
+    const uint32_t full0 = pair_map(&hdr->full[0], 0);
+    int kb_seg = kb00, rem = rem0;
+    int own = wg / kbs, slot = own, wslot = own;  // `own`: this warpgroup's next stage, counted over all segments
+    int st = 0;
+    uint32_t phase = 0, wphase = 0;
+    while (rem > 0) {
+      const int seg_len = kbpt - kb_seg < rem ? kbpt - kb_seg : rem;
+      const int ns = (seg_len + kbs - 1) / kbs;
+      for (; own < st + ns; own += step) {
+        const int in_seg = (own - st) * kbs;   // k-blocks of the segment before this stage
+        const int kb0 = kb_seg + in_seg;
+        const bool some = in_seg + j < seg_len;  // false: the stage was cut short before this k-block
+        const uint8_t* ws = w_stages + wslot * w_stage_bytes;
+        mbar_wait(&hdr->w_full[wslot], wphase, abort_flag, p.status, 35);
+        uint32_t r[32];
+        if (some) {
+          const uint4* wp = reinterpret_cast<const uint4*>(ws + j * kTcBlockBytes);
+          const uint4 v0 = wp[row], v1 = wp[kTcTileN + row];
+          const int gl = ((kb0 + j) >> p.kbpg_shift) - (kb0 >> p.kbpg_shift);
+          const uint32_t szw = reinterpret_cast<const uint32_t*>(ws + kbs * kTcBlockBytes)[gl * kTcTileN + row];
+          pair_dequant<IN_PLACE>(v0, v1, szw, r);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&hdr->w_free[wslot]);
+        mbar_wait(&hdr->free_[slot], phase ^ 1, abort_flag, p.status, 36);
+        tc_fence_after_sync();
+        __syncwarp();  // the TMEM store is a warp-wide instruction
+        if (some) {
+          tmem_st_x32(a_lane + slot * (kbs * 32), r);
+          tc_wait_st();
+        }
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) pair_arrive(full0 + slot * 8);
+        slot += step;
+        if (slot >= n_stages) {
+          slot -= n_stages;
+          phase ^= 1;
+        }
+        wslot += step;
+        if (wslot >= n_wring) {
+          wslot -= n_wring;
+          wphase ^= 1;
+        }
+      }
+      st += ns;
+      rem -= seg_len;
+      kb_seg = 0;
+    }
+  } else if (warp >= kRoleWarps) {
+    // ---- epilogue: two warpgroups, 16 tokens at a time in turn ----
+    const int q = warp & 3, eg = (warp - kRoleWarps) >> 2, et = tid - kRoleWarps * 32;
+    const int row = q * 32 + lane;
+    const uint32_t d_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+    const uint32_t d_empty0 = pair_map(&hdr->d_empty, 0);
+    grid_dependency_wait();  // y, the fused operands and the workspace belong to this grid now
+    int item = item0, kb0 = kb00, rem = rem0;
+    uint32_t seg_no = 0;
+    auto to_tile = [&](int c0, const float (&v)[16], float bias) {  // 16 tokens of this row, as bf16
+      uint8_t* dst = out_tile + c0 * kOutPitch + row * 2;
+#pragma unroll
+      for (int e = 0; e < 16; ++e) *reinterpret_cast<__nv_bfloat16*>(dst + e * kOutPitch) = __float2bfloat16_rn(v[e] + bias);
+    };
+    auto accumulators_read = [&]() {
+      tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) pair_arrive(d_empty0);
+    };
+    while (rem > 0) {
+      const int seg_len = kbpt - kb0 < rem ? kbpt - kb0 : rem;
+      const bool whole = seg_len == kbpt;
+      const int tile = item / p.tok_tiles * 2 + static_cast<int>(rank);
+      const int tok0 = item % p.tok_tiles * p.n_tok;
+      const int mv = p.m - tok0 < p.n_tok ? p.m - tok0 : p.n_tok;
+      const bool real = tile < p.tiles;
+      float bias = 0.f;
+      if (p.bias && real) {
+        const int n = tc_tile_row_to_n(p.n, p.gate_up, tile, row);
+        if (n < p.n) bias = p.bias[n];
+      }
+      // the bf16 tile of the previous segment has been copied out by everybody
+      named_bar_sync(kEpiBar, kEpiThreads);
+      mbar_wait(&hdr->d_full, seg_no & 1, abort_flag, p.status, 37);
+      tc_fence_after_sync();
+      __syncwarp();
+      bool finish = whole && real;
+      if (whole || !real) {
+        if (real)
+          for (int c0 = eg * 16; c0 < mv; c0 += 32) {
+            uint32_t t[16];
+            tmem_ld_x16(d_lane + c0, t);
+            tc_wait_ld();
+            float v[16];
+#pragma unroll
+            for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(t[e]);
+            to_tile(c0, v, bias);
+          }
+        accumulators_read();
+      } else {
+        // part of a tile
+        const int64_t tb0 = static_cast<int64_t>(item) * kbpt / p.unit;  // the tile's first unit
+        const int c_first = pair_owner_of(tb0, units, pairs), c_last = pair_owner_of(tb0 + kbpt / p.unit - 1, units, pairs);
+        const unsigned others = static_cast<unsigned>(c_last - c_first);
+        uint32_t* counter = p.counters + c_first * 2 + rank;
+        auto slot_of = [&](int c) {  // partial tile of pair c, this CTA's rows
+          const int s = (c == c_first && c * units / pairs < tb0) ? 1 : 0;
+          return p.partials + static_cast<size_t>((c * 2 + static_cast<int>(rank)) * 2 + s) * p.n_tok * kTcTileN + row;
+        };
+        bool from_tmem = false;
+        if (kb0 == 0) {
+          // the beginning of the tile, the last segment of this pair: have all others arrived?
+          if (et == 0) {
+            uint32_t seen;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
+            if (seen == others) *counter = 0;
+            hdr->decision = seen == others;
+          }
+          named_bar_sync(kEpiBar, kEpiThreads);
+          from_tmem = hdr->decision != 0;
+          finish = from_tmem;
+        }
+        if (!from_tmem) {
+          float* dst = slot_of(pair);
+          for (int c0 = eg * 16; c0 < mv; c0 += 32) {
+            uint32_t t[16];
+            tmem_ld_x16(d_lane + c0, t);
+            tc_wait_ld();
+#pragma unroll
+            for (int e = 0; e < 16; ++e)
+              if (c0 + e < mv) __stcg(dst + static_cast<size_t>(c0 + e) * kTcTileN, __uint_as_float(t[e]));
+          }
+          accumulators_read();
+          __threadfence();
+          named_bar_sync(kEpiBar, kEpiThreads);
+          if (et == 0) {
+            const unsigned old = atomicAdd(counter, 1u);
+            if (old == others) *counter = 0;
+            hdr->decision = old == others;
+          }
+          named_bar_sync(kEpiBar, kEpiThreads);
+          finish = hdr->decision != 0;
+        }
+        if (finish) {
+          __threadfence();
+          for (int c0 = eg * 16; c0 < mv; c0 += 32) {
+            float v[16];
+            int c = c_first;
+            if (from_tmem) {
+              uint32_t t[16];
+              tmem_ld_x16(d_lane + c0, t);
+              tc_wait_ld();
+#pragma unroll
+              for (int e = 0; e < 16; ++e) v[e] = __uint_as_float(t[e]);
+              ++c;
+            } else {
+#pragma unroll
+              for (int e = 0; e < 16; ++e) v[e] = 0.f;
+            }
+            for (; c <= c_last; ++c) {
+              const float* src = slot_of(c) + static_cast<size_t>(c0) * kTcTileN;
+              float t[16];
+#pragma unroll
+              for (int e = 0; e < 16; ++e) t[e] = c0 + e < mv ? __ldcg(src + e * kTcTileN) : 0.f;
+#pragma unroll
+              for (int e = 0; e < 16; ++e) v[e] += t[e];
+            }
+            to_tile(c0, v, bias);
+          }
+          if (from_tmem) accumulators_read();
+        }
+      }
+      named_bar_sync(kEpiBar, kEpiThreads);
+      if (finish) pair_copy_out(p, out_tile, tile, tok0, mv, et);
+      rem -= seg_len;
+      kb0 = 0;
+      ++item;
+      ++seg_no;
+    }
+  }
+
+  __syncwarp();
+  tc_fence_before_sync();
+  __syncthreads();
+  pair_sync();
+  if (warp == 3) {
+    tc_fence_after_sync();
+    pair_tmem_dealloc(tmem_base, kPairTmemCols);
+  }
+}
+
+}  // namespace
+
+// Token tiles of a call: as few as 256 columns allow, then as narrow as they can be (a multiple of 32,
+// which is what a pair's MMA takes), so that 300 tokens are two tiles of 160, not of 256.
+void pair_token_tiles(int64_t m, int* n_tok, int* tok_tiles) {
+  const int t = static_cast<int>((m + 255) / 256);
+  *tok_tiles = t < 1 ? 1 : t;
+  *n_tok = static_cast<int>(((m + *tok_tiles - 1) / *tok_tiles + 31) / 32 * 32);
+  if (*n_tok < 32) *n_tok = 32;
+}
+
+// Pipeline shape for p.n_tok token columns; returns the dynamic shared memory in bytes.
+//   k-blocks per stage: four up to 128 columns, two above.  Every stage costs each single-thread role
+//     300-400 cycles of waiting, issuing and bookkeeping beside the busy dequantising warps, whatever
+//     the stage holds; a k-block's MMAs take 2 x n_tok cycles.
+//   Rings: a parity wait cannot tell a barrier that is one completion short from one that is three
+//     short, so whoever waits for use u of a slot must know that use u - 1 has completed.  With stages
+//     of four k-blocks every warpgroup waits for every use of every slot.  With stages of two a
+//     warpgroup sees every second stage: an even weight ring gives each slot to one pair of
+//     warpgroups, and on the A / activation ring the wait for stage s - 2 (the MMAs of stage
+//     s - 2 - stages, which complete in order) covers stage s - 2 * stages.
+size_t pair_plan(PairParams& p) {
+  const int budget = 227 * 1024 - kPairHeaderBytes - p.n_tok * kOutPitch;
+  p.kbs = p.n_tok <= 128 ? 4 : 2;
+  const int x_stage = p.kbs * (p.n_tok / 2) * 128;
+  const int w_stage = p.kbs * (kTcBlockBytes + 512);
+  int stages = (kPairTmemCols - p.n_tok) / 32 / p.kbs;
+  if (stages > kMaxXRing) stages = kMaxXRing;
+  while (stages > 2 && budget - stages * x_stage < 3 * w_stage) --stages;
+  int ring = (budget - stages * x_stage) / w_stage;
+  if (ring > kMaxPairWRing) ring = kMaxPairWRing;
+  if (p.kbs == 2) ring &= ~1;
+  if (stages < 2 || ring < 2) return 0;
+  p.stages = stages;
+  p.w_ring = ring;
+  // shares in whole stages where they are long enough for the rounding not to matter
+  const int64_t total = static_cast<int64_t>(p.w_tiles) * p.tok_tiles * p.kb_per_tile;
+  p.unit = p.kb_per_tile % p.kbs == 0 && total >= static_cast<int64_t>(74) * 8 * p.kbs ? p.kbs : 1;
+  return kPairHeaderBytes + static_cast<size_t>(stages) * x_stage + static_cast<size_t>(ring) * w_stage +
+         static_cast<size_t>(p.n_tok) * kOutPitch;
+}
+
+// Pairs of a launch: all SMs, or one per k-block when there are fewer.
+int pair_grid(const PairParams& p, int num_sms) {
+  const int64_t total = static_cast<int64_t>(p.w_tiles) * p.tok_tiles * p.kb_per_tile;
+  int64_t pairs = num_sms / 2;
+  if (pairs > total) pairs = total;
+  return static_cast<int>(pairs < 1 ? 1 : pairs) * 2;
+}
+
+size_t pair_partial_bytes(int num_sms, int n_tok) {
+  return static_cast<size_t>(num_sms) * 2 * n_tok * kTcTileN * sizeof(float);
+}
+
+cudaError_t launch_int4_pair(PairParams p, const CUtensorMap& xmap, int num_sms, cudaStream_t stream) {
+  const size_t smem = pair_plan(p);
+  if (smem == 0) return cudaErrorInvalidConfiguration;
+  void (*kern)(const PairParams, const CUtensorMap) = p.in_place ? woq_int4_pair_kernel<true> : woq_int4_pair_kernel<false>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       static_cast<int>(smem));
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(pair_grid(p, num_sms));
+  cfg.blockDim = dim3(kPairThreads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (dependent_launch_enabled()) {
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 2;
+  }
+  return cudaLaunchKernelEx(&cfg, kern, p, xmap);
+}
+
+}  // namespace woq
