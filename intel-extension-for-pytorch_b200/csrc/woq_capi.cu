@@ -78,7 +78,7 @@ struct woq_b200_ctx {
   float* scale_f32;  // INT8: per-channel fp32 scales [n_pad]
   int32_t* comp;     // INT8 with asymmetric activations: per-row sums of the weight codes [n_pad]
   int is_int8;       // INT8 weights with INT8 compute
-  int plain_scales;  // INT4: every scale is normal and below 0.5, every zero point below 16
+  int plain_scales;  // every scale (and INT4 zero point) is in the in-place range of the dequantiser
   int kc_per_tile;   // INT8: K / 128
   float* bias;       // fp32 [n] or null
   size_t wq_bytes, sz_bytes;
@@ -88,7 +88,8 @@ struct woq_b200_ctx {
   // that needs it, so that loading many layers does not synchronise once per layer.
   // general route (woq_generic.cu): plain weight bytes, fp32 scales / zero points [n][groups]
   int is_generic;
-  uint8_t* g_w;
+  uint8_t* g_w;  // null once the weight is kept in the row layout of the CTA-pair kernel (`rows`)
+  int rows;      // INT8 / NF4: weight in wq_tc, scale words in sz_tc (tiles_tc, kb_per_tile, kbpg_shift, groups)
   float* g_scales;
   float* g_zps;
   int g_row_bytes, g_group, g_groups;
@@ -297,7 +298,7 @@ I8BlockWs i8block_ws(const woq_b200_ctx* c, int64_t m) {
 }
 
 int create_generic(const woq_b200_desc* d, const void* qweight, const void* scales, const void* zero_points,
-                   const void* bias, cudaStream_t stream, woq_b200_ctx** out);
+                   const void* bias, cudaStream_t stream, woq_b200_ctx** out, bool allow_rows);
 
 int create_i8block(const woq_b200_desc* d, const void* qweight, const void* scales, const void* zero_points,
                    const void* bias, cudaStream_t stream, woq_b200_ctx** out) {
@@ -315,7 +316,7 @@ int create_i8block(const woq_b200_desc* d, const void* qweight, const void* scal
   g.lowp_mode = WOQ_B200_LOWP_BF16;
   g.layout_flags |= WOQ_B200_LAYOUT_GENERIC;
   woq_b200_ctx* c = nullptr;
-  if (int rc = create_generic(&g, qweight, scales, zero_points, bias, stream, &c)) return rc;
+  if (int rc = create_generic(&g, qweight, scales, zero_points, bias, stream, &c, /*allow_rows=*/false)) return rc;
   c->desc = *d;
   c->is_generic = 0;
   c->is_i8block = 1;
@@ -397,8 +398,62 @@ int run_i8block(const woq_b200_ctx* c, const void* x, int64_t m, int64_t ldx, in
   return WOQ_B200_OK;
 }
 
+// INT8 / NF4 weights that the CTA-pair kernel can take (64-aligned K, power-of-two groups of 64 or more, zero
+// points that are INT8 codes) move to its row layout; the general kernel reads that layout too, so there is
+// one copy of the weight.  A layer that does not qualify keeps the plain layout.
+cudaError_t move_to_rows(woq_b200_ctx* c, cudaStream_t stream) {
+  const woq_b200_desc& d = c->desc;
+  const bool int8 = d.weight_dtype == WOQ_B200_DTYPE_INT8;
+  if (!int8 && d.weight_dtype != WOQ_B200_DTYPE_NF4) return cudaSuccess;
+  if (d.lowp_mode == WOQ_B200_LOWP_FP16 || d.k % 64 != 0) return cudaSuccess;
+  const int64_t g = c->g_group;
+  if (g < d.k && (g % 64 != 0 || (g & (g - 1)) != 0)) return cudaSuccess;
+  c->tiles_tc = static_cast<int>((d.n + 127) / 128);
+  c->kb_per_tile = static_cast<int>(d.k / 64);
+  c->groups = c->g_groups;
+  c->kbpg_shift = 30;
+  if (g < d.k)
+    for (c->kbpg_shift = 0; (64ll << c->kbpg_shift) < g;) ++c->kbpg_shift;
+  const size_t w_bytes = static_cast<size_t>(c->tiles_tc) * c->kb_per_tile *
+                         woq::pair_block_bytes(int8 ? woq::kWeightInt8 : woq::kWeightNf4);
+  const size_t s_bytes = static_cast<size_t>(c->tiles_tc) * c->groups * 128 * 4;
+  int* flag = nullptr;
+  int bits = 1;
+  cudaError_t e = cudaMalloc(&c->sz_tc, s_bytes);
+  if (e == cudaSuccess) e = cudaMalloc(&flag, sizeof(int));
+  if (e == cudaSuccess) e = cudaMemsetAsync(flag, 0, sizeof(int), stream);
+  if (e == cudaSuccess)
+    e = woq::launch_pack_row_scales(c->g_scales, c->g_zps, c->sz_tc, (int)d.n, c->groups, flag, stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&bits, flag, sizeof(int), cudaMemcpyDeviceToHost, stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+  if (e == cudaSuccess && !(bits & 1)) {
+    woq::count_launch();
+    e = cudaMalloc(&c->wq_tc, w_bytes);
+    if (e == cudaSuccess) e = woq::launch_pack_rows(c->g_w, c->wq_tc, (int)d.n, (int)d.k, int8, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    if (e == cudaSuccess) {
+      woq::count_launch();
+      cudaFree(c->g_w);
+      c->g_w = nullptr;
+      c->wq_bytes = 0;
+      c->wq_tc_bytes = w_bytes;
+      c->sz_tc_bytes = s_bytes;
+      c->plain_scales = (bits & 2) ? 0 : 1;
+      c->rows = 1;
+    }
+  }
+  if (flag) cudaFree(flag);
+  if (!c->rows) {
+    cudaFree(c->sz_tc);
+    cudaFree(c->wq_tc);
+    c->sz_tc = nullptr;
+    c->wq_tc = nullptr;
+  }
+  return e;
+}
+
 int create_generic(const woq_b200_desc* d, const void* qweight, const void* scales, const void* zero_points,
-                   const void* bias, cudaStream_t stream, woq_b200_ctx** out) {
+                   const void* bias, cudaStream_t stream, woq_b200_ctx** out, bool allow_rows) {
   if (d->lowp_mode == WOQ_B200_LOWP_INT8)
     return fail(WOQ_B200_ERR_UNSUPPORTED, "the general route computes in fp32 / fp16 / bf16, not INT8");
   if (d->weight_format != WOQ_B200_FMT_PLAIN)
@@ -458,6 +513,7 @@ int create_generic(const woq_b200_desc* d, const void* qweight, const void* scal
   }
   CUDA_TRY_G(cudaGetLastError());
   CUDA_TRY_G(cudaStreamSynchronize(stream));
+  if (allow_rows) CUDA_TRY_G(move_to_rows(c, stream));
 #undef CUDA_TRY_G
   c->magic = kMagic;
   *out = c;
@@ -472,7 +528,8 @@ int generic_compute_dtype(const woq_b200_ctx* c, int io_dtype) {
 }
 
 void fill_generic(const woq_b200_ctx* c, woq::GenericParams* p) {
-  p->w = c->g_w;
+  p->w = c->rows ? c->wq_tc : c->g_w;
+  p->kb_per_tile = c->rows ? c->kb_per_tile : 0;
   p->scales = c->g_scales;
   p->zps = c->g_zps;
   p->bias = c->bias;
@@ -533,7 +590,7 @@ int woq_b200_ctx_create(const woq_b200_desc* d, const void* qweight, const void*
     return fail(WOQ_B200_ERR_INVALID_ARG, "scales must be fp32, fp16 or bf16");
 
   if (wants_i8block(d)) return create_i8block(d, qweight, scales, zero_points, bias, stream, out);
-  if (wants_generic(d)) return create_generic(d, qweight, scales, zero_points, bias, stream, out);
+  if (wants_generic(d)) return create_generic(d, qweight, scales, zero_points, bias, stream, out, /*allow_rows=*/true);
   if (d->weight_dtype == WOQ_B200_DTYPE_INT8) return create_int8(d, qweight, scales, zero_points, bias, stream, out);
   // ---- INT4 ----
   if (d->k % 64 != 0)
@@ -730,6 +787,12 @@ int woq_b200_ctx_unpack(const woq_b200_ctx* c, void* qweight_plain, void* stream
   if (int rc = check_ctx(c)) return rc;
   if (!qweight_plain) return fail(WOQ_B200_ERR_INVALID_ARG, "output is null");
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (c->rows) {
+    CUDA_TRY(woq::launch_unpack_rows(c->wq_tc, static_cast<uint8_t*>(qweight_plain), (int)c->desc.n, (int)c->desc.k,
+                                     c->desc.weight_dtype == WOQ_B200_DTYPE_INT8, stream));
+    woq::count_launch();
+    return WOQ_B200_OK;
+  }
   if (c->is_generic || c->is_i8block) {
     CUDA_TRY(cudaMemcpyAsync(qweight_plain, c->g_w, c->wq_bytes, cudaMemcpyDeviceToDevice, stream));
     return WOQ_B200_OK;
@@ -748,7 +811,8 @@ int woq_b200_ctx_unpack(const woq_b200_ctx* c, void* qweight_plain, void* stream
 
 size_t woq_b200_workspace_bytes(const woq_b200_ctx* c, int64_t m) {
   if (check_ctx(c)) return 0;
-  if (c->is_generic) return kWsHeaderBytes;  // the general route needs no scratch
+  if (c->is_generic)  // the general kernel needs no scratch
+    return kWsHeaderBytes + (c->rows ? woq::pair_partial_bytes(c->num_sms, m < 1 ? 1 : m < 256 ? (int)m : 256) : 0);
   if (c->is_i8block) return i8block_ws(c, m < 1 ? 1 : m).total;
   if (c->is_int8) return int8_ws_layout(c, m < 1 ? 1 : m).total;
   // header + one pair of partial tiles per CTA of the largest grid
@@ -860,7 +924,6 @@ static int make_kmajor_map(CUtensorMap* map, const void* base, int64_t rows, int
   return WOQ_B200_OK;
 }
 
-// More than 16 tokens: one launch on CTA pairs, whatever the token count.
 // The activations as [K / 64][rows][64] with 128-byte swizzle: one box is `kbs` k-blocks of `box_rows` rows.
 static int make_kblock_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_rows,
                            int kbs) {
@@ -877,6 +940,7 @@ static int make_kblock_map(CUtensorMap* map, const void* base, int64_t rows, int
   return WOQ_B200_OK;
 }
 
+// One launch on CTA pairs, whatever the token count.
 static int run_pair(const woq_b200_ctx* c, const void* x, int64_t m, int64_t ldx, int32_t fusion, const void* o0,
                     const void* o1, const int32_t* row_idx, const void* row_w, void* y, int64_t ldy, uint8_t* w8,
                     cudaStream_t stream) {
@@ -905,11 +969,17 @@ static int run_pair(const woq_b200_ctx* c, const void* x, int64_t m, int64_t ldx
   p.fusion = fusion;
   p.gate_up = c->gate_up;
   p.vec = ldy % 8 == 0 && aligned16(y) && (!o0 || aligned16(o0)) && (!o1 || aligned16(o1));
-  p.in_place = c->plain_scales;
+  p.part_tok = m < p.n_tok ? (int)m : p.n_tok;
+  if (c->desc.weight_dtype == WOQ_B200_DTYPE_INT8)
+    p.kind = c->plain_scales ? woq::kWeightInt8InPlace : woq::kWeightInt8;
+  else if (c->desc.weight_dtype == WOQ_B200_DTYPE_NF4)
+    p.kind = woq::kWeightNf4;
+  else
+    p.kind = c->plain_scales ? woq::kWeightInt4InPlace : woq::kWeightInt4;
   if (woq::pair_plan(p) == 0) return fail(WOQ_B200_ERR_UNSUPPORTED, "no pipeline shape for %d token columns", p.n_tok);
   CUtensorMap xmap;
   if (int rc = make_kblock_map(&xmap, x, m, c->desc.k, ldx, p.n_tok / 2, p.kbs)) return rc;
-  CUDA_TRY(woq::launch_int4_pair(p, xmap, c->num_sms, stream));
+  CUDA_TRY(woq::launch_pair(p, xmap, c->num_sms, stream));
   woq::count_launch();
   return WOQ_B200_OK;
 }
@@ -1075,6 +1145,14 @@ int woq_b200_linear_any(const woq_b200_ctx* c, const void* x, int32_t io_dtype, 
   }
   if (n_others != need || (need > 0 && (!others || !others[0])) || (need > 1 && !others[1]))
     return fail(WOQ_B200_ERR_INVALID_ARG, "fusion %#x takes %d extra tensors, got %d", fusion, need, n_others);
+  // bf16 activations and compute on a row-layout weight: the tensor-core kernel.  Calls that it cannot take
+  // (activation rows that a TMA copy cannot start at, a workspace of the size the general kernel needs) run
+  // on the general kernel.
+  if (c->rows && io_dtype == WOQ_B200_T_BF16 && generic_compute_dtype(c, io_dtype) == WOQ_B200_T_BF16 &&
+      m < (1ll << 31) && ldx % 8 == 0 && aligned16(x) && workspace &&
+      workspace_bytes >= woq_b200_workspace_bytes(c, m))
+    return run_pair(c, x, m, ldx, fusion, need > 0 ? others[0] : nullptr, need > 1 ? others[1] : nullptr, nullptr,
+                    nullptr, y, ldy, static_cast<uint8_t*>(workspace), static_cast<cudaStream_t>(stream_));
   woq::GenericParams p{};
   fill_generic(c, &p);
   p.x = x;
@@ -1099,8 +1177,6 @@ int woq_b200_linear_any(const woq_b200_ctx* c, const void* x, int32_t io_dtype, 
     CUDA_TRY(woq::launch_generic(q, static_cast<cudaStream_t>(stream_)));
     woq::count_launch();
   }
-  (void)workspace;
-  (void)workspace_bytes;
   return WOQ_B200_OK;
 }
 

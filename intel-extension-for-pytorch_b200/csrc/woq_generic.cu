@@ -5,7 +5,8 @@
 //
 // It is the route for what the tuned kernels do not take (they cover INT4 with bf16 compute on
 // 64-aligned shapes and INT8 with INT8 compute): a functional kernel on the CUDA cores, not a
-// tuned one.  A warp owns four output rows and walks the whole K for eight tokens at a time;
+// tuned one (INT8 and NF4 weights with bf16 activations and compute go to the CTA-pair kernel where their
+// shape allows it: woq_pair_tc.cu).  A warp owns four output rows and walks the whole K for eight tokens at a time;
 // a lane dequantises eight consecutive weights of each row per step,
 //     w = round_c((code - zp) * round_c(scale)),   round_c = rounding to the compute dtype,
 // multiplies them with the activations (rounded to the compute dtype) and accumulates in fp32;
@@ -24,24 +25,6 @@ constexpr int kRows = 4;    // output rows per warp
 constexpr int kTok = 8;     // tokens per pass
 constexpr int kWarps = 4;   // warps per CTA
 
-// NF4 code -> value (reference: csrc/cpu/aten/utils/woq_utils.h:34-51)
-__constant__ float kNf4[16] = {-1.0f,
-                               -0.6961928009986877f,
-                               -0.5250730514526367f,
-                               -0.39491748809814453f,
-                               -0.28444138169288635f,
-                               -0.18477343022823334f,
-                               -0.09105003625154495f,
-                               0.0f,
-                               0.07958029955625534f,
-                               0.16093020141124725f,
-                               0.24611230194568634f,
-                               0.33791524171829224f,
-                               0.44070982933044434f,
-                               0.5626170039176941f,
-                               0.7229568362236023f,
-                               1.0f};
-
 // FP8 e4m3 byte -> fp32, bit for bit the reference's conversion
 // (csrc/cpu/aten/utils/woq.h:465-483): exponent rebias by 120, three mantissa bits, zero when
 // the low seven bits are zero; no special case for NaN or subnormal codes.
@@ -49,6 +32,16 @@ __device__ __forceinline__ float fp8_e4m3_to_f32(uint32_t x) {
   if ((x & 127u) == 0u) return __uint_as_float((x & 128u) << 24);
   const uint32_t bits = ((x & 7u) << 20) | ((((x >> 3) & 15u) + 120u) << 23) | ((x & 128u) << 24);
   return __uint_as_float(bits);
+}
+
+// where code (row, kk) of a row-layout block lies: word of the block, bit of the code in its word
+__device__ __forceinline__ int row_layout_word(int int8, int row, int kk) {
+  const int i = kk / (int8 ? 4 : 8);
+  return ((i >> 2) * kTcTileN + row) * 4 + (i & 3);
+}
+__device__ __forceinline__ int row_layout_shift(int int8, int kk) {
+  if (int8) return (kk & 1) * 16 + ((kk >> 1) & 1) * 8;
+  return 4 * ((kk & 7) >> 1) + 16 * (kk & 1);
 }
 
 template <int C>
@@ -101,7 +94,21 @@ __device__ __forceinline__ float post_op_io(float y, const GenericParams& p, siz
 // the eight codes of one 8-k chunk of row `row` as floats (before zero point and scale)
 template <int WD>
 __device__ __forceinline__ void load_codes(const GenericParams& p, int row, int k0, float (&c)[8]) {
-  if (WD == WOQ_B200_DTYPE_INT4 || WD == WOQ_B200_DTYPE_NF4) {
+  if ((WD == WOQ_B200_DTYPE_NF4 || WD == WOQ_B200_DTYPE_INT8) && p.kb_per_tile > 0) {
+    const size_t blk = static_cast<size_t>(row / kTcTileN) * p.kb_per_tile + k0 / kBlockK;
+    const int r = row % kTcTileN, kk = k0 % kBlockK;
+    if (WD == WOQ_B200_DTYPE_NF4) {
+      const uint32_t word = *reinterpret_cast<const uint32_t*>(p.w + blk * kTcBlockBytes +
+                                                               row_layout_word(0, r, kk) * 4);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) c[i] = kNf4Table[(word >> (4 * (i >> 1) + 16 * (i & 1))) & 15u];
+    } else {
+      const uint2 v = *reinterpret_cast<const uint2*>(p.w + blk * 2 * kTcBlockBytes + row_layout_word(1, r, kk) * 4);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+        c[i] = static_cast<float>(static_cast<int>(((i < 4 ? v.x : v.y) >> row_layout_shift(1, i)) & 0xffu) - 128);
+    }
+  } else if (WD == WOQ_B200_DTYPE_INT4 || WD == WOQ_B200_DTYPE_NF4) {
     const uint8_t* src = p.w + static_cast<size_t>(row) * p.row_bytes + (k0 >> 1);
     uint32_t word;
     if ((p.row_bytes & 3) == 0 && k0 + 8 <= ((p.k + 1) & ~1)) {
@@ -114,7 +121,7 @@ __device__ __forceinline__ void load_codes(const GenericParams& p, int row, int 
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const uint32_t q = (word >> (4 * i)) & 15u;
-      c[i] = WD == WOQ_B200_DTYPE_NF4 ? kNf4[q] : static_cast<float>(q);
+      c[i] = WD == WOQ_B200_DTYPE_NF4 ? kNf4Table[q] : static_cast<float>(q);
     }
   } else {
     const uint8_t* src = p.w + static_cast<size_t>(row) * p.row_bytes + k0;
@@ -230,7 +237,101 @@ __global__ void dump_generic_kernel(const GenericParams p, float* out) {
   }
 }
 
+// ---- row layout of INT8 / NF4 weights: one thread per word ------------------------------------
+template <bool INT8>
+__global__ void pack_rows_kernel(const uint8_t* plain, uint32_t* rows, int n, int k, int64_t words) {
+  const int64_t wi = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (wi >= words) return;
+  constexpr int kWords = INT8 ? 2048 : 1024, kPer = INT8 ? 4 : 8;  // words of a block, codes of a word
+  const int64_t blk = wi / kWords;
+  const int in = static_cast<int>(wi % kWords), j = in & 3, row = (in >> 2) & 127, part = in >> 9;
+  const int kbpt = k / kBlockK;
+  const int64_t nn = blk / kbpt * kTcTileN + row;
+  const int k0 = static_cast<int>(blk % kbpt) * kBlockK + (part * 4 + j) * kPer;
+  uint32_t w = 0;
+  if (nn < n) {
+    if (INT8) {
+      const uint32_t v = *reinterpret_cast<const uint32_t*>(plain + nn * k + k0) ^ 0x80808080u;
+      w = __byte_perm(v, 0, 0x3120);
+    } else {
+      const uint32_t v = *reinterpret_cast<const uint32_t*>(plain + (nn * k + k0) / 2);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) w |= ((v >> (4 * i)) & 15u) << row_layout_shift(0, i);
+    }
+  }
+  rows[wi] = w;
+}
+
+template <bool INT8>
+__global__ void unpack_rows_kernel(const uint32_t* rows, uint8_t* plain, int n, int k, int64_t words) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;  // 32-bit word of the plain weight
+  if (i >= words) return;
+  constexpr int kPer = INT8 ? 4 : 8;
+  const int64_t per_row = k / kPer;
+  const int nn = static_cast<int>(i / per_row), k0 = static_cast<int>(i % per_row) * kPer;
+  const int64_t blk = static_cast<int64_t>(nn / kTcTileN) * (k / kBlockK) + k0 / kBlockK;
+  const uint32_t w = rows[blk * (INT8 ? 2048 : 1024) + row_layout_word(INT8, nn % kTcTileN, k0 % kBlockK)];
+  uint32_t v = 0;
+  if (INT8) {
+    v = __byte_perm(w, 0, 0x3120) ^ 0x80808080u;
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v |= ((w >> row_layout_shift(0, e)) & 15u) << (4 * e);
+  }
+  uint8_t* dst = plain + i * 4;  // the caller's buffer may be unaligned
+#pragma unroll
+  for (int b = 0; b < 4; ++b) dst[b] = static_cast<uint8_t>(v >> (8 * b));
+}
+
+__global__ void pack_row_scales_kernel(const float* scales, const float* zps, uint32_t* sz, int n, int groups,
+                                       int64_t words, int* flag) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= words) return;
+  const int row = static_cast<int>(i % kTcTileN), g = static_cast<int>(i / kTcTileN % groups);
+  const int64_t nn = i / (static_cast<int64_t>(kTcTileN) * groups) * kTcTileN + row;
+  float s = 0.f, z = 0.f;
+  if (nn < n) {
+    s = scales[nn * groups + g];
+    if (zps) z = zps[nn * groups + g];
+    if (!(z >= -128.f && z <= 127.f && z == rintf(z)) || !(fabsf(s) <= 0x1p100f)) {
+      atomicOr(flag, 1);
+      z = 0.f;
+    }
+  }
+  const uint32_t sb = __bfloat16_as_ushort(__float2bfloat16_rn(s)), sexp = (sb >> 7) & 0xffu;
+  if (nn < n && (sexp < 1u || sexp > 121u)) atomicOr(flag, 2);
+  sz[i] = (sb << 16) | static_cast<uint32_t>(static_cast<int>(z) + 128);
+}
+
 }  // namespace
+
+cudaError_t launch_pack_rows(const uint8_t* plain, uint8_t* rows, int n, int k, int int8, cudaStream_t stream) {
+  const int64_t words = ceil_div(n, kTcTileN) * (k / kBlockK) * (int8 ? 2048 : 1024);
+  const unsigned blocks = static_cast<unsigned>(ceil_div(words, 256));
+  if (int8)
+    pack_rows_kernel<true><<<blocks, 256, 0, stream>>>(plain, reinterpret_cast<uint32_t*>(rows), n, k, words);
+  else
+    pack_rows_kernel<false><<<blocks, 256, 0, stream>>>(plain, reinterpret_cast<uint32_t*>(rows), n, k, words);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_unpack_rows(const uint8_t* rows, uint8_t* plain, int n, int k, int int8, cudaStream_t stream) {
+  const int64_t words = static_cast<int64_t>(n) * k / (int8 ? 4 : 8);
+  const unsigned blocks = static_cast<unsigned>(ceil_div(words, 256));
+  if (int8)
+    unpack_rows_kernel<true><<<blocks, 256, 0, stream>>>(reinterpret_cast<const uint32_t*>(rows), plain, n, k, words);
+  else
+    unpack_rows_kernel<false><<<blocks, 256, 0, stream>>>(reinterpret_cast<const uint32_t*>(rows), plain, n, k, words);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_pack_row_scales(const float* scales, const float* zps, uint32_t* sz, int n, int groups, int* flag,
+                                   cudaStream_t stream) {
+  const int64_t words = ceil_div(n, kTcTileN) * groups * kTcTileN;
+  pack_row_scales_kernel<<<static_cast<unsigned>(ceil_div(words, 256)), 256, 0, stream>>>(scales, zps, sz, n, groups,
+                                                                                          words, flag);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_generic(const GenericParams& p, cudaStream_t stream) {
   const dim3 grid(static_cast<unsigned>(ceil_div(p.n, kWarps * kRows)), static_cast<unsigned>(ceil_div(p.m, kTok)));

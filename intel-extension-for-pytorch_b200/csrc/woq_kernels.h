@@ -132,7 +132,32 @@ size_t tc_partial_bytes(int grid, int n_tok);
 size_t tc_plan(TcParams& p);  // fills a_col0, kbs, stages, w_ring from n_tok; returns the dynamic shared memory (0: none)
 cudaError_t launch_int4_tc(TcParams p, const CUtensorMap& xmap, int grid, cudaStream_t stream);
 
-// ---- tensor-core path on CTA pairs (more than 16 tokens) ---------------------------------
+// ---- tensor-core path on CTA pairs (INT4: more than 16 tokens; INT8 / NF4 with bf16 compute: any) ----
+// Row layouts of a 128-row x 64-k block: INT4 as above; NF4 the same words (codes are table indices);
+// INT8 8192 bytes [quarter][row][16 B], codes biased by 128 (u8), a word holds k, k + 2, k + 1, k + 3
+// from its low byte up, so w & 0x00ff00ff and (w >> 8) & 0x00ff00ff are pairs of neighbouring k.
+// Scale words: INT4 {bf16 scale, bf16 128 + zp}; INT8 {bf16 scale, 128 + zp as an integer}; NF4 {bf16 scale, 0}.
+enum WeightKind { kWeightInt4InPlace = 0, kWeightInt4, kWeightInt8InPlace, kWeightInt8, kWeightNf4 };
+__host__ __device__ constexpr int pair_block_bytes(int kind) {
+  return kind == kWeightInt8InPlace || kind == kWeightInt8 ? 2 * kTcBlockBytes : kTcBlockBytes;
+}
+// NF4 code -> value (reference: csrc/cpu/aten/utils/woq_utils.h:34-51)
+__constant__ const float kNf4Table[16] = {-1.0f,
+                                          -0.6961928009986877f,
+                                          -0.5250730514526367f,
+                                          -0.39491748809814453f,
+                                          -0.28444138169288635f,
+                                          -0.18477343022823334f,
+                                          -0.09105003625154495f,
+                                          0.0f,
+                                          0.07958029955625534f,
+                                          0.16093020141124725f,
+                                          0.24611230194568634f,
+                                          0.33791524171829224f,
+                                          0.44070982933044434f,
+                                          0.5626170039176941f,
+                                          0.7229568362236023f,
+                                          1.0f};
 struct PairParams {
   const uint8_t* wq;   // row layout, as TcParams
   const uint32_t* sz;
@@ -142,7 +167,7 @@ struct PairParams {
   const __nv_bfloat16* other1;
   const int32_t* row_idx;
   const __nv_bfloat16* row_w;
-  float* partials;     // [CTAs][2][n_tok][128]
+  float* partials;     // [CTAs][2][part_tok][128]
   uint32_t* counters;  // [CTAs], zero between calls
   int* status;
   int64_t ldy;
@@ -153,13 +178,14 @@ struct PairParams {
   int kbs, stages, w_ring;      // k-blocks per stage; slots of the two rings
   int unit;                     // shares are multiples of this many k-blocks
   int fusion, gate_up;
-  int in_place;  // every scale normal and below 0.5, every zero point below 16
+  int kind;      // WeightKind
+  int part_tok;  // tokens of a partial tile: min(m, n_tok)
   int vec;  // y and the extra operands can be accessed 16 bytes at a time
 };
 void pair_token_tiles(int64_t m, int* n_tok, int* tok_tiles);
 size_t pair_plan(PairParams& p);  // fills kbs, stages, w_ring, unit; dynamic shared memory (0: none)
-size_t pair_partial_bytes(int num_sms, int n_tok);
-cudaError_t launch_int4_pair(PairParams p, const CUtensorMap& xmap, int num_sms, cudaStream_t stream);
+size_t pair_partial_bytes(int num_sms, int part_tok);
+cudaError_t launch_pair(PairParams p, const CUtensorMap& xmap, int num_sms, cudaStream_t stream);
 
 __host__ __device__ inline int tc_tile_row_to_n(int n_total, int gate_up, int tile, int row) {
   if (gate_up) return row < 64 ? tile * 64 + row : n_total / 2 + tile * 64 + (row - 64);
@@ -230,7 +256,7 @@ cudaError_t launch_i8_block(const I8BlockParams& p, cudaStream_t stream);
 
 // ---- general route: any weight dtype, fp32 / fp16 / bf16 compute, plain layout -----------
 struct GenericParams {
-  const uint8_t* w;     // plain [n][row_bytes]: nibbles (even k low) or bytes
+  const uint8_t* w;     // plain [n][row_bytes]: nibbles (even k low) or bytes; kb_per_tile > 0: row layout
   const float* scales;  // [n][groups] fp32 as given (rounded to the compute dtype in the kernel)
   const float* zps;     // [n][groups] or null (then default_zp)
   const float* bias;    // [n] or null
@@ -240,11 +266,19 @@ struct GenericParams {
   const void* other1;
   int64_t ldx, ldy;
   int m, n, k, group, groups, row_bytes;
+  int kb_per_tile;      // K / 64 when w is in the row layout of INT8 / NF4 (see WeightKind), else 0
   int weight_dtype, compute_dtype, io_dtype, fusion;  // WOQ_B200_DTYPE_* / WOQ_B200_T_*
   float default_zp;
 };
 cudaError_t launch_generic(const GenericParams& p, cudaStream_t stream);
 cudaError_t launch_dump_generic(const GenericParams& p, float* out, cudaStream_t stream);
+// Row layout of plain INT8 (`int8`) or NF4 weights and of their scales, and the weights back.  `flag`
+// (zeroed): bit 0 a zero point is not an integer in -128..127 or a scale not finite or above 2^100 (the
+// layout cannot be used), bit 1 a scale is outside the in-place range.
+cudaError_t launch_pack_rows(const uint8_t* plain, uint8_t* rows, int n, int k, int int8, cudaStream_t stream);
+cudaError_t launch_unpack_rows(const uint8_t* rows, uint8_t* plain, int n, int k, int int8, cudaStream_t stream);
+cudaError_t launch_pack_row_scales(const float* scales, const float* zps, uint32_t* sz, int n, int groups, int* flag,
+                                   cudaStream_t stream);
 
 // ---- pack / unpack / dump ------------------------------------------------------------
 struct PackInt4Args {

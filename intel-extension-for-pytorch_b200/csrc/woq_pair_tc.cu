@@ -29,6 +29,9 @@
 // was 125 us).  A lone thread beside sixteen dequantising warps gets an instruction issued every ten
 // cycles or so, so the roles' work per stage is what has to be small: one activation copy per stage,
 // several k-blocks per stage, no wait or fence that is not needed.
+//
+// Weights: INT4, INT8 and NF4 in the row layout of their kind (WeightKind); only the dequantiser and
+// the bytes of a k-block differ.
 #include "woq_kernels.h"
 #include "woq_pair_common.cuh"
 
@@ -56,6 +59,7 @@ struct PairHeader {
   int abort_flag;
   int decision;
 };
+constexpr int kNf4LutBytes = 16 * 32 * 4;  // the NF4 table, one copy per lane (no bank conflicts)
 static_assert(sizeof(PairHeader) <= kPairHeaderBytes, "header too large");
 
 __device__ __forceinline__ int pair_owner_of(int64_t b, int64_t total, int64_t pairs) {
@@ -188,12 +192,18 @@ __device__ __forceinline__ void pair_copy_out(const PairParams& p, const uint8_t
   }
 }
 
-// IN_PLACE: every scale is normal and below 0.5 and every zero point below 16, so nibbles at bits 4..7
+// A k-block's 64 weights of one row -> 32 bf16x2 registers (k order).  `ws` + 16 * row is the row's first
+// 16 bytes, the next ones are kTcTileN * 16 further on.  All variants give bf16((code - zp) * bf16(scale)),
+// rounded once, bit for bit the general kernel's values.
+//
+// INT4 in place: every scale is normal and below 0.5 and every zero point below 16, so nibbles at bits 4..7
 // of a half-word can be used where they are: masked, the half-word read as bf16 is 16 q 2^-133 exactly
 // (the encoding is linear below 2^-125); subtract 16 zp 2^-133, multiply by scale * 2^129.  13 instead
-// of 15 instructions per eight weights, bit for bit the same results.
+// of 15 instructions per eight weights.
 template <bool IN_PLACE>
-__device__ __forceinline__ void pair_dequant(const uint4& v0, const uint4& v1, uint32_t szw, uint32_t (&r)[32]) {
+__device__ __forceinline__ void pair_dequant_int4(const uint8_t* ws, int row, uint32_t szw, uint32_t (&r)[32]) {
+  const uint4* wp = reinterpret_cast<const uint4*>(ws) + row;
+  const uint4 v0 = wp[0], v1 = wp[kTcTileN];
   const uint32_t z0 = __byte_perm(szw, 0, 0x1010), s0 = __byte_perm(szw, 0, 0x3232);
   const uint32_t z1 = IN_PLACE ? (szw & 0xfu) * 0x00100010u : z0;
   const uint32_t s1 = IN_PLACE ? s0 + 0x40804080u : s0;
@@ -213,9 +223,64 @@ __device__ __forceinline__ void pair_dequant(const uint4& v0, const uint4& v1, u
   }
 }
 
+// INT8: codes biased by 128; a byte in a half-word read as bf16 is q 2^-133 exactly (0..255: the subnormals
+// and the first binade), so the difference to the zero point's byte is exact too and one multiplication by
+// scale * 2^133 finishes (IN_PLACE: every scale normal and below 2^-5); otherwise 2^120 first, exact, then
+// scale * 2^13 with the same single rounding.
 template <bool IN_PLACE>
+__device__ __forceinline__ void pair_dequant_int8(const uint8_t* ws, int row, uint32_t szw, uint32_t (&r)[32]) {
+  const uint4* wp = reinterpret_cast<const uint4*>(ws) + row;
+  const uint32_t z = (szw & 0xffu) * 0x00010001u, s = __byte_perm(szw, 0, 0x3232);
+  const uint32_t s1 = IN_PLACE ? s + 0x42804280u : bf16x2_mul(s, 0x46004600u);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const uint4 v = wp[q * kTcTileN];
+    const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t lo = bf16x2_sub(words[j] & 0x00ff00ffu, z), hi = bf16x2_sub(__byte_perm(words[j], 0, 0x4341), z);
+      r[q * 8 + j * 2] = bf16x2_mul(IN_PLACE ? lo : bf16x2_mul(lo, 0x7b807b80u), s1);
+      r[q * 8 + j * 2 + 1] = bf16x2_mul(IN_PLACE ? hi : bf16x2_mul(hi, 0x7b807b80u), s1);
+    }
+  }
+}
+
+// NF4: fp32 table values (24 bits) times the bf16 scale, rounded to fp32 and then to bf16 as the general
+// kernel does, so a table of bf16 values would not do.  One conflict-free shared load per weight: lane l
+// reads its own copy at 128 * code + 4 l.
+__device__ __forceinline__ void pair_dequant_nf4(const uint8_t* ws, int row, uint32_t szw, const uint8_t* lut_lane,
+                                                 uint32_t (&r)[32]) {
+  const uint4* wp = reinterpret_cast<const uint4*>(ws) + row;
+  const float s = __uint_as_float(szw & 0xffff0000u);
+  auto value = [&](uint32_t code128) { return *reinterpret_cast<const float*>(lut_lane + (code128 & 0x780u)) * s; };
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const uint4 v = wp[h * kTcTileN];
+    const uint32_t words[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t w = words[j];
+      r[h * 16 + j * 4] = bf_pack(value(w << 7), value(w >> 9));
+      r[h * 16 + j * 4 + 1] = bf_pack(value(w << 3), value(w >> 13));
+      r[h * 16 + j * 4 + 2] = bf_pack(value(w >> 1), value(w >> 17));
+      r[h * 16 + j * 4 + 3] = bf_pack(value(w >> 5), value(w >> 21));
+    }
+  }
+}
+
+template <int KIND>
+__device__ __forceinline__ void pair_dequant(const uint8_t* ws, int row, uint32_t szw, const uint8_t* lut_lane,
+                                             uint32_t (&r)[32]) {
+  if (KIND == kWeightInt4InPlace) pair_dequant_int4<true>(ws, row, szw, r);
+  if (KIND == kWeightInt4) pair_dequant_int4<false>(ws, row, szw, r);
+  if (KIND == kWeightInt8InPlace) pair_dequant_int8<true>(ws, row, szw, r);
+  if (KIND == kWeightInt8) pair_dequant_int8<false>(ws, row, szw, r);
+  if (KIND == kWeightNf4) pair_dequant_nf4(ws, row, szw, lut_lane, r);
+}
+
+template <int KIND>
 __global__ void __launch_bounds__(kPairThreads, 1)
-    woq_int4_pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtensorMap xmap) {
+    woq_pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtensorMap xmap) {
   extern __shared__ __align__(1024) uint8_t smem[];
   PairHeader* hdr = reinterpret_cast<PairHeader*>(smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -226,10 +291,13 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   const int half_tok = p.n_tok >> 1;
   const int x_blk = half_tok * 128;
   const int x_stage_bytes = p.kbs * x_blk;
-  const int w_stage_bytes = p.kbs * (kTcBlockBytes + 512);
+  constexpr int kBlock = pair_block_bytes(KIND);
+  const int w_stage_bytes = p.kbs * (kBlock + 512);
   uint8_t* x_stages = smem + kPairHeaderBytes;
   uint8_t* w_stages = x_stages + static_cast<size_t>(p.stages) * x_stage_bytes;
   uint8_t* out_tile = w_stages + static_cast<size_t>(p.w_ring) * w_stage_bytes;
+  uint8_t* lut = out_tile + p.n_tok * kOutPitch;  // NF4 only
+  if (KIND == kWeightNf4 && tid < 512) reinterpret_cast<float*>(lut)[tid] = kNf4Table[tid >> 5];
 
   const uint32_t rank = pair_cta_rank();
   const int pair = blockIdx.x >> 1;
@@ -276,7 +344,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       while (rem > 0) {
         int tile = item / p.tok_tiles * 2 + static_cast<int>(rank);
         if (tile >= p.tiles) tile = p.tiles - 1;  // odd tile count: the last pair's second half repeats it
-        const uint8_t* wsrc = p.wq + (static_cast<size_t>(tile) * kbpt + kb0) * kTcBlockBytes;
+        const uint8_t* wsrc = p.wq + (static_cast<size_t>(tile) * kbpt + kb0) * kBlock;
         const uint32_t* ssrc = p.sz + static_cast<size_t>(tile) * p.groups * kTcTileN;
         int seg = kbpt - kb0 < rem ? kbpt - kb0 : rem;
         rem -= seg;
@@ -286,10 +354,10 @@ __global__ void __launch_bounds__(kPairThreads, 1)
           const int g0 = kb0 >> p.kbpg_shift;
           const int ng = ((kb0 + nkb - 1) >> p.kbpg_shift) - g0 + 1;
           mbar_wait(&hdr->w_free[wslot], wphase ^ 1, abort_flag, p.status, 31);
-          mbar_arrive_expect_tx(&hdr->w_full[wslot], nkb * kTcBlockBytes + ng * 512);
-          bulk_g2s(ws, wsrc, nkb * kTcBlockBytes, &hdr->w_full[wslot]);
-          bulk_g2s(ws + kbs * kTcBlockBytes, ssrc + static_cast<size_t>(g0) * kTcTileN, ng * 512, &hdr->w_full[wslot]);
-          wsrc += nkb * kTcBlockBytes;
+          mbar_arrive_expect_tx(&hdr->w_full[wslot], nkb * kBlock + ng * 512);
+          bulk_g2s(ws, wsrc, nkb * kBlock, &hdr->w_full[wslot]);
+          bulk_g2s(ws + kbs * kBlock, ssrc + static_cast<size_t>(g0) * kTcTileN, ng * 512, &hdr->w_full[wslot]);
+          wsrc += nkb * kBlock;
           kb0 += nkb;
           seg -= nkb;
           if (++wslot == n_wring) {
@@ -397,11 +465,9 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         mbar_wait(&hdr->w_full[wslot], wphase, abort_flag, p.status, 35);
         uint32_t r[32];
         if (some) {
-          const uint4* wp = reinterpret_cast<const uint4*>(ws + j * kTcBlockBytes);
-          const uint4 v0 = wp[row], v1 = wp[kTcTileN + row];
           const int gl = ((kb0 + j) >> p.kbpg_shift) - (kb0 >> p.kbpg_shift);
-          const uint32_t szw = reinterpret_cast<const uint32_t*>(ws + kbs * kTcBlockBytes)[gl * kTcTileN + row];
-          pair_dequant<IN_PLACE>(v0, v1, szw, r);
+          const uint32_t szw = reinterpret_cast<const uint32_t*>(ws + kbs * kBlock)[gl * kTcTileN + row];
+          pair_dequant<KIND>(ws + j * kBlock, row, szw, lut + lane * 4, r);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(&hdr->w_free[wslot]);
@@ -487,7 +553,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         uint32_t* counter = p.counters + c_first * 2 + rank;
         auto slot_of = [&](int c) {  // partial tile of pair c, this CTA's rows
           const int s = (c == c_first && c * units / pairs < tb0) ? 1 : 0;
-          return p.partials + static_cast<size_t>((c * 2 + static_cast<int>(rank)) * 2 + s) * p.n_tok * kTcTileN + row;
+          return p.partials + static_cast<size_t>((c * 2 + static_cast<int>(rank)) * 2 + s) * p.part_tok * kTcTileN + row;
         };
         bool from_tmem = false;
         if (kb0 == 0) {
@@ -593,13 +659,16 @@ void pair_token_tiles(int64_t m, int* n_tok, int* tok_tiles) {
 //     warpgroups, and on the A / activation ring the wait for stage s - 2 (the MMAs of stage
 //     s - 2 - stages, which complete in order) covers stage s - 2 * stages.
 size_t pair_plan(PairParams& p) {
-  const int budget = 227 * 1024 - kPairHeaderBytes - p.n_tok * kOutPitch;
+  const int lut = p.kind == kWeightNf4 ? kNf4LutBytes : 0;
+  const int budget = 227 * 1024 - kPairHeaderBytes - lut - p.n_tok * kOutPitch;
   p.kbs = p.n_tok <= 128 ? 4 : 2;
   const int x_stage = p.kbs * (p.n_tok / 2) * 128;
-  const int w_stage = p.kbs * (kTcBlockBytes + 512);
+  const int w_stage = p.kbs * (pair_block_bytes(p.kind) + 512);
   int stages = (kPairTmemCols - p.n_tok) / 32 / p.kbs;
   if (stages > kMaxXRing) stages = kMaxXRing;
-  while (stages > 2 && budget - stages * x_stage < 3 * w_stage) --stages;
+  // (two slots of 17 KB are enough for the 8-bit weights of a 256-column tile: the A ring buffers as well)
+  const int min_ring = p.kbs == 2 && w_stage > 16 * 1024 ? 2 : 3;
+  while (stages > 2 && budget - stages * x_stage < min_ring * w_stage) --stages;
   int ring = (budget - stages * x_stage) / w_stage;
   if (ring > kMaxPairWRing) ring = kMaxPairWRing;
   if (p.kbs == 2) ring &= ~1;
@@ -610,7 +679,7 @@ size_t pair_plan(PairParams& p) {
   const int64_t total = static_cast<int64_t>(p.w_tiles) * p.tok_tiles * p.kb_per_tile;
   p.unit = p.kb_per_tile % p.kbs == 0 && total >= static_cast<int64_t>(74) * 8 * p.kbs ? p.kbs : 1;
   return kPairHeaderBytes + static_cast<size_t>(stages) * x_stage + static_cast<size_t>(ring) * w_stage +
-         static_cast<size_t>(p.n_tok) * kOutPitch;
+         static_cast<size_t>(p.n_tok) * kOutPitch + lut;
 }
 
 // Pairs of a launch: all SMs, or one per k-block when there are fewer.
@@ -621,14 +690,22 @@ int pair_grid(const PairParams& p, int num_sms) {
   return static_cast<int>(pairs < 1 ? 1 : pairs) * 2;
 }
 
-size_t pair_partial_bytes(int num_sms, int n_tok) {
-  return static_cast<size_t>(num_sms) * 2 * n_tok * kTcTileN * sizeof(float);
+size_t pair_partial_bytes(int num_sms, int part_tok) {
+  return static_cast<size_t>(num_sms) * 2 * part_tok * kTcTileN * sizeof(float);
 }
 
-cudaError_t launch_int4_pair(PairParams p, const CUtensorMap& xmap, int num_sms, cudaStream_t stream) {
+cudaError_t launch_pair(PairParams p, const CUtensorMap& xmap, int num_sms, cudaStream_t stream) {
   const size_t smem = pair_plan(p);
   if (smem == 0) return cudaErrorInvalidConfiguration;
-  void (*kern)(const PairParams, const CUtensorMap) = p.in_place ? woq_int4_pair_kernel<true> : woq_int4_pair_kernel<false>;
+  void (*kern)(const PairParams, const CUtensorMap) = nullptr;
+  switch (p.kind) {
+    case kWeightInt4InPlace: kern = woq_pair_kernel<kWeightInt4InPlace>; break;
+    case kWeightInt4: kern = woq_pair_kernel<kWeightInt4>; break;
+    case kWeightInt8InPlace: kern = woq_pair_kernel<kWeightInt8InPlace>; break;
+    case kWeightInt8: kern = woq_pair_kernel<kWeightInt8>; break;
+    case kWeightNf4: kern = woq_pair_kernel<kWeightNf4>; break;
+    default: return cudaErrorInvalidValue;
+  }
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem));
   if (e != cudaSuccess) return e;
