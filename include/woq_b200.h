@@ -344,6 +344,31 @@ int woq_b200_moe_expert(const woq_b200_ctx* w13, const woq_b200_ctx* w2, const v
                         const int32_t* token_idx, const void* token_weight, int64_t tokens, void* out,
                         int64_t ld_out, void* workspace, size_t workspace_bytes, void* stream);
 
+/* Several INT4 linears of one shape and group size in one launch, each on its own row range of x:
+ * y[g][i, :] = x[row0[g] + i, :] * W[g]^T + bias[g] for 0 <= i < rows[g].  ctxs, row0, rows and y are HOST
+ * arrays of `groups` entries; every context needs the tensor-core tiling and plain row order; rows[g] >= 1;
+ * total_rows is the number of rows of x.  Row ranges may repeat (gate and up of an expert).  Workspace:
+ * woq_b200_workspace_bytes(ctxs[0], max(17, most rows)).  No reference counterpart: mixtral_moe_woq runs one
+ * linear after another (csrc/cpu/aten/kernels/MoEKrnl.cpp:254-285). */
+int woq_b200_linear_grouped(const woq_b200_ctx* const* ctxs, const int64_t* row0, const int64_t* rows,
+                            void* const* y, int32_t groups, const void* x, int64_t total_rows, int64_t ldx,
+                            int64_t ldy, void* workspace, size_t workspace_bytes, void* stream);
+
+/* The other steps of a mixture-of-experts layer (csrc/cpu/aten/MoE.cpp:290-330).
+ * moe_route: ids [tokens, top_k] sorted stably by expert: counts[e] pairs for expert e and counts[experts]
+ *   nonzero when an id is outside 0 .. experts - 1; token_of[position], pos_of[pair].
+ * gather_rows: out[i, :] = x[idx[i], :], bf16 rows of k (a multiple of 8) elements.
+ * silu_mul: out = bf16(up * silu(gate)), rounded as WOQ_B200_FUSE_SILU_MUL does.
+ * moe_combine: out[t, :] = sum of rows[pos_of[t, s], :] * weights[t, s] in expert order, one bf16 rounding
+ *   per addition, as scattering expert after expert gives; at most 64 slots. */
+int woq_b200_moe_route(const int64_t* ids, int64_t tokens, int32_t top_k, int32_t experts, int32_t* counts,
+                       int32_t* token_of, int32_t* pos_of, void* stream);
+int woq_b200_gather_rows(const void* x, int64_t ldx, const int32_t* idx, int64_t rows, int64_t k, void* out,
+                         void* stream);
+int woq_b200_silu_mul(const void* gate, const void* up, void* out, int64_t count, void* stream);
+int woq_b200_moe_combine(const void* rows, const int64_t* ids, const int32_t* pos_of, const void* weights,
+                         int64_t tokens, int32_t top_k, int64_t hidden, void* out, void* stream);
+
 /* RMSNorm fused with the per-token activation quantiser of the INT8 path.  For every row of
  * x (bf16 [m, k], k a multiple of 16):
  *   y  = bf16(x * rsqrt(mean(x^2) + eps) * gamma)        fp32 arithmetic, one rounding; gamma bf16 [k]

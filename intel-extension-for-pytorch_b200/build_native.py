@@ -28,6 +28,7 @@ CUDA_SOURCES = [
     "woq_static_scratch.cu",
     "woq_generic.cu",
     "woq_int8_block.cu",
+    "woq_moe.cu",
 ]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -486,9 +486,29 @@ at::Tensor mixtral_moe_woq(const at::Tensor& hidden_states, const at::Tensor& to
   return output;
 }
 
+// Contexts the grouped mixture-of-experts launches take: INT4 weights with bf16 compute, channels in
+// checkpoint order, gate and up separate, one shape and group size for all experts.
+bool moe_grouped(const std::vector<c10::intrusive_ptr<WoqLinearOpContext>>& ctxs, int64_t n, int64_t k, int device) {
+  for (const auto& c : ctxs) {
+    if (!c || !c->ctx || c->device != device || c->perm.defined() || c->weight_shape[0] != n ||
+        c->weight_shape[1] != k || c->group_size != ctxs[0]->group_size || c->weight_dtype != WOQ_B200_DTYPE_INT4 ||
+        (c->layout_flags & WOQ_B200_LAYOUT_GATE_UP) || woq_b200_ctx_route(c->ctx) != WOQ_B200_ROUTE_INT4_BF16)
+      return false;
+  }
+  return true;
+}
+
 // reference: csrc/cpu/aten/MoE.cpp:290-330.  topk_ids [tokens, top_k] names each token's experts; every
-// selected expert runs the per-expert routine above on its tokens.  The (token, slot) pairs of all
-// experts come from one stable sort on the device and one copy of the per-expert counts to the host.
+// selected expert runs gate, up, silu * up and down on its tokens, and the results are added to the output
+// in expert order with their routing weights.
+//
+// The (token, slot) pairs are sorted by expert on the device; the per-expert counts come to the host, which
+// shapes the launches with them (and refuses ids that name no expert).  When an expert has more than 16
+// tokens, all gate and up projections are one launch and all down projections another: an expert's linear
+// alone is too small to fill the GPU for long (4096 x 14336, 64 tokens: 25 us by itself, 12 us of a grouped
+// launch).  Up to 16 tokens the streaming kernel runs expert by expert, so that a model that only decodes
+// keeps one copy of its weights.  Everything else (other weight types, act-order, ...) goes through the
+// per-expert operator above.
 at::Tensor deepseek_moe_woq(const at::Tensor& hidden_states, const at::Tensor& topk_ids,
                             const std::vector<c10::intrusive_ptr<WoqLinearOpContext>>& gate_ctx,
                             const std::vector<c10::intrusive_ptr<WoqLinearOpContext>>& up_ctx,
@@ -499,10 +519,89 @@ at::Tensor deepseek_moe_woq(const at::Tensor& hidden_states, const at::Tensor& t
               "WOQ: deepseek_moe_woq takes one gate, up and down context per expert");
   TORCH_CHECK(topk_ids.dim() == 2 && topk_ids.size(0) == hidden_states.size(0),
               "WOQ: topk_ids must be [tokens, top_k]");
-  at::Tensor output = at::zeros_like(hidden_states);
-  if (experts == 0 || topk_ids.numel() == 0) return output;
-  const int64_t top_k = topk_ids.size(1);
+  if (experts == 0 || topk_ids.numel() == 0) return at::zeros_like(hidden_states);
+  const int64_t top_k = topk_ids.size(1), tokens = topk_ids.size(0), pairs = tokens * top_k;
   at::Tensor flat = topk_ids.to(hidden_states.device()).reshape({-1}).to(at::kLong);
+
+  const int dev = hidden_states.is_cuda() ? hidden_states.get_device() : -1;
+  const bool plain = dev >= 0 && hidden_states.scalar_type() == at::kBFloat16 && hidden_states.dim() == 2 &&
+                     hidden_states.is_contiguous() && !(reinterpret_cast<uintptr_t>(hidden_states.data_ptr()) & 15);
+  const int64_t hidden = plain ? hidden_states.size(1) : 0, ffn = gate_ctx[0] ? gate_ctx[0]->weight_shape[0] : 0;
+  if (plain && !is_distributed && top_k <= 64 && experts <= 65535 && pairs < (1ll << 30) && ffn % 8 == 0 &&
+      routing_weights.dim() == 2 && routing_weights.size(0) == tokens && routing_weights.size(1) == top_k &&
+      moe_grouped(gate_ctx, ffn, hidden, dev) && moe_grouped(up_ctx, ffn, hidden, dev) &&
+      moe_grouped(down_ctx, hidden, ffn, dev) && gate_ctx[0]->group_size == up_ctx[0]->group_size) {
+    c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(dev));
+    cudaStream_t stream = at::cuda::getCurrentCUDAStream(dev).stream();
+    flat = flat.contiguous();
+    const auto ints = flat.options().dtype(at::kInt);
+    at::Tensor dcounts = at::empty({experts + 1}, ints), token_of = at::empty({pairs}, ints);
+    at::Tensor pos_of = at::empty({pairs}, ints);
+    WOQ_CHECK(woq_b200_moe_route(flat.data_ptr<int64_t>(), tokens, static_cast<int32_t>(top_k),
+                                 static_cast<int32_t>(experts), dcounts.data_ptr<int32_t>(),
+                                 token_of.data_ptr<int32_t>(), pos_of.data_ptr<int32_t>(), stream));
+    at::Tensor w = routing_weights.to(hidden_states.device(), at::kBFloat16).contiguous();
+    at::Tensor counts = dcounts.cpu();
+    const int32_t* cnt = counts.data_ptr<int32_t>();
+    TORCH_CHECK(cnt[experts] == 0, "WOQ: topk_ids names an expert beyond the contexts given");
+    auto rows_of = [&](int64_t width) { return at::empty({pairs, width}, hidden_states.options()); };
+    at::Tensor x = rows_of(hidden), gate = rows_of(ffn), act = rows_of(ffn), res = rows_of(hidden);
+    WOQ_CHECK(woq_b200_gather_rows(hidden_states.data_ptr(), hidden, token_of.data_ptr<int32_t>(), pairs, hidden,
+                                   x.data_ptr(), stream));
+    int32_t most = 0;
+    for (int64_t e = 0; e < experts; ++e) most = std::max(most, cnt[e]);
+    auto row = [](const at::Tensor& t, int64_t r) { return static_cast<uint8_t*>(t.data_ptr()) + r * t.size(1) * 2; };
+    if (most > 16) {
+      at::Tensor up = rows_of(ffn);
+      std::vector<const woq_b200_ctx*> gu, d;
+      std::vector<int64_t> row0, rows, row0d, rowsd;
+      std::vector<void*> y, yd;
+      int64_t off = 0;
+      for (int64_t e = 0; e < experts; ++e) {
+        if (cnt[e] == 0) continue;
+        for (const auto* c : {&gate_ctx[e], &up_ctx[e]}) {
+          gu.push_back((*c)->ctx_for(17));  // the tensor-core tiling
+          row0.push_back(off);
+          rows.push_back(cnt[e]);
+          y.push_back(row(c == &gate_ctx[e] ? gate : up, off));
+        }
+        d.push_back(down_ctx[e]->ctx_for(17));
+        row0d.push_back(off);
+        rowsd.push_back(cnt[e]);
+        yd.push_back(row(res, off));
+        off += cnt[e];
+      }
+      at::Tensor& ws = workspace_for(dev, stream, woq_b200_workspace_bytes(gu[0], std::max<int64_t>(17, most)));
+      WOQ_CHECK(woq_b200_linear_grouped(gu.data(), row0.data(), rows.data(), y.data(), static_cast<int32_t>(gu.size()),
+                                        x.data_ptr(), pairs, hidden, ffn, ws.data_ptr(), ws.numel(), stream));
+      WOQ_CHECK(woq_b200_silu_mul(gate.data_ptr(), up.data_ptr(), act.data_ptr(), pairs * ffn, stream));
+      WOQ_CHECK(woq_b200_linear_grouped(d.data(), row0d.data(), rowsd.data(), yd.data(),
+                                        static_cast<int32_t>(d.size()), act.data_ptr(), pairs, ffn, hidden,
+                                        ws.data_ptr(), ws.numel(), stream));
+    } else {
+      int64_t off = 0;
+      for (int64_t e = 0; e < experts; ++e) {
+        if (cnt[e] == 0) continue;
+        auto linear = [&](const c10::intrusive_ptr<WoqLinearOpContext>& c, const at::Tensor& in, int32_t fusion,
+                          const void* other, const at::Tensor& out) {
+          woq_b200_ctx* k = c->ctx_for(cnt[e]);
+          at::Tensor& ws = workspace_for(dev, stream, woq_b200_workspace_bytes(k, cnt[e]));
+          WOQ_CHECK(woq_b200_linear(k, row(in, off), cnt[e], in.size(1), fusion, other ? &other : nullptr,
+                                    other ? 1 : 0, row(out, off), out.size(1), ws.data_ptr(), ws.numel(), stream));
+        };
+        linear(gate_ctx[e], x, WOQ_B200_FUSE_SILU, nullptr, gate);
+        linear(up_ctx[e], x, WOQ_B200_FUSE_MUL, row(gate, off), act);
+        linear(down_ctx[e], act, WOQ_B200_FUSE_NONE, nullptr, res);
+        off += cnt[e];
+      }
+    }
+    at::Tensor output = at::empty_like(hidden_states);
+    WOQ_CHECK(woq_b200_moe_combine(res.data_ptr(), flat.data_ptr<int64_t>(), pos_of.data_ptr<int32_t>(), w.data_ptr(),
+                                   tokens, static_cast<int32_t>(top_k), hidden, output.data_ptr(), stream));
+    return output;
+  }
+
+  at::Tensor output = at::zeros_like(hidden_states);
   at::Tensor order = at::argsort(flat, /*stable=*/true, /*dim=*/0, /*descending=*/false);
   at::Tensor counts = at::bincount(flat, {}, experts).cpu();
   TORCH_CHECK(counts.size(0) == experts, "WOQ: topk_ids names an expert beyond the contexts given");

@@ -940,46 +940,162 @@ static int make_kblock_map(CUtensorMap* map, const void* base, int64_t rows, int
   return WOQ_B200_OK;
 }
 
+static int pair_kind(const woq_b200_ctx* c) {
+  if (c->desc.weight_dtype == WOQ_B200_DTYPE_INT8) return c->plain_scales ? woq::kWeightInt8InPlace : woq::kWeightInt8;
+  if (c->desc.weight_dtype == WOQ_B200_DTYPE_NF4) return woq::kWeightNf4;
+  return c->plain_scales ? woq::kWeightInt4InPlace : woq::kWeightInt4;
+}
+
+// what the groups of a launch share; n_tok, the groups and the epilogue are the caller's
+static void fill_pair(const woq_b200_ctx* c, woq::PairParams* p, uint8_t* w8) {
+  p->status = reinterpret_cast<int*>(w8);
+  p->counters = reinterpret_cast<uint32_t*>(w8 + 256);
+  p->partials = reinterpret_cast<float*>(w8 + kWsHeaderBytes);
+  p->n = (int)c->desc.n;
+  p->n_out = (int)c->desc.n;
+  p->tiles = c->tiles_tc;
+  p->w_tiles = (c->tiles_tc + 1) / 2;
+  p->kb_per_tile = c->kb_per_tile;
+  p->kbpg_shift = c->kbpg_shift;
+  p->groups = c->groups;
+  p->gate_up = c->gate_up;
+  p->kind = pair_kind(c);
+}
+
+// Appends a group of `rows` tokens from row `row0` of x (n_tok must be set).
+static void add_pair_group(const woq_b200_ctx* c, woq::PairParams* p, int64_t row0, int64_t rows, void* y) {
+  woq::PairGroup& g = p->group[p->n_groups++];
+  g.wq = c->wq_tc;
+  g.sz = c->sz_tc;
+  g.bias = c->bias;
+  g.y = static_cast<__nv_bfloat16*>(y);
+  g.row0 = (int)row0;
+  g.m = (int)rows;
+  g.tok_tiles = (int)((rows + p->n_tok - 1) / p->n_tok);
+  g.item0 = p->items;
+  p->items += p->w_tiles * g.tok_tiles;
+  const int part = rows < p->n_tok ? (int)rows : p->n_tok;
+  if (part > p->part_tok) p->part_tok = part;
+}
+
 // One launch on CTA pairs, whatever the token count.
 static int run_pair(const woq_b200_ctx* c, const void* x, int64_t m, int64_t ldx, int32_t fusion, const void* o0,
                     const void* o1, const int32_t* row_idx, const void* row_w, void* y, int64_t ldy, uint8_t* w8,
                     cudaStream_t stream) {
   woq::PairParams p{};
-  p.wq = c->wq_tc;
-  p.sz = c->sz_tc;
-  p.bias = c->bias;
-  p.y = static_cast<__nv_bfloat16*>(y);
+  fill_pair(c, &p, w8);
+  int tok_tiles;
+  woq::pair_token_tiles(m, &p.n_tok, &tok_tiles);
+  add_pair_group(c, &p, 0, m, y);
   p.other0 = static_cast<const __nv_bfloat16*>(o0);
   p.other1 = static_cast<const __nv_bfloat16*>(o1);
   p.row_idx = row_idx;
   p.row_w = static_cast<const __nv_bfloat16*>(row_w);
-  p.status = reinterpret_cast<int*>(w8);
-  p.counters = reinterpret_cast<uint32_t*>(w8 + 256);
-  p.partials = reinterpret_cast<float*>(w8 + kWsHeaderBytes);
   p.ldy = ldy;
-  p.m = (int)m;
-  p.n = (int)c->desc.n;
-  p.n_out = fusion == WOQ_B200_FUSE_SILU_MUL ? (int)(c->desc.n / 2) : (int)c->desc.n;
-  woq::pair_token_tiles(m, &p.n_tok, &p.tok_tiles);
-  p.tiles = c->tiles_tc;
-  p.w_tiles = (c->tiles_tc + 1) / 2;
-  p.kb_per_tile = c->kb_per_tile;
-  p.kbpg_shift = c->kbpg_shift;
-  p.groups = c->groups;
+  if (fusion == WOQ_B200_FUSE_SILU_MUL) p.n_out = (int)(c->desc.n / 2);
   p.fusion = fusion;
-  p.gate_up = c->gate_up;
   p.vec = ldy % 8 == 0 && aligned16(y) && (!o0 || aligned16(o0)) && (!o1 || aligned16(o1));
-  p.part_tok = m < p.n_tok ? (int)m : p.n_tok;
-  if (c->desc.weight_dtype == WOQ_B200_DTYPE_INT8)
-    p.kind = c->plain_scales ? woq::kWeightInt8InPlace : woq::kWeightInt8;
-  else if (c->desc.weight_dtype == WOQ_B200_DTYPE_NF4)
-    p.kind = woq::kWeightNf4;
-  else
-    p.kind = c->plain_scales ? woq::kWeightInt4InPlace : woq::kWeightInt4;
   if (woq::pair_plan(p) == 0) return fail(WOQ_B200_ERR_UNSUPPORTED, "no pipeline shape for %d token columns", p.n_tok);
   CUtensorMap xmap;
   if (int rc = make_kblock_map(&xmap, x, m, c->desc.k, ldx, p.n_tok / 2, p.kbs)) return rc;
   CUDA_TRY(woq::launch_pair(p, xmap, c->num_sms, stream));
+  woq::count_launch();
+  return WOQ_B200_OK;
+}
+
+int woq_b200_linear_grouped(const woq_b200_ctx* const* ctxs, const int64_t* row0, const int64_t* rows, void* const* y,
+                            int32_t groups, const void* x, int64_t total_rows, int64_t ldx, int64_t ldy,
+                            void* workspace, size_t workspace_bytes, void* stream_) {
+  if (groups < 0) return fail(WOQ_B200_ERR_INVALID_ARG, "negative number of groups");
+  if (groups == 0) return WOQ_B200_OK;
+  if (!ctxs || !row0 || !rows || !y || !x || !workspace) return fail(WOQ_B200_ERR_INVALID_ARG, "null argument");
+  int64_t most = 0;
+  int in_place = 1;
+  for (int g = 0; g < groups; ++g) {
+    const woq_b200_ctx* c = ctxs[g];
+    if (int rc = check_ctx(c)) return rc;
+    if (c->is_int8 || c->is_i8block || c->is_generic || !c->wq_tc || c->gate_up)
+      return fail(WOQ_B200_ERR_UNSUPPORTED, "group %d: an INT4 context with the tensor-core tiling and plain row order "
+                  "is needed", g);
+    if (c->device != ctxs[0]->device || c->desc.n != ctxs[0]->desc.n || c->desc.k != ctxs[0]->desc.k ||
+        c->groups != ctxs[0]->groups || c->kbpg_shift != ctxs[0]->kbpg_shift)
+      return fail(WOQ_B200_ERR_INVALID_ARG, "group %d differs from group 0 in device, shape or group size", g);
+    if (rows[g] <= 0 || row0[g] < 0 || row0[g] + rows[g] > total_rows || !y[g])
+      return fail(WOQ_B200_ERR_INVALID_ARG, "group %d: rows [%lld, +%lld) of %lld, or a null result", g,
+                  (long long)row0[g], (long long)rows[g], (long long)total_rows);
+    if (int rc = settle_prepack_flag(c)) return rc;
+    in_place &= c->plain_scales;
+    if (rows[g] > most) most = rows[g];
+  }
+  const woq_b200_ctx* c0 = ctxs[0];
+  if (int rc = check_current_device(c0)) return rc;
+  if (total_rows > (1ll << 30) || ldx < c0->desc.k || (ldx % 8) != 0 || !aligned16(x))
+    return fail(WOQ_B200_ERR_INVALID_ARG, "x must be 16-byte aligned with ldx >= K and ldx %% 8 == 0");
+  if (ldy < c0->desc.n) return fail(WOQ_B200_ERR_INVALID_ARG, "ldy smaller than the output width");
+  const int n_tok = woq::pair_group_columns(rows, groups);
+  const size_t need = kWsHeaderBytes + woq::pair_partial_bytes(c0->num_sms, most < n_tok ? (int)most : n_tok);
+  if (workspace_bytes < need) return fail(WOQ_B200_ERR_WORKSPACE, "workspace has %zu bytes, need %zu", workspace_bytes, need);
+  CUtensorMap xmap;
+  for (int g0 = 0; g0 < groups; g0 += woq::kMaxPairGroups) {
+    woq::PairParams p{};
+    fill_pair(c0, &p, static_cast<uint8_t*>(workspace));
+    p.kind = in_place ? woq::kWeightInt4InPlace : woq::kWeightInt4;
+    p.n_tok = n_tok;
+    p.ldy = ldy;
+    p.vec = ldy % 8 == 0;
+    for (int g = g0; g < groups && g < g0 + woq::kMaxPairGroups; ++g) {
+      add_pair_group(ctxs[g], &p, row0[g], rows[g], y[g]);
+      p.vec = p.vec && aligned16(y[g]);
+    }
+    if (woq::pair_plan(p) == 0) return fail(WOQ_B200_ERR_UNSUPPORTED, "no pipeline shape for %d token columns", n_tok);
+    if (g0 == 0)
+      if (int rc = make_kblock_map(&xmap, x, total_rows, c0->desc.k, ldx, n_tok / 2, p.kbs)) return rc;
+    CUDA_TRY(woq::launch_pair(p, xmap, c0->num_sms, static_cast<cudaStream_t>(stream_)));
+    woq::count_launch();
+  }
+  return WOQ_B200_OK;
+}
+
+int woq_b200_moe_route(const int64_t* ids, int64_t tokens, int32_t top_k, int32_t experts, int32_t* counts,
+                       int32_t* token_of, int32_t* pos_of, void* stream_) {
+  if (!ids || !counts || !token_of || !pos_of || tokens < 0 || top_k < 1 || experts < 1 || experts > 65535 ||
+      tokens * top_k >= (1ll << 31))
+    return fail(WOQ_B200_ERR_INVALID_ARG, "moe_route: null pointer or sizes out of range");
+  CUDA_TRY(woq::launch_moe_route(ids, tokens * top_k, top_k, experts, counts, token_of, pos_of,
+                                 static_cast<cudaStream_t>(stream_)));
+  woq::count_launch();
+  return WOQ_B200_OK;
+}
+
+int woq_b200_gather_rows(const void* x, int64_t ldx, const int32_t* idx, int64_t rows, int64_t k, void* out,
+                         void* stream_) {
+  if (rows == 0) return WOQ_B200_OK;
+  if (!x || !idx || !out || rows < 0 || k <= 0 || k % 8 != 0 || ldx % 8 != 0 || !aligned16(x) || !aligned16(out))
+    return fail(WOQ_B200_ERR_INVALID_ARG, "gather_rows: rows must be 16-byte aligned, K and ldx multiples of 8");
+  CUDA_TRY(woq::launch_gather_rows(static_cast<const __nv_bfloat16*>(x), ldx, idx, static_cast<__nv_bfloat16*>(out),
+                                   rows, (int)k, static_cast<cudaStream_t>(stream_)));
+  return WOQ_B200_OK;
+}
+
+int woq_b200_silu_mul(const void* gate, const void* up, void* out, int64_t count, void* stream_) {
+  if (count == 0) return WOQ_B200_OK;
+  if (!gate || !up || !out || count < 0 || count % 8 != 0 || !aligned16(gate) || !aligned16(up) || !aligned16(out))
+    return fail(WOQ_B200_ERR_INVALID_ARG, "silu_mul: 16-byte aligned tensors of a multiple of 8 elements");
+  CUDA_TRY(woq::launch_silu_mul(static_cast<const __nv_bfloat16*>(gate), static_cast<const __nv_bfloat16*>(up),
+                                static_cast<__nv_bfloat16*>(out), count, static_cast<cudaStream_t>(stream_)));
+  woq::count_launch();
+  return WOQ_B200_OK;
+}
+
+int woq_b200_moe_combine(const void* rows, const int64_t* ids, const int32_t* pos_of, const void* weights,
+                         int64_t tokens, int32_t top_k, int64_t hidden, void* out, void* stream_) {
+  if (tokens == 0) return WOQ_B200_OK;
+  if (!rows || !ids || !pos_of || !weights || !out || tokens < 0 || tokens >= (1ll << 31) || top_k < 1 || top_k > 64 ||
+      hidden <= 0 || hidden % 8 != 0 || !aligned16(rows) || !aligned16(out))
+    return fail(WOQ_B200_ERR_INVALID_ARG, "moe_combine: at most 64 experts per token, 16-byte aligned rows");
+  CUDA_TRY(woq::launch_moe_combine(static_cast<const __nv_bfloat16*>(rows), ids, pos_of,
+                                   static_cast<const __nv_bfloat16*>(weights), tokens, top_k, (int)hidden,
+                                   static_cast<__nv_bfloat16*>(out), static_cast<cudaStream_t>(stream_)));
   woq::count_launch();
   return WOQ_B200_OK;
 }

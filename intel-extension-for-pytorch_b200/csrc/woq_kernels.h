@@ -158,12 +158,22 @@ __constant__ const float kNf4Table[16] = {-1.0f,
                                           0.5626170039176941f,
                                           0.7229568362236023f,
                                           1.0f};
-struct PairParams {
-  const uint8_t* wq;   // row layout, as TcParams
+// A launch runs one linear, or several of one shape on consecutive row ranges of x (the experts of a
+// mixture): `groups` of them, their items one after the other.
+constexpr int kMaxPairGroups = 32;
+struct PairGroup {
+  const uint8_t* wq;   // row layout
   const uint32_t* sz;
   const float* bias;
-  __nv_bfloat16* y;
-  const __nv_bfloat16* other0;
+  __nv_bfloat16* y;    // result of the group's first token
+  int row0, m;         // first row of x, tokens
+  int tok_tiles;       // tiles of tokens
+  int item0;           // number of the group's first (256-row tile, token tile) item
+};
+struct PairParams {
+  PairGroup group[kMaxPairGroups];
+  int n_groups, items;
+  const __nv_bfloat16* other0;  // extra operands: one group only
   const __nv_bfloat16* other1;
   const int32_t* row_idx;
   const __nv_bfloat16* row_w;
@@ -171,18 +181,19 @@ struct PairParams {
   uint32_t* counters;  // [CTAs], zero between calls
   int* status;
   int64_t ldy;
-  int m, n, n_out;
-  int n_tok, tok_tiles;         // token columns of a tile (a multiple of 32, <= 256); tiles of tokens
+  int n, n_out;
+  int n_tok;                    // token columns of a tile (a multiple of 32, <= 256)
   int tiles, w_tiles;           // 128-row tiles; pairs of them (rounded up)
   int kb_per_tile, kbpg_shift, groups;
   int kbs, stages, w_ring;      // k-blocks per stage; slots of the two rings
   int unit;                     // shares are multiples of this many k-blocks
   int fusion, gate_up;
   int kind;      // WeightKind
-  int part_tok;  // tokens of a partial tile: min(m, n_tok)
+  int part_tok;  // tokens of a partial tile: min(most tokens of a group, n_tok)
   int vec;  // y and the extra operands can be accessed 16 bytes at a time
 };
 void pair_token_tiles(int64_t m, int* n_tok, int* tok_tiles);
+int pair_group_columns(const int64_t* rows, int groups);
 size_t pair_plan(PairParams& p);  // fills kbs, stages, w_ring, unit; dynamic shared memory (0: none)
 size_t pair_partial_bytes(int num_sms, int part_tok);
 cudaError_t launch_pair(PairParams p, const CUtensorMap& xmap, int num_sms, cudaStream_t stream);
@@ -313,6 +324,15 @@ cudaError_t launch_dump_dequant_int4_tc(const uint8_t* tiled, const uint32_t* sz
 
 cudaError_t launch_gather_rows(const __nv_bfloat16* x, int64_t ldx, const int32_t* idx,
                                __nv_bfloat16* out, int64_t rows, int k, cudaStream_t stream);
+
+// ---- mixture of experts: routing, activation and combination around the experts' linears (woq_moe.cu) ----
+cudaError_t launch_moe_route(const int64_t* ids, int64_t pairs, int top_k, int experts, int32_t* counts,
+                             int32_t* token_of, int32_t* pos_of, cudaStream_t stream);
+cudaError_t launch_silu_mul(const __nv_bfloat16* gate, const __nv_bfloat16* up, __nv_bfloat16* out, int64_t count,
+                            cudaStream_t stream);
+cudaError_t launch_moe_combine(const __nv_bfloat16* rows, const int64_t* ids, const int32_t* pos_of,
+                               const __nv_bfloat16* w, int64_t tokens, int top_k, int hidden, __nv_bfloat16* out,
+                               cudaStream_t stream);
 
 // AWQ / GPTQ int32 checkpoints -> plain nibble layout [n][k/2]
 cudaError_t launch_awq_to_plain(const int32_t* qweight_kn8, uint8_t* plain, int n, int k,

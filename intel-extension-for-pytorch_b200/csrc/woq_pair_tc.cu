@@ -16,7 +16,7 @@
 //               memory runs beside the next tile's MMAs.
 //   warps 12-27 dequantise: thread = output row, one k-block of a stage per warpgroup
 //
-// Work split: the sequence of (256-row tile, token tile, k-block), token tiles innermost but
+// Work split: the sequence of (linear, 256-row tile, token tile, k-block), token tiles innermost but
 // for k, is cut into equal contiguous shares, one per pair ("stream-K").  A tile that several
 // pairs share is summed in k order: whoever arrives last adds the others' fp32 partial tiles from
 // the workspace (the pair that holds the beginning of the tile reaches it at the end of its own
@@ -66,6 +66,13 @@ __device__ __forceinline__ int pair_owner_of(int64_t b, int64_t total, int64_t p
   return static_cast<int>(((b + 1) * pairs - 1) / total);
 }
 
+// group of an item, and the item's place in it
+__device__ __forceinline__ int pair_group_of(const PairParams& p, int item) {
+  int g = 0;
+  while (g + 1 < p.n_groups && item >= p.group[g + 1].item0) ++g;
+  return g;
+}
+
 __device__ __forceinline__ float bf_lo(uint32_t v) { return __uint_as_float(v << 16); }
 __device__ __forceinline__ float bf_hi(uint32_t v) { return __uint_as_float(v & 0xffff0000u); }
 __device__ __forceinline__ uint32_t bf_pack(float lo, float hi) {
@@ -112,7 +119,7 @@ __device__ __forceinline__ void store8(__nv_bfloat16* p, size_t o, const float (
 // The finished bf16 tile S[token][128 rows] -> fused post-op -> y, by the epilogue warps.  A thread
 // takes eight neighbouring columns of a token at a time, two such pieces together, so that the
 // operand loads of both are in flight before the first is used.
-__device__ __forceinline__ void pair_copy_out(const PairParams& p, const uint8_t* S, int tile, int tok0, int mv, int tid) {
+__device__ __forceinline__ void pair_copy_out(const PairParams& p, __nv_bfloat16* y, const uint8_t* S, int tile, int tok0, int mv, int tid) {
   constexpr int kBatch = 2;
   const bool silu_mul = p.fusion == FUSE_SILU_MUL;
   const int sh = silu_mul ? 3 : 4;  // pieces per token: 8 or 16
@@ -146,7 +153,7 @@ __device__ __forceinline__ void pair_copy_out(const PairParams& p, const uint8_t
       if (valid[u] > 0) {
         if (fusion == FUSE_ADD || fusion == FUSE_ADD_ADD || fusion == FUSE_MUL) f0[u] = load8(p.other0, off[u], valid[u], vec);
         if (fusion == FUSE_ADD_ADD) f1[u] = load8(p.other1, off[u], valid[u], vec);
-        if (fusion == FUSE_SCALED_SCATTER_ADD) f0[u] = load8(p.y, off[u], valid[u], vec);
+        if (fusion == FUSE_SCALED_SCATTER_ADD) f0[u] = load8(y, off[u], valid[u], vec);
       }
     }
 #pragma unroll
@@ -187,7 +194,7 @@ __device__ __forceinline__ void pair_copy_out(const PairParams& p, const uint8_t
 #pragma unroll
         for (int e = 0; e < 8; ++e) r[e] = unary_post_op(r[e], fusion);
       }
-      store8(p.y, off[u], r, valid[u], vec);
+      store8(y, off[u], r, valid[u], vec);
     }
   }
 }
@@ -304,9 +311,9 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   const int64_t pairs = gridDim.x >> 1;
   const int kbpt = p.kb_per_tile, kbs = p.kbs, n_stages = p.stages, n_wring = p.w_ring;
   // shares are dealt in units of p.unit k-blocks
-  const int64_t units = static_cast<int64_t>(p.w_tiles) * p.tok_tiles * kbpt / p.unit;
+  const int64_t units = static_cast<int64_t>(p.items) * kbpt / p.unit;
   const int64_t b_begin = pair * units / pairs * p.unit, b_end = (pair + 1) * units / pairs * p.unit;
-  const int item0 = static_cast<int>(b_begin / kbpt);       // item = weight tile * tok_tiles + token tile
+  const int item0 = static_cast<int>(b_begin / kbpt);  // item - group.item0 = weight tile * tok_tiles + token tile
   const int kb00 = static_cast<int>(b_begin % kbpt);
   const int rem0 = static_cast<int>(b_end - b_begin);
 
@@ -339,13 +346,14 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   if (warp == 0) {
     // ---- packed weights and their group scales (never written by an earlier launch) ----
     if (lane == 0) {
-      int item = item0, kb0 = kb00, rem = rem0, wslot = 0;
+      int item = item0, kb0 = kb00, rem = rem0, wslot = 0, g = pair_group_of(p, item0);
       uint32_t wphase = 0;
       while (rem > 0) {
-        int tile = item / p.tok_tiles * 2 + static_cast<int>(rank);
+        if (g + 1 < p.n_groups && item >= p.group[g + 1].item0) ++g;
+        int tile = (item - p.group[g].item0) / p.group[g].tok_tiles * 2 + static_cast<int>(rank);
         if (tile >= p.tiles) tile = p.tiles - 1;  // odd tile count: the last pair's second half repeats it
-        const uint8_t* wsrc = p.wq + (static_cast<size_t>(tile) * kbpt + kb0) * kBlock;
-        const uint32_t* ssrc = p.sz + static_cast<size_t>(tile) * p.groups * kTcTileN;
+        const uint8_t* wsrc = p.group[g].wq + (static_cast<size_t>(tile) * kbpt + kb0) * kBlock;
+        const uint32_t* ssrc = p.group[g].sz + static_cast<size_t>(tile) * p.groups * kTcTileN;
         int seg = kbpt - kb0 < rem ? kbpt - kb0 : rem;
         rem -= seg;
         while (seg > 0) {
@@ -376,11 +384,14 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     // ---- the share still loads whole: its last k-blocks are not used) ----
     if (lane == 0) {
       grid_dependency_wait();
-      int item = item0, kb0 = kb00, rem = rem0, slot = 0;
+      int item = item0, kb0 = kb00, rem = rem0, slot = 0, g = pair_group_of(p, item0);
       uint32_t phase = 0;
       const uint32_t full0 = pair_map(&hdr->full[0], 0);
       while (rem > 0) {
-        const int row = item % p.tok_tiles * p.n_tok + static_cast<int>(rank) * half_tok;
+        if (g + 1 < p.n_groups && item >= p.group[g + 1].item0) ++g;
+        // (rows past the group's last belong to another group or to nobody: their columns are not used)
+        const int row = p.group[g].row0 + (item - p.group[g].item0) % p.group[g].tok_tiles * p.n_tok +
+                        static_cast<int>(rank) * half_tok;
         int seg = kbpt - kb0 < rem ? kbpt - kb0 : rem;
         rem -= seg;
         for (; seg > 0; seg -= kbs) {
@@ -503,7 +514,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     const uint32_t d_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
     const uint32_t d_empty0 = pair_map(&hdr->d_empty, 0);
     grid_dependency_wait();  // y, the fused operands and the workspace belong to this grid now
-    int item = item0, kb0 = kb00, rem = rem0;
+    int item = item0, kb0 = kb00, rem = rem0, g = pair_group_of(p, item0);
     uint32_t seg_no = 0;
     auto to_tile = [&](int c0, const float (&v)[16], float bias) {  // 16 tokens of this row, as bf16
       uint8_t* dst = out_tile + c0 * kOutPitch + row * 2;
@@ -518,14 +529,17 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     while (rem > 0) {
       const int seg_len = kbpt - kb0 < rem ? kbpt - kb0 : rem;
       const bool whole = seg_len == kbpt;
-      const int tile = item / p.tok_tiles * 2 + static_cast<int>(rank);
-      const int tok0 = item % p.tok_tiles * p.n_tok;
-      const int mv = p.m - tok0 < p.n_tok ? p.m - tok0 : p.n_tok;
+      if (g + 1 < p.n_groups && item >= p.group[g + 1].item0) ++g;
+      const PairGroup& grp = p.group[g];
+      const int in_group = item - grp.item0;
+      const int tile = in_group / grp.tok_tiles * 2 + static_cast<int>(rank);
+      const int tok0 = in_group % grp.tok_tiles * p.n_tok;
+      const int mv = grp.m - tok0 < p.n_tok ? grp.m - tok0 : p.n_tok;
       const bool real = tile < p.tiles;
       float bias = 0.f;
-      if (p.bias && real) {
+      if (grp.bias && real) {
         const int n = tc_tile_row_to_n(p.n, p.gate_up, tile, row);
-        if (n < p.n) bias = p.bias[n];
+        if (n < p.n) bias = grp.bias[n];
       }
       // the bf16 tile of the previous segment has been copied out by everybody
       named_bar_sync(kEpiBar, kEpiThreads);
@@ -619,7 +633,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         }
       }
       named_bar_sync(kEpiBar, kEpiThreads);
-      if (finish) pair_copy_out(p, out_tile, tile, tok0, mv, et);
+      if (finish) pair_copy_out(p, grp.y, out_tile, tile, tok0, mv, et);
       rem -= seg_len;
       kb0 = 0;
       ++item;
@@ -646,6 +660,23 @@ void pair_token_tiles(int64_t m, int* n_tok, int* tok_tiles) {
   *tok_tiles = t < 1 ? 1 : t;
   *n_tok = static_cast<int>(((m + *tok_tiles - 1) / *tok_tiles + 31) / 32 * 32);
   if (*n_tok < 32) *n_tok = 32;
+}
+
+// Token columns for several linears in one launch, by the number of tokens each has: the width with the least
+// sum over their tiles.  A k-block costs a tile about 120 + columns in units of a column's MMAs (8192 x 57344
+// weights: 91 us at 32 columns, 150 at 128, one tile each).
+int pair_group_columns(const int64_t* rows, int groups) {
+  int best = 256;
+  int64_t best_cost = -1;
+  for (int n = 256; n >= 32; n -= 32) {
+    int64_t cost = 0;
+    for (int g = 0; g < groups; ++g) cost += (rows[g] + n - 1) / n * (120 + n);
+    if (best_cost < 0 || cost < best_cost) {
+      best_cost = cost;
+      best = n;
+    }
+  }
+  return best;
 }
 
 // Pipeline shape for p.n_tok token columns; returns the dynamic shared memory in bytes.
@@ -676,7 +707,7 @@ size_t pair_plan(PairParams& p) {
   p.stages = stages;
   p.w_ring = ring;
   // shares in whole stages where they are long enough for the rounding not to matter
-  const int64_t total = static_cast<int64_t>(p.w_tiles) * p.tok_tiles * p.kb_per_tile;
+  const int64_t total = static_cast<int64_t>(p.items) * p.kb_per_tile;
   p.unit = p.kb_per_tile % p.kbs == 0 && total >= static_cast<int64_t>(74) * 8 * p.kbs ? p.kbs : 1;
   return kPairHeaderBytes + static_cast<size_t>(stages) * x_stage + static_cast<size_t>(ring) * w_stage +
          static_cast<size_t>(p.n_tok) * kOutPitch + lut;
@@ -684,7 +715,7 @@ size_t pair_plan(PairParams& p) {
 
 // Pairs of a launch: all SMs, or one per k-block when there are fewer.
 int pair_grid(const PairParams& p, int num_sms) {
-  const int64_t total = static_cast<int64_t>(p.w_tiles) * p.tok_tiles * p.kb_per_tile;
+  const int64_t total = static_cast<int64_t>(p.items) * p.kb_per_tile;
   int64_t pairs = num_sms / 2;
   if (pairs > total) pairs = total;
   return static_cast<int>(pairs < 1 ? 1 : pairs) * 2;

@@ -50,6 +50,11 @@ EXPORTS = [
     "woq_b200_static_scratch_status",
     "woq_b200_moe_workspace_bytes",
     "woq_b200_moe_expert",
+    "woq_b200_linear_grouped",
+    "woq_b200_moe_route",
+    "woq_b200_gather_rows",
+    "woq_b200_silu_mul",
+    "woq_b200_moe_combine",
     "woq_b200_dump_dequant",
     "woq_b200_int8_internals",
     "woq_b200_rmsnorm_quant",
@@ -133,6 +138,11 @@ def lib() -> ctypes.CDLL:
     L.woq_b200_moe_workspace_bytes.argtypes = [vp, vp, i64]
     L.woq_b200_moe_workspace_bytes.restype = sz
     L.woq_b200_moe_expert.argtypes = [vp, vp, vp, i64, vp, vp, i64, vp, i64, vp, sz, vp]
+    L.woq_b200_linear_grouped.argtypes = [vp, vp, vp, vp, i32, vp, i64, i64, i64, vp, sz, vp]
+    L.woq_b200_moe_route.argtypes = [vp, i64, i32, i32, vp, vp, vp, vp]
+    L.woq_b200_gather_rows.argtypes = [vp, i64, vp, i64, i64, vp, vp]
+    L.woq_b200_silu_mul.argtypes = [vp, vp, vp, i64, vp]
+    L.woq_b200_moe_combine.argtypes = [vp, vp, vp, vp, i64, i32, i64, vp, vp]
     L.woq_b200_dump_dequant.argtypes = [vp, vp, vp]
     L.woq_b200_int8_internals.argtypes = [vp, vp, i64, i64, vp, vp, vp, vp, sz, vp]
     L.woq_b200_rmsnorm_quant.argtypes = [vp, i64, vp, ctypes.c_float, i64, i64, i32, vp, i64, vp, vp, vp, vp]

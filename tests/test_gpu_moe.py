@@ -170,3 +170,39 @@ def test_config4_expert_shapes_one_token(env):
                               O.WOQ_DTYPE_INT4, G)
         acc = O.rne_bf16(acc + y * np.float32(wt))
     parity(bf16_numpy(out), acc)
+
+
+@pytest.mark.parametrize("tokens,experts,top_k", [(1, 4, 2), (17, 4, 2), (33, 3, 1), (70, 40, 6), (700, 8, 2)])
+def test_deepseek_moe_expert_counts(env, tokens, experts, top_k):
+    """Every expert on the streaming kernel, mixed and all grouped, more groups than one launch takes, experts
+    nobody chose, uneven counts; against the per-expert operator (same bf16 weights and results, other order of
+    the fp32 sums) and an id beyond the experts is refused."""
+    hidden, ffn, g = 320, 192, 64
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+
+    def ctx(n, k):
+        w = torch.randn((n, k), device="cuda", generator=gen) * 0.05
+        q, s, z = env.quantization.quantize_per_block(w, 2, g)
+        return torch.ops.ipex_prepack.weight_only_qlinear_prepack(q, 2, [n, k], s, z, None, None, None, g, 2, -1)
+
+    gate, up = [ctx(ffn, hidden) for _ in range(experts)], [ctx(ffn, hidden) for _ in range(experts)]
+    down = [ctx(hidden, ffn) for _ in range(experts)]
+    x = torch.randn((tokens, hidden), device="cuda", generator=gen).bfloat16()
+    p = torch.softmax(torch.randn((tokens, experts), device="cuda", generator=gen) +
+                      torch.arange(experts, device="cuda") * (2.0 / experts), -1)
+    if experts > 3:
+        p[:, 1] = 0  # nobody's expert
+    w, ids = torch.topk(p, top_k, -1)
+    w = w.bfloat16()
+    out = torch.ops.torch_ipex.deepseek_moe_woq(x, ids, gate, up, down, w, False)
+    ref = torch.zeros_like(out)
+    for e in range(experts):
+        top_x, j = torch.where(ids == e)
+        ref = torch.ops.torch_ipex.mixtral_moe_woq(x, top_x, j, gate[e].get_data_handle(), up[e].get_data_handle(),
+                                                   down[e].get_data_handle(), w, ref, False)
+    # a sum that rounds to the neighbouring bf16 value moves a product and an addition by one unit each
+    assert (out.float() - ref.float()).norm() <= 4e-3 * ref.float().norm()
+    bad = ids.clone()
+    bad[tokens // 2, 0] = experts
+    with pytest.raises(RuntimeError):
+        torch.ops.torch_ipex.deepseek_moe_woq(x, bad, gate, up, down, w, False)
