@@ -95,6 +95,9 @@ struct woq_b200_ctx {
   int g_row_bytes, g_group, g_groups;
   // INT8 compute with K-block scaling (woq_int8_block.cu): the buffers above plus comp
   int is_i8block, kb, kc;
+  int btc;          // INT4, symmetric activations, K blocks of 128: weight in wq_tc for the tcgen05 kernel
+  float* btc_sw;    // [tiles_tc][groups][128]
+  uint32_t* btc_zw; // [tiles_tc][groups][128]
   int* d_flag;
   int* h_flag;
   cudaEvent_t flag_ready;
@@ -281,7 +284,8 @@ bool wants_i8block(const woq_b200_desc* d) {
 }
 
 struct I8BlockWs {
-  size_t qa, sa, zpa, sumqa, range, folded, total;
+  size_t qa, sa, zpa, sumqa, range, folded, sat, partials, total;
+  int n_tok, tok_tiles, part_tok;  // tcgen05 kernel
 };
 I8BlockWs i8block_ws(const woq_b200_ctx* c, int64_t m) {
   I8BlockWs w;
@@ -293,12 +297,72 @@ I8BlockWs i8block_ws(const woq_b200_ctx* c, int64_t m) {
   w.range = off;   off += (mk * 8 + 255) / 256 * 256;
   w.folded = off;  off += (static_cast<size_t>(m > c->kc ? m : c->kc) * 8 + 255) / 256 * 256;
   w.qa = off;      off += (static_cast<size_t>(m) * c->desc.k + 255) / 256 * 256;
+  w.sat = w.partials = off;
+  w.n_tok = w.tok_tiles = w.part_tok = 0;
+  if (c->btc) {
+    w.n_tok = woq::i8_block_tc_columns(m);
+    w.tok_tiles = static_cast<int>((m + w.n_tok - 1) / w.n_tok);
+    w.part_tok = m < w.n_tok ? static_cast<int>(m) : w.n_tok;
+    off += (static_cast<size_t>(w.tok_tiles) * c->kc * w.n_tok * 4 + 255) / 256 * 256;
+    w.partials = off;
+    off += woq::i8_block_tc_partial_bytes(c->num_sms, w.part_tok);
+  }
   w.total = off;
   return w;
 }
 
 int create_generic(const woq_b200_desc* d, const void* qweight, const void* scales, const void* zero_points,
                    const void* bias, cudaStream_t stream, woq_b200_ctx** out, bool allow_rows);
+
+// INT4 weights with symmetric activation codes and K blocks of 128 move to the layout of the tcgen05 kernel
+// (one copy of the weight); zero points outside 0..127 keep the layer on the mma.sync kernels.
+cudaError_t move_to_btc(woq_b200_ctx* c, cudaStream_t stream) {
+  const woq_b200_desc& d = c->desc;
+  if (d.weight_dtype != WOQ_B200_DTYPE_INT4 || !(d.act_quant_mode & 4) || c->kb != 128) return cudaSuccess;
+  if (c->g_group < d.k && c->g_group % 128 != 0) return cudaSuccess;
+  c->tiles_tc = static_cast<int>((d.n + 127) / 128);
+  c->groups = c->g_groups;
+  const size_t w_bytes = static_cast<size_t>(c->tiles_tc) * c->kc * 8192;
+  const size_t s_bytes = static_cast<size_t>(c->tiles_tc) * c->groups * 128 * 4;
+  int* flag = nullptr;
+  int bits = 1;
+  cudaError_t e = cudaMalloc(&c->btc_sw, s_bytes);
+  if (e == cudaSuccess) e = cudaMalloc(&c->btc_zw, s_bytes);
+  if (e == cudaSuccess) e = cudaMalloc(&flag, sizeof(int));
+  if (e == cudaSuccess) e = cudaMemsetAsync(flag, 0, sizeof(int), stream);
+  if (e == cudaSuccess)
+    e = woq::launch_btc_pack_scales(c->g_scales, c->g_zps, c->btc_sw, c->btc_zw, (int)d.n, c->groups, flag, stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&bits, flag, sizeof(int), cudaMemcpyDeviceToHost, stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+  if (e == cudaSuccess && !bits) {
+    woq::count_launch();
+    e = cudaMalloc(&c->wq_tc, w_bytes);
+    if (e == cudaSuccess) e = woq::launch_btc_pack(c->g_w, c->wq_tc, (int)d.n, (int)d.k, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
+    if (e == cudaSuccess) {
+      woq::count_launch();
+      cudaFree(c->g_w);
+      cudaFree(c->g_scales);
+      cudaFree(c->g_zps);
+      c->g_w = nullptr;
+      c->g_scales = c->g_zps = nullptr;
+      c->wq_bytes = c->sz_bytes = 0;
+      c->wq_tc_bytes = w_bytes;
+      c->sz_tc_bytes = 2 * s_bytes;
+      c->btc = 1;
+    }
+  }
+  if (flag) cudaFree(flag);
+  if (!c->btc) {
+    cudaFree(c->btc_sw);
+    cudaFree(c->btc_zw);
+    cudaFree(c->wq_tc);
+    c->btc_sw = nullptr;
+    c->btc_zw = nullptr;
+    c->wq_tc = nullptr;
+  }
+  return e;
+}
 
 int create_i8block(const woq_b200_desc* d, const void* qweight, const void* scales, const void* zero_points,
                    const void* bias, cudaStream_t stream, woq_b200_ctx** out) {
@@ -335,9 +399,17 @@ int create_i8block(const woq_b200_desc* d, const void* qweight, const void* scal
     }
     woq::count_launch();
   }
+  if (cudaError_t e = move_to_btc(c, stream)) {
+    woq_b200_ctx_destroy(c);
+    return fail(WOQ_B200_ERR_CUDA, "weight layout of the K-block INT8 kernel: %s", cudaGetErrorString(e));
+  }
   *out = c;
   return WOQ_B200_OK;
 }
+
+int run_i8block_tc(const woq_b200_ctx* c, const I8BlockWs& L, const __nv_bfloat16* x, int64_t m, int64_t ldx,
+                   int32_t fusion, const void* o0, const void* o1, void* y, int64_t ldy, float* sa_out, int32_t* zpa_out,
+                   int32_t* acc_out, uint8_t* w8, cudaStream_t stream);
 
 int run_i8block(const woq_b200_ctx* c, const void* x, int64_t m, int64_t ldx, int32_t fusion, const void* o0,
                 const void* o1, void* y, int64_t ldy, uint8_t* qa_natural, float* sa_out, int32_t* zpa_out,
@@ -360,6 +432,7 @@ int run_i8block(const woq_b200_ctx* c, const void* x, int64_t m, int64_t ldx, in
                                          range, folded, stream));
     woq::count_launch();
   }
+  if (c->btc) return run_i8block_tc(c, L, xb, m, ldx, fusion, o0, o1, y, ldy, sa_out, zpa_out, acc_out, w8, stream);
   CUDA_TRY(woq::launch_act_block_quant(xb, ldx, (int)m, (int)c->desc.k, c->kb, mode, w4, w8 + L.qa, sa, zpa, sumqa,
                                        range, folded, stream));
   woq::count_launch();
@@ -760,6 +833,8 @@ int woq_b200_ctx_destroy(woq_b200_ctx* c) {
   cudaFree(c->g_w);
   cudaFree(c->g_scales);
   cudaFree(c->g_zps);
+  cudaFree(c->btc_sw);
+  cudaFree(c->btc_zw);
   cudaFree(c->wq);
   cudaFree(c->sz);
   cudaFree(c->wq_tc);
@@ -787,6 +862,12 @@ int woq_b200_ctx_unpack(const woq_b200_ctx* c, void* qweight_plain, void* stream
   if (int rc = check_ctx(c)) return rc;
   if (!qweight_plain) return fail(WOQ_B200_ERR_INVALID_ARG, "output is null");
   cudaStream_t stream = static_cast<cudaStream_t>(stream_);
+  if (c->btc) {
+    CUDA_TRY(woq::launch_btc_unpack(c->wq_tc, static_cast<uint8_t*>(qweight_plain), (int)c->desc.n, (int)c->desc.k,
+                                    stream));
+    woq::count_launch();
+    return WOQ_B200_OK;
+  }
   if (c->rows) {
     CUDA_TRY(woq::launch_unpack_rows(c->wq_tc, static_cast<uint8_t*>(qweight_plain), (int)c->desc.n, (int)c->desc.k,
                                      c->desc.weight_dtype == WOQ_B200_DTYPE_INT8, stream));
@@ -924,21 +1005,79 @@ static int make_kmajor_map(CUtensorMap* map, const void* base, int64_t rows, int
   return WOQ_B200_OK;
 }
 
-// The activations as [K / 64][rows][64] with 128-byte swizzle: one box is `kbs` k-blocks of `box_rows` rows.
-static int make_kblock_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int box_rows,
-                           int kbs) {
+// The activations as [K blocks of 128 bytes][rows][128 bytes] with 128-byte swizzle: one box is `kbs` K blocks of
+// `box_rows` rows.  elt_bytes 2: bf16 (K blocks of 64), 1: 8-bit codes (K blocks of 128).
+static int make_kblock_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, int elt_bytes,
+                           int box_rows, int kbs) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return fail(WOQ_B200_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
-  cuuint64_t dims[3] = {64, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(cols / 64)};
-  cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld) * 2, 128};
-  cuuint32_t box[3] = {64, static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(kbs)};
+  const cuuint32_t inner = static_cast<cuuint32_t>(128 / elt_bytes);
+  cuuint64_t dims[3] = {inner, static_cast<cuuint64_t>(rows), static_cast<cuuint64_t>(cols) / inner};
+  cuuint64_t strides[2] = {static_cast<cuuint64_t>(ld) * elt_bytes, 128};
+  cuuint32_t box[3] = {inner, static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(kbs)};
   cuuint32_t estr[3] = {1, 1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  const CUtensorMapDataType dt = elt_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8;
+  CUresult r = fn(map, dt, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(WOQ_B200_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
   return WOQ_B200_OK;
 }
+
+extern "C++" {
+namespace {
+int run_i8block_tc(const woq_b200_ctx* c, const I8BlockWs& L, const __nv_bfloat16* x, int64_t m, int64_t ldx,
+                   int32_t fusion, const void* o0, const void* o1, void* y, int64_t ldy, float* sa_out, int32_t* zpa_out,
+                   int32_t* acc_out, uint8_t* w8, cudaStream_t stream) {
+  const int mode = c->desc.act_quant_mode;
+  float* sa = reinterpret_cast<float*>(w8 + L.sa);
+  int32_t* zpa = reinterpret_cast<int32_t*>(w8 + L.zpa);
+  float* sat = reinterpret_cast<float*>(w8 + L.sat);
+  if (mode == WOQ_B200_ACT_PER_M_K_BLOCK_SYM) {
+    CUDA_TRY(woq::launch_act_block128_quant(x, ldx, (int)m, c->kc, w8 + L.qa, sa, zpa, sat, L.n_tok, stream));
+  } else {
+    CUDA_TRY(woq::launch_act_block_quant(x, ldx, (int)m, (int)c->desc.k, 128, mode, 0, w8 + L.qa, sa, zpa,
+                                         reinterpret_cast<int32_t*>(w8 + L.sumqa), reinterpret_cast<float*>(w8 + L.range),
+                                         reinterpret_cast<float*>(w8 + L.folded), stream));
+    CUDA_TRY(woq::launch_transpose_scales(sa, (int)m, c->kc, sat, L.n_tok, stream));
+    woq::count_launch();
+  }
+  woq::count_launch();
+  const size_t mk = static_cast<size_t>(m) * c->kc;
+  if (sa_out) CUDA_TRY(cudaMemcpyAsync(sa_out, sa, mk * 4, cudaMemcpyDeviceToDevice, stream));
+  if (zpa_out) CUDA_TRY(cudaMemcpyAsync(zpa_out, zpa, mk * 4, cudaMemcpyDeviceToDevice, stream));
+  if (!y && !acc_out) return WOQ_B200_OK;
+  woq::I8BlockTcParams p{};
+  p.w = c->wq_tc;
+  p.zw = c->btc_zw;
+  p.sw = c->btc_sw;
+  p.sat = sat;
+  p.bias = c->bias;
+  p.y = static_cast<__nv_bfloat16*>(y);
+  p.other0 = static_cast<const __nv_bfloat16*>(o0);
+  p.other1 = static_cast<const __nv_bfloat16*>(o1);
+  p.acc_out = acc_out;
+  p.partials = reinterpret_cast<float*>(w8 + L.partials);
+  p.counters = reinterpret_cast<uint32_t*>(w8 + 256);
+  p.status = reinterpret_cast<int*>(w8);
+  p.ldy = ldy;
+  p.m = (int)m;
+  p.n = (int)c->desc.n;
+  p.kc = c->kc;
+  p.groups = c->groups;
+  p.bpg = c->g_group >= c->desc.k ? 1 << 30 : c->g_group / 128;
+  p.n_tok = L.n_tok;
+  p.tok_tiles = L.tok_tiles;
+  p.part_tok = L.part_tok;
+  p.tiles = c->tiles_tc;
+  p.fusion = fusion;
+  CUtensorMap qamap;
+  if (int rc = make_kblock_map(&qamap, w8 + L.qa, m, c->desc.k, c->desc.k, 1, L.n_tok, 2)) return rc;
+  CUDA_TRY(woq::launch_i8_block_tc(p, qamap, c->num_sms, stream));
+  woq::count_launch();
+  return WOQ_B200_OK;
+}
+}  // namespace
+}  // extern "C++"
 
 static int pair_kind(const woq_b200_ctx* c) {
   if (c->desc.weight_dtype == WOQ_B200_DTYPE_INT8) return c->plain_scales ? woq::kWeightInt8InPlace : woq::kWeightInt8;
@@ -997,7 +1136,7 @@ static int run_pair(const woq_b200_ctx* c, const void* x, int64_t m, int64_t ldx
   p.vec = ldy % 8 == 0 && aligned16(y) && (!o0 || aligned16(o0)) && (!o1 || aligned16(o1));
   if (woq::pair_plan(p) == 0) return fail(WOQ_B200_ERR_UNSUPPORTED, "no pipeline shape for %d token columns", p.n_tok);
   CUtensorMap xmap;
-  if (int rc = make_kblock_map(&xmap, x, m, c->desc.k, ldx, p.n_tok / 2, p.kbs)) return rc;
+  if (int rc = make_kblock_map(&xmap, x, m, c->desc.k, ldx, 2, p.n_tok / 2, p.kbs)) return rc;
   CUDA_TRY(woq::launch_pair(p, xmap, c->num_sms, stream));
   woq::count_launch();
   return WOQ_B200_OK;
@@ -1049,7 +1188,7 @@ int woq_b200_linear_grouped(const woq_b200_ctx* const* ctxs, const int64_t* row0
     }
     if (woq::pair_plan(p) == 0) return fail(WOQ_B200_ERR_UNSUPPORTED, "no pipeline shape for %d token columns", n_tok);
     if (g0 == 0)
-      if (int rc = make_kblock_map(&xmap, x, total_rows, c0->desc.k, ldx, n_tok / 2, p.kbs)) return rc;
+      if (int rc = make_kblock_map(&xmap, x, total_rows, c0->desc.k, ldx, 2, n_tok / 2, p.kbs)) return rc;
     CUDA_TRY(woq::launch_pair(p, xmap, c0->num_sms, static_cast<cudaStream_t>(stream_)));
     woq::count_launch();
   }

@@ -265,6 +265,37 @@ cudaError_t launch_weight_block_sum(const uint8_t* w, const float* zpw, int n, i
                                     float default_zp, int w4, int32_t* comp, cudaStream_t stream);
 cudaError_t launch_i8_block(const I8BlockParams& p, cudaStream_t stream);
 
+// ---- the same for INT4 weights, symmetric activations and K blocks of 128 on tcgen05 (woq_i8_block_tc.cu) ----
+struct I8BlockTcParams {
+  const uint8_t* w;      // [tiles][kc][8192] nibbles, see btc_pack_kernel
+  const uint32_t* zw;    // [tiles][groups][128] zero point in every byte
+  const float* sw;       // [tiles][groups][128] weight scales
+  const float* sat;      // [tok_tiles][kc][n_tok] activation scales
+  const float* bias;
+  __nv_bfloat16* y;      // may be null when only the accumulators are wanted
+  const __nv_bfloat16* other0;
+  const __nv_bfloat16* other1;
+  int32_t* acc_out;      // optional [kc][m][n] block accumulators
+  float* partials;       // [CTAs][2][part_tok][128]
+  uint32_t* counters;    // [CTAs], zero between calls
+  int* status;
+  int64_t ldy;
+  int m, n, kc, groups, bpg;  // bpg: K blocks per weight group (a large number: one group)
+  int n_tok, tok_tiles, tiles, part_tok;
+  int w_ring, unit;           // slots of the packed-weight ring; shares are multiples of `unit` K blocks
+  int fusion;
+};
+int i8_block_tc_columns(int64_t m);
+size_t i8_block_tc_partial_bytes(int num_sms, int part_tok);
+cudaError_t launch_i8_block_tc(I8BlockTcParams p, const CUtensorMap& qamap, int num_sms, cudaStream_t stream);
+cudaError_t launch_act_block128_quant(const __nv_bfloat16* x, int64_t ldx, int m, int kc, uint8_t* qa, float* sa,
+                                      int32_t* zpa, float* sat, int n_tok, cudaStream_t stream);
+cudaError_t launch_transpose_scales(const float* sa, int m, int kc, float* sat, int n_tok, cudaStream_t stream);
+cudaError_t launch_btc_pack(const uint8_t* plain, uint8_t* packed, int n, int k, cudaStream_t stream);
+cudaError_t launch_btc_unpack(const uint8_t* packed, uint8_t* plain, int n, int k, cudaStream_t stream);
+cudaError_t launch_btc_pack_scales(const float* scales, const float* zps, float* sw, uint32_t* zw, int n, int groups,
+                                   int* flag, cudaStream_t stream);
+
 // ---- general route: any weight dtype, fp32 / fp16 / bf16 compute, plain layout -----------
 struct GenericParams {
   const uint8_t* w;     // plain [n][row_bytes]: nibbles (even k low) or bytes; kb_per_tile > 0: row layout

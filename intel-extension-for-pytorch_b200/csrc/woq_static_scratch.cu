@@ -22,9 +22,9 @@
 
 namespace {
 
-// 4 MiB covers the split-K scratch of a 16-token call on GPUs with up to 252 SMs
-// (64 KiB header + 16 KiB of partial tiles per SM).
-constexpr size_t kStaticScratchBytes = 4u << 20;
+// 8 MiB covers the split-K scratch of a 16-token call on GPUs with up to 252 SMs (64 KiB header + 16 KiB of
+// partial tiles per SM) and the activation codes of the INT8 routes beside it (16 x K bytes and the scales).
+constexpr size_t kStaticScratchBytes = 8u << 20;
 constexpr int kMaxTokens = 16;
 constexpr int kMaxDevices = 64;
 
