@@ -30,6 +30,7 @@ CUDA_SOURCES = [
     "woq_int8_block.cu",
     "woq_moe.cu",
     "woq_i8_block_tc.cu",
+    "woq_i8_pair.cu",
 ]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -312,14 +312,24 @@ I8BlockWs i8block_ws(const woq_b200_ctx* c, int64_t m) {
 }
 
 int create_generic(const woq_b200_desc* d, const void* qweight, const void* scales, const void* zero_points,
-                   const void* bias, cudaStream_t stream, woq_b200_ctx** out, bool allow_rows);
+                   const void* bias, cudaStream_t stream, woq_b200_ctx** out, int weight_form);
+// how create_generic leaves the weight: a plain copy, the row layout where the layer qualifies, not at all
+enum { kPlainWeight, kRowWeight, kNoWeight };
+cudaError_t keep_plain(woq_b200_ctx* c, const void* qweight, cudaStream_t stream) {
+  c->wq_bytes = static_cast<size_t>(c->desc.n) * c->g_row_bytes;
+  cudaError_t e = cudaMalloc(&c->g_w, c->wq_bytes);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(c->g_w, qweight, c->wq_bytes, cudaMemcpyDeviceToDevice, stream);
+  return e == cudaSuccess ? cudaStreamSynchronize(stream) : e;
+}
 
 // INT4 weights with symmetric activation codes and K blocks of 128 move to the layout of the tcgen05 kernel
 // (one copy of the weight); zero points outside 0..127 keep the layer on the mma.sync kernels.
-cudaError_t move_to_btc(woq_b200_ctx* c, cudaStream_t stream) {
+bool btc_candidate(const woq_b200_desc& d, int kb) {
+  const int64_t g = d.group_size > 0 && d.group_size < d.k ? d.group_size : d.k;
+  return d.weight_dtype == WOQ_B200_DTYPE_INT4 && (d.act_quant_mode & 4) && kb == 128 && (g == d.k || g % 128 == 0);
+}
+cudaError_t move_to_btc(woq_b200_ctx* c, const void* qweight, cudaStream_t stream) {
   const woq_b200_desc& d = c->desc;
-  if (d.weight_dtype != WOQ_B200_DTYPE_INT4 || !(d.act_quant_mode & 4) || c->kb != 128) return cudaSuccess;
-  if (c->g_group < d.k && c->g_group % 128 != 0) return cudaSuccess;
   c->tiles_tc = static_cast<int>((d.n + 127) / 128);
   c->groups = c->g_groups;
   const size_t w_bytes = static_cast<size_t>(c->tiles_tc) * c->kc * 8192;
@@ -337,16 +347,15 @@ cudaError_t move_to_btc(woq_b200_ctx* c, cudaStream_t stream) {
   if (e == cudaSuccess && !bits) {
     woq::count_launch();
     e = cudaMalloc(&c->wq_tc, w_bytes);
-    if (e == cudaSuccess) e = woq::launch_btc_pack(c->g_w, c->wq_tc, (int)d.n, (int)d.k, stream);
+    if (e == cudaSuccess)
+      e = woq::launch_btc_pack(static_cast<const uint8_t*>(qweight), c->wq_tc, (int)d.n, (int)d.k, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e == cudaSuccess) {
       woq::count_launch();
-      cudaFree(c->g_w);
       cudaFree(c->g_scales);
       cudaFree(c->g_zps);
-      c->g_w = nullptr;
       c->g_scales = c->g_zps = nullptr;
-      c->wq_bytes = c->sz_bytes = 0;
+      c->sz_bytes = 0;
       c->wq_tc_bytes = w_bytes;
       c->sz_tc_bytes = 2 * s_bytes;
       c->btc = 1;
@@ -360,6 +369,7 @@ cudaError_t move_to_btc(woq_b200_ctx* c, cudaStream_t stream) {
     c->btc_sw = nullptr;
     c->btc_zw = nullptr;
     c->wq_tc = nullptr;
+    if (e == cudaSuccess) e = keep_plain(c, qweight, stream);
   }
   return e;
 }
@@ -380,7 +390,8 @@ int create_i8block(const woq_b200_desc* d, const void* qweight, const void* scal
   g.lowp_mode = WOQ_B200_LOWP_BF16;
   g.layout_flags |= WOQ_B200_LAYOUT_GENERIC;
   woq_b200_ctx* c = nullptr;
-  if (int rc = create_generic(&g, qweight, scales, zero_points, bias, stream, &c, /*allow_rows=*/false)) return rc;
+  const bool btc = btc_candidate(*d, kb) && (reinterpret_cast<uintptr_t>(qweight) & 3) == 0;
+  if (int rc = create_generic(&g, qweight, scales, zero_points, bias, stream, &c, btc ? kNoWeight : kPlainWeight)) return rc;
   c->desc = *d;
   c->is_generic = 0;
   c->is_i8block = 1;
@@ -399,10 +410,11 @@ int create_i8block(const woq_b200_desc* d, const void* qweight, const void* scal
     }
     woq::count_launch();
   }
-  if (cudaError_t e = move_to_btc(c, stream)) {
-    woq_b200_ctx_destroy(c);
-    return fail(WOQ_B200_ERR_CUDA, "weight layout of the K-block INT8 kernel: %s", cudaGetErrorString(e));
-  }
+  if (btc)
+    if (cudaError_t e = move_to_btc(c, qweight, stream)) {
+      woq_b200_ctx_destroy(c);
+      return fail(WOQ_B200_ERR_CUDA, "weight layout of the K-block INT8 kernel: %s", cudaGetErrorString(e));
+    }
   *out = c;
   return WOQ_B200_OK;
 }
@@ -474,13 +486,16 @@ int run_i8block(const woq_b200_ctx* c, const void* x, int64_t m, int64_t ldx, in
 // INT8 / NF4 weights that the CTA-pair kernel can take (64-aligned K, power-of-two groups of 64 or more, zero
 // points that are INT8 codes) move to its row layout; the general kernel reads that layout too, so there is
 // one copy of the weight.  A layer that does not qualify keeps the plain layout.
-cudaError_t move_to_rows(woq_b200_ctx* c, cudaStream_t stream) {
+bool rows_candidate(const woq_b200_desc& d, const void* qweight) {
+  const int64_t g = d.group_size > 0 && d.group_size < d.k ? d.group_size : d.k;
+  return (d.weight_dtype == WOQ_B200_DTYPE_INT8 || d.weight_dtype == WOQ_B200_DTYPE_NF4) &&
+         d.lowp_mode != WOQ_B200_LOWP_FP16 && d.k % 64 == 0 && (g == d.k || (g % 64 == 0 && (g & (g - 1)) == 0)) &&
+         (reinterpret_cast<uintptr_t>(qweight) & 3) == 0;
+}
+cudaError_t move_to_rows(woq_b200_ctx* c, const void* qweight, cudaStream_t stream) {
   const woq_b200_desc& d = c->desc;
   const bool int8 = d.weight_dtype == WOQ_B200_DTYPE_INT8;
-  if (!int8 && d.weight_dtype != WOQ_B200_DTYPE_NF4) return cudaSuccess;
-  if (d.lowp_mode == WOQ_B200_LOWP_FP16 || d.k % 64 != 0) return cudaSuccess;
   const int64_t g = c->g_group;
-  if (g < d.k && (g % 64 != 0 || (g & (g - 1)) != 0)) return cudaSuccess;
   c->tiles_tc = static_cast<int>((d.n + 127) / 128);
   c->kb_per_tile = static_cast<int>(d.k / 64);
   c->groups = c->g_groups;
@@ -502,13 +517,11 @@ cudaError_t move_to_rows(woq_b200_ctx* c, cudaStream_t stream) {
   if (e == cudaSuccess && !(bits & 1)) {
     woq::count_launch();
     e = cudaMalloc(&c->wq_tc, w_bytes);
-    if (e == cudaSuccess) e = woq::launch_pack_rows(c->g_w, c->wq_tc, (int)d.n, (int)d.k, int8, stream);
+    if (e == cudaSuccess)
+      e = woq::launch_pack_rows(static_cast<const uint8_t*>(qweight), c->wq_tc, (int)d.n, (int)d.k, int8, stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     if (e == cudaSuccess) {
       woq::count_launch();
-      cudaFree(c->g_w);
-      c->g_w = nullptr;
-      c->wq_bytes = 0;
       c->wq_tc_bytes = w_bytes;
       c->sz_tc_bytes = s_bytes;
       c->plain_scales = (bits & 2) ? 0 : 1;
@@ -521,12 +534,13 @@ cudaError_t move_to_rows(woq_b200_ctx* c, cudaStream_t stream) {
     cudaFree(c->wq_tc);
     c->sz_tc = nullptr;
     c->wq_tc = nullptr;
+    if (e == cudaSuccess) e = keep_plain(c, qweight, stream);
   }
   return e;
 }
 
 int create_generic(const woq_b200_desc* d, const void* qweight, const void* scales, const void* zero_points,
-                   const void* bias, cudaStream_t stream, woq_b200_ctx** out, bool allow_rows) {
+                   const void* bias, cudaStream_t stream, woq_b200_ctx** out, int weight_form) {
   if (d->lowp_mode == WOQ_B200_LOWP_INT8)
     return fail(WOQ_B200_ERR_UNSUPPORTED, "the general route computes in fp32 / fp16 / bf16, not INT8");
   if (d->weight_format != WOQ_B200_FMT_PLAIN)
@@ -564,12 +578,9 @@ int create_generic(const woq_b200_desc* d, const void* qweight, const void* scal
   } while (0)
   CUDA_TRY_G(cudaGetDevice(&c->device));
   CUDA_TRY_G(cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, c->device));
-  c->wq_bytes = static_cast<size_t>(d->n) * c->g_row_bytes;
   const int64_t sg = d->n * c->g_groups;
   c->sz_bytes = static_cast<size_t>(sg) * sizeof(float) * (zero_points ? 2 : 1);
-  CUDA_TRY_G(cudaMalloc(&c->g_w, c->wq_bytes));
   CUDA_TRY_G(cudaMalloc(&c->g_scales, sg * sizeof(float)));
-  CUDA_TRY_G(cudaMemcpyAsync(c->g_w, qweight, c->wq_bytes, cudaMemcpyDeviceToDevice, stream));
   to_f32_kernel<<<static_cast<unsigned>((sg + 255) / 256), 256, 0, stream>>>(scales, c->g_scales, sg, d->scale_dtype);
   woq::count_launch();
   if (zero_points) {
@@ -585,8 +596,12 @@ int create_generic(const woq_b200_desc* d, const void* qweight, const void* scal
     woq::count_launch();
   }
   CUDA_TRY_G(cudaGetLastError());
-  CUDA_TRY_G(cudaStreamSynchronize(stream));
-  if (allow_rows) CUDA_TRY_G(move_to_rows(c, stream));
+  if (weight_form == kRowWeight && rows_candidate(*d, qweight))
+    CUDA_TRY_G(move_to_rows(c, qweight, stream));
+  else if (weight_form != kNoWeight)
+    CUDA_TRY_G(keep_plain(c, qweight, stream));
+  else
+    CUDA_TRY_G(cudaStreamSynchronize(stream));
 #undef CUDA_TRY_G
   c->magic = kMagic;
   *out = c;
@@ -663,7 +678,7 @@ int woq_b200_ctx_create(const woq_b200_desc* d, const void* qweight, const void*
     return fail(WOQ_B200_ERR_INVALID_ARG, "scales must be fp32, fp16 or bf16");
 
   if (wants_i8block(d)) return create_i8block(d, qweight, scales, zero_points, bias, stream, out);
-  if (wants_generic(d)) return create_generic(d, qweight, scales, zero_points, bias, stream, out, /*allow_rows=*/true);
+  if (wants_generic(d)) return create_generic(d, qweight, scales, zero_points, bias, stream, out, kRowWeight);
   if (d->weight_dtype == WOQ_B200_DTYPE_INT8) return create_int8(d, qweight, scales, zero_points, bias, stream, out);
   // ---- INT4 ----
   if (d->k % 64 != 0)
@@ -1023,6 +1038,20 @@ static int make_kblock_map(CUtensorMap* map, const void* base, int64_t rows, int
   return WOQ_B200_OK;
 }
 
+// INT8 operand images [tiles64][k-chunks][64 rows][128 bytes]: one box is a k-chunk of 128 rows.
+static int make_image_map(CUtensorMap* map, const void* base, int64_t tiles64, int64_t kc) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return fail(WOQ_B200_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+  cuuint64_t dims[3] = {128, static_cast<cuuint64_t>(kc) * 64, static_cast<cuuint64_t>(tiles64)};
+  cuuint64_t strides[2] = {128, static_cast<cuuint64_t>(kc) * 8192};
+  cuuint32_t box[3] = {128, 64, 2}, estr[3] = {1, 1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(base), dims, strides, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(WOQ_B200_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
+  return WOQ_B200_OK;
+}
+
 extern "C++" {
 namespace {
 int run_i8block_tc(const woq_b200_ctx* c, const I8BlockWs& L, const __nv_bfloat16* x, int64_t m, int64_t ldx,
@@ -1290,50 +1319,45 @@ static int run_tc(const woq_b200_ctx* c, const void* x, int64_t m, int64_t ldx, 
   return WOQ_B200_OK;
 }
 
-// The tcgen05 int8 kernel, 256 tokens per launch, on activations that are already quantised:
-// codes qa [m, K], scales sa [m], zero points zpa [m] (null for the symmetric modes).
+// The INT8 kernel on activations that are already quantised: codes qa [m, K], scales sa [m], zero points zpa [m]
+// (null for the symmetric modes).
 static int run_int8_gemm(const woq_b200_ctx* c, const int8_t* qa, const float* sa, const int32_t* zpa, int64_t m,
                          int32_t fusion, const void* o0, const void* o1, void* y, int64_t ldy, int32_t* acc_out,
                          uint8_t* w8, size_t partial_off, cudaStream_t stream) {
-  const int64_t k = c->desc.k;
-  const int64_t mt = m < 256 ? m : 256;
-  const int n_tok = static_cast<int>((mt + 15) / 16 * 16);
-  CUtensorMap qamap;
-  if (int rc = make_kmajor_map(&qamap, qa, m, k, k, 1, n_tok)) return rc;
-  for (int64_t m0 = 0; m0 < m; m0 += 256) {
-    const int64_t mm = m - m0 < 256 ? m - m0 : 256;
-    woq::I8Params p{};
-    p.wq = reinterpret_cast<const int8_t*>(c->wq);
-    p.sw = c->scale_f32;
-    p.sa = sa + m0;
-    p.zpa = zpa ? zpa + m0 : nullptr;
-    p.comp = c->comp;
-    p.bias = c->bias;
-    p.y = y ? static_cast<__nv_bfloat16*>(y) + m0 * ldy : nullptr;
-    p.other0 = o0 ? static_cast<const __nv_bfloat16*>(o0) + m0 * ldy : nullptr;
-    p.other1 = o1 ? static_cast<const __nv_bfloat16*>(o1) + m0 * ldy : nullptr;
-    p.acc_out = acc_out ? acc_out + m0 * c->desc.n : nullptr;
-    p.status = reinterpret_cast<int*>(w8);
-    p.counters = reinterpret_cast<uint32_t*>(w8 + 256);
-    p.partials = w8 + partial_off;
-    p.ldy = ldy;
-    p.m = (int)mm;
-    p.n = (int)c->desc.n;
-    p.n_out = fusion == WOQ_B200_FUSE_SILU_MUL ? (int)(c->desc.n / 2) : (int)c->desc.n;
-    p.m0 = (int)m0;
-    p.n_tok = n_tok;
-    p.tiles = c->tiles_tc;
-    p.kc_per_tile = c->kc_per_tile;
-    p.fusion = fusion;
-    p.gate_up = c->gate_up;
-    const int64_t total = static_cast<int64_t>(c->tiles_tc) * c->kc_per_tile;
-    const int grid = static_cast<int>(total < c->num_sms ? total : c->num_sms);
-    CUDA_TRY(woq::launch_int8_tc(p, qamap, grid, stream));
-  }
+  woq::I8PairParams p{};
+  p.sw = c->scale_f32;
+  p.sa = sa;
+  p.zpa = zpa;
+  p.comp = c->comp;
+  p.bias = c->bias;
+  p.y = static_cast<__nv_bfloat16*>(y);
+  p.other0 = static_cast<const __nv_bfloat16*>(o0);
+  p.other1 = static_cast<const __nv_bfloat16*>(o1);
+  p.acc_out = acc_out;
+  p.partials = reinterpret_cast<int*>(w8 + partial_off);
+  p.counters = reinterpret_cast<uint32_t*>(w8 + 256);
+  p.status = reinterpret_cast<int*>(w8);
+  p.ldy = ldy;
+  p.m = (int)m;
+  p.n = (int)c->desc.n;
+  p.n_out = fusion == WOQ_B200_FUSE_SILU_MUL ? (int)(c->desc.n / 2) : (int)c->desc.n;
+  woq::pair_token_tiles(m, &p.n_tok, &p.tok_tiles);
+  p.part_tok = m < p.n_tok ? (int)m : p.n_tok;
+  p.tiles = c->tiles_tc;
+  p.w_tiles = (c->tiles_tc + 1) / 2;
+  p.kc_per_tile = c->kc_per_tile;
+  p.fusion = fusion;
+  p.gate_up = c->gate_up;
+  p.vec = ldy % 8 == 0 && aligned16(y) && (!o0 || aligned16(o0)) && (!o1 || aligned16(o1));
+  CUtensorMap wmap, qamap;
+  if (int rc = make_image_map(&wmap, c->wq, c->tiles_tc * 2, c->kc_per_tile)) return rc;
+  if (int rc = make_kblock_map(&qamap, qa, m, c->desc.k, c->desc.k, 1, p.n_tok / 2, 1)) return rc;
+  CUDA_TRY(woq::launch_i8_pair(p, wmap, qamap, c->num_sms, stream));
+  woq::count_launch();
   return WOQ_B200_OK;
 }
 
-// INT8 compute: quantise the activations per token, then the tcgen05 int8 kernel per 256 tokens
+// INT8 compute: quantise the activations per token, then the tensor-core kernel
 static int run_int8(const woq_b200_ctx* c, const void* x, int64_t m, int64_t ldx, int32_t fusion,
                     const void* o0, const void* o1, void* y, int64_t ldy, int8_t* qa_out, float* sa_out,
                     int32_t* acc_out, void* ws, size_t ws_bytes, cudaStream_t stream) {

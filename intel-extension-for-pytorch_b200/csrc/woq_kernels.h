@@ -224,6 +224,30 @@ struct I8Params {
   int tiles, kc_per_tile;  // 128-row tiles, 128-k chunks
   int stages, fusion, gate_up;
 };
+// the same on CTA pairs (woq_i8_pair.cu)
+struct I8PairParams {
+  const float* sw;      // per-channel weight scales [n_pad]
+  const float* sa;      // per-token activation scales [m]
+  const int32_t* zpa;   // per-token activation zero points [m] (asymmetric codes are u8), or null
+  const int32_t* comp;  // with zpa: per-row sums of the weight codes [n_pad]
+  const float* bias;
+  __nv_bfloat16* y;     // may be null when only the accumulators are wanted
+  const __nv_bfloat16* other0;
+  const __nv_bfloat16* other1;
+  int* acc_out;         // optional [m][n] int32 accumulators
+  int* partials;        // [CTAs][2][part_tok][128]
+  uint32_t* counters;   // [CTAs], zero between calls
+  int* status;
+  int64_t ldy;
+  int m, n, n_out;
+  int n_tok, tok_tiles;  // as pair_token_tiles
+  int tiles, w_tiles;    // 128-row tiles; pairs of them (rounded up)
+  int kc_per_tile, part_tok, stages, fusion, gate_up;
+  int vec;  // y and the extra operands can be accessed 16 bytes at a time
+};
+size_t i8_pair_partial_bytes(int num_sms, int part_tok);
+cudaError_t launch_i8_pair(I8PairParams p, const CUtensorMap& wmap, const CUtensorMap& qamap, int num_sms,
+                           cudaStream_t stream);
 cudaError_t launch_pack_int8(const int8_t* plain, int8_t* tiled, int n, int k, int tiles64,
                              int gate_up, cudaStream_t stream);
 cudaError_t launch_unpack_int8(const int8_t* tiled, int8_t* plain, int n, int k, int gate_up,
