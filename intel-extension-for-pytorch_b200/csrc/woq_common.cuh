@@ -104,19 +104,27 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
                "r"(bytes)
                : "memory");
 }
+// IDLE: the wait is expected to be long and nothing hurries after it; the warp may stay suspended for 10 us per
+// test instead of polling every few dozen cycles beside the warps that work.
+template <bool IDLE = false>
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-#ifdef WOQ_USE_TEST_WAIT
-      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-#else
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-#endif
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
+  if (IDLE)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(10000u)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
   return ok != 0;
 }
 __device__ __forceinline__ uint64_t global_timer_ns() {
@@ -132,13 +140,14 @@ __device__ __forceinline__ uint64_t global_timer_ns() {
 // case (the barrier flips within a few polls) costs nothing beyond the polls themselves.
 constexpr long long kWaitLimitCycles = 4000000000ll;  // about 2 s
 
+template <bool IDLE = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           int* status, int code) {
-  if (mbar_test(bar, parity)) return true;
+  if (mbar_test<IDLE>(bar, parity)) return true;
   uint32_t spins = 0;
   long long t0 = 0;
-  while (!mbar_test(bar, parity)) {
-    if ((++spins & 1023u) == 0) {
+  while (!mbar_test<IDLE>(bar, parity)) {
+    if ((++spins & (IDLE ? 63u : 1023u)) == 0) {
       if (*abort_flag) return false;
       const long long now = clock64();
       if (t0 == 0) {

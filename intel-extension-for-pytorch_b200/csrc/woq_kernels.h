@@ -185,7 +185,7 @@ struct PairParams {
   int n_tok;                    // token columns of a tile (a multiple of 32, <= 256)
   int tiles, w_tiles;           // 128-row tiles; pairs of them (rounded up)
   int kb_per_tile, kbpg_shift, groups;
-  int kbs, stages, w_ring;      // k-blocks per stage; slots of the two rings
+  int kbs, kpw, stages, w_ring; // k-blocks per stage, and of them per warpgroup; slots of the two rings
   int unit;                     // shares are multiples of this many k-blocks
   int fusion, gate_up;
   int kind;      // WeightKind

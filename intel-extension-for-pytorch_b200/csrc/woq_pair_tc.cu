@@ -26,7 +26,7 @@
 // What bounds it: at 256 token columns the tensor cores under the power limit (57344 x 8192, 512
 // tokens: 339 us, 1420 TFLOP/s, against 501 us for one CTA per tile and 256 tokens per launch); at 32
 // columns the dequantiser's issue slots and the hand-overs between roles (91 us, 2.7 TB/s of weights,
-// was 125 us).  A lone thread beside sixteen dequantising warps gets an instruction issued every ten
+// was 125 us; 72 us with two k-blocks per visit and idle warps suspended).  A lone thread beside sixteen dequantising warps gets an instruction issued every ten
 // cycles or so, so the roles' work per stage is what has to be small: one activation copy per stage,
 // several k-blocks per stage, no wait or fence that is not needed.
 //
@@ -157,7 +157,7 @@ __device__ __forceinline__ void pair_dequant(const uint8_t* ws, int row, uint32_
   if (KIND == kWeightNf4) pair_dequant_nf4(ws, row, szw, lut_lane, r);
 }
 
-template <int KIND>
+template <int KIND, int KPW>
 __global__ void __launch_bounds__(kPairThreads, 1)
     woq_pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtensorMap xmap) {
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -191,12 +191,12 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 
   if (tid == 0) {
     for (int s = 0; s < n_stages; ++s) {
-      mbar_init(&hdr->full[s], 8 * kbs + 1);  // four warps per k-block and CTA, the leader's x producer
+      mbar_init(&hdr->full[s], 8 * kbs / KPW + 1);  // the dequantising warps of both CTAs, the leader's x producer
       mbar_init(&hdr->free_[s], 1);
     }
     for (int s = 0; s < n_wring; ++s) {
       mbar_init(&hdr->w_full[s], 1);
-      mbar_init(&hdr->w_free[s], 4 * kbs);
+      mbar_init(&hdr->w_free[s], 4 * kbs / KPW);
     }
     mbar_init(&hdr->d_full, 1);
     mbar_init(&hdr->d_empty, 2 * kEpiWarps);
@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
           uint8_t* ws = w_stages + static_cast<size_t>(wslot) * w_stage_bytes;
           const int g0 = kb0 >> p.kbpg_shift;
           const int ng = ((kb0 + nkb - 1) >> p.kbpg_shift) - g0 + 1;
-          mbar_wait(&hdr->w_free[wslot], wphase ^ 1, abort_flag, p.status, 31);
+          mbar_wait<true>(&hdr->w_free[wslot], wphase ^ 1, abort_flag, p.status, 31);
           mbar_arrive_expect_tx(&hdr->w_full[wslot], nkb * kBlock + ng * 512);
           bulk_g2s(ws, wsrc, nkb * kBlock, &hdr->w_full[wslot]);
           bulk_g2s(ws + kbs * kBlock, ssrc + static_cast<size_t>(g0) * kTcTileN, ng * 512, &hdr->w_full[wslot]);
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
         int seg = kbpt - kb0 < rem ? kbpt - kb0 : rem;
         rem -= seg;
         for (; seg > 0; seg -= kbs) {
-          mbar_wait(&hdr->free_[slot], phase ^ 1, abort_flag, p.status, 32);
+          mbar_wait<true>(&hdr->free_[slot], phase ^ 1, abort_flag, p.status, 32);
           if (rank == 0) mbar_arrive_expect_tx(&hdr->full[slot], 2 * x_stage_bytes);
           pair_tma_load_3d(x_stages + slot * x_stage_bytes, &xmap, 0, row, kb0, full0 + slot * 8);
           kb0 += kbs;
@@ -325,16 +325,16 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       }
     }
   } else if (warp >= kDeqWarp0) {
-    // ---- dequantise: one k-block of a stage per warpgroup.  Stages of four k-blocks involve all four
-    // ---- warpgroups, stages of two alternate between two halves of them. ----
+    // ---- dequantise: KPW neighbouring k-blocks of a stage per warpgroup, so kbs / KPW warpgroups share a
+    // ---- stage and each takes every step-th one ----
     const int wg = (warp - kDeqWarp0) >> 2, q = warp & 3;
     const int row = q * 32 + lane;
-    const int step = kDeqGroups / kbs;  // 1 or 2
-    const int j = wg & (kbs - 1);       // k-block within the stage
-    const uint32_t a_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + p.n_tok + j * 32;
+    const int wgs = kbs / KPW, step = kDeqGroups / wgs;
+    const int j0 = wg % wgs * KPW;  // first k-block within the stage
+    const uint32_t a_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + p.n_tok + j0 * 32;
     const uint32_t full0 = pair_map(&hdr->full[0], 0);
     int kb_seg = kb00, rem = rem0;
-    int own = wg / kbs, slot = own, wslot = own;  // `own`: this warpgroup's next stage, counted over all segments
+    int own = wg / wgs, slot = own, wslot = own;  // `own`: this warpgroup's next stage, counted over all segments
     int st = 0;
     uint32_t phase = 0, wphase = 0;
     while (rem > 0) {
@@ -343,24 +343,31 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       for (; own < st + ns; own += step) {
         const int in_seg = (own - st) * kbs;   // k-blocks of the segment before this stage
         const int kb0 = kb_seg + in_seg;
-        const bool some = in_seg + j < seg_len;  // false: the stage was cut short before this k-block
+        const int nj = seg_len - in_seg - j0;  // below KPW where the stage was cut short
         const uint8_t* ws = w_stages + wslot * w_stage_bytes;
+        const uint32_t a_slot = a_lane + slot * (kbs * 32);
         mbar_wait(&hdr->w_full[wslot], wphase, abort_flag, p.status, 35);
-        uint32_t r[32];
-        if (some) {
-          const int gl = ((kb0 + j) >> p.kbpg_shift) - (kb0 >> p.kbpg_shift);
-          const uint32_t szw = reinterpret_cast<const uint32_t*>(ws + kbs * kBlock)[gl * kTcTileN + row];
-          pair_dequant<KIND>(ws + j * kBlock, row, szw, lut + lane * 4, r);
+        const int g0 = kb0 >> p.kbpg_shift;
+#pragma unroll
+        for (int j = 0; j < KPW; ++j) {
+          uint32_t r[32];
+          if (j < nj) {
+            const int gl = ((kb0 + j0 + j) >> p.kbpg_shift) - g0;
+            const uint32_t szw = reinterpret_cast<const uint32_t*>(ws + kbs * kBlock)[gl * kTcTileN + row];
+            pair_dequant<KIND>(ws + (j0 + j) * kBlock, row, szw, lut + lane * 4, r);
+          }
+          if (j == KPW - 1) {
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&hdr->w_free[wslot]);
+          }
+          if (j == 0) {
+            mbar_wait(&hdr->free_[slot], phase ^ 1, abort_flag, p.status, 36);
+            tc_fence_after_sync();
+            __syncwarp();  // the TMEM store is a warp-wide instruction
+          }
+          if (j < nj) tmem_st_x32(a_slot + j * 32, r);
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&hdr->w_free[wslot]);
-        mbar_wait(&hdr->free_[slot], phase ^ 1, abort_flag, p.status, 36);
-        tc_fence_after_sync();
-        __syncwarp();  // the TMEM store is a warp-wide instruction
-        if (some) {
-          tmem_st_x32(a_lane + slot * (kbs * 32), r);
-          tc_wait_st();
-        }
+        if (nj > 0) tc_wait_st();
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) pair_arrive(full0 + slot * 8);
@@ -415,7 +422,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       }
       // the bf16 tile of the previous segment has been copied out by everybody
       named_bar_sync(kEpiBar, kEpiThreads);
-      mbar_wait(&hdr->d_full, seg_no & 1, abort_flag, p.status, 37);
+      mbar_wait<true>(&hdr->d_full, seg_no & 1, abort_flag, p.status, 37);
       tc_fence_after_sync();
       __syncwarp();
       bool finish = whole && real;
@@ -554,17 +561,24 @@ int pair_group_columns(const int64_t* rows, int groups) {
 // Pipeline shape for p.n_tok token columns; returns the dynamic shared memory in bytes.
 //   k-blocks per stage: four up to 128 columns, two above.  Every stage costs each single-thread role
 //     300-400 cycles of waiting, issuing and bookkeeping beside the busy dequantising warps, whatever
-//     the stage holds; a k-block's MMAs take 2 x n_tok cycles.
+//     the stage holds; a k-block's MMAs take at least 64 cycles, 4 x n_tok / 2 when that is more.
+//   k-blocks per warpgroup and visit: two up to 128 columns, so that the two waits, the store's completion
+//     and the arrival (600 of 1490 cycles, most of it latency) come once per two k-blocks.  57344 x 8192 INT4,
+//     32 / 64 / 128 tokens: 80 / 83 / 105 us with one, 72 / 77 / 101 with two; 57344 x 4096 INT8, 8 tokens:
+//     46 and 44 us.  (Stages of two with one warpgroup each: 89 / 92 / 110 us.)  At 128 columns of 8-bit
+//     weights only three weight slots fit, too few for that: 68 us with one, 73 with two.
 //   Rings: a parity wait cannot tell a barrier that is one completion short from one that is three
-//     short, so whoever waits for use u of a slot must know that use u - 1 has completed.  With stages
-//     of four k-blocks every warpgroup waits for every use of every slot.  With stages of two a
-//     warpgroup sees every second stage: an even weight ring gives each slot to one pair of
-//     warpgroups, and on the A / activation ring the wait for stage s - 2 (the MMAs of stage
-//     s - 2 - stages, which complete in order) covers stage s - 2 * stages.
+//     short, so whoever waits for use u of a slot must know that use u - 1 has completed.  A warpgroup sees
+//     every step-th stage (step = 4 kpw / kbs: 1 or 2).  A weight ring that is a multiple of step gives each
+//     slot to the same warpgroups every time; on the A / activation ring the wait for stage s - step (the
+//     MMAs of stage s - step - stages, which complete in order) covers stage s - 2 * stages when there are
+//     at least step stages.
 size_t pair_plan(PairParams& p) {
   const int lut = p.kind == kWeightNf4 ? kNf4LutBytes : 0;
   const int budget = 227 * 1024 - kPairHeaderBytes - lut - p.n_tok * kOutPitch;
   p.kbs = p.n_tok <= 128 ? 4 : 2;
+  p.kpw = p.kbs == 4 && (p.n_tok < 128 || pair_block_bytes(p.kind) == kTcBlockBytes) ? 2 : 1;
+  const int step = kDeqGroups * p.kpw / p.kbs;
   const int x_stage = p.kbs * (p.n_tok / 2) * 128;
   const int w_stage = p.kbs * (pair_block_bytes(p.kind) + 512);
   int stages = (kPairTmemCols - p.n_tok) / 32 / p.kbs;
@@ -574,7 +588,7 @@ size_t pair_plan(PairParams& p) {
   while (stages > 2 && budget - stages * x_stage < min_ring * w_stage) --stages;
   int ring = (budget - stages * x_stage) / w_stage;
   if (ring > kMaxPairWRing) ring = kMaxPairWRing;
-  if (p.kbs == 2) ring &= ~1;
+  ring -= ring % step;
   if (stages < 2 || ring < 2) return 0;
   p.stages = stages;
   p.w_ring = ring;
@@ -601,12 +615,13 @@ cudaError_t launch_pair(PairParams p, const CUtensorMap& xmap, int num_sms, cuda
   const size_t smem = pair_plan(p);
   if (smem == 0) return cudaErrorInvalidConfiguration;
   void (*kern)(const PairParams, const CUtensorMap) = nullptr;
+  const bool two = p.kpw == 2;
   switch (p.kind) {
-    case kWeightInt4InPlace: kern = woq_pair_kernel<kWeightInt4InPlace>; break;
-    case kWeightInt4: kern = woq_pair_kernel<kWeightInt4>; break;
-    case kWeightInt8InPlace: kern = woq_pair_kernel<kWeightInt8InPlace>; break;
-    case kWeightInt8: kern = woq_pair_kernel<kWeightInt8>; break;
-    case kWeightNf4: kern = woq_pair_kernel<kWeightNf4>; break;
+    case kWeightInt4InPlace: kern = two ? woq_pair_kernel<kWeightInt4InPlace, 2> : woq_pair_kernel<kWeightInt4InPlace, 1>; break;
+    case kWeightInt4: kern = two ? woq_pair_kernel<kWeightInt4, 2> : woq_pair_kernel<kWeightInt4, 1>; break;
+    case kWeightInt8InPlace: kern = two ? woq_pair_kernel<kWeightInt8InPlace, 2> : woq_pair_kernel<kWeightInt8InPlace, 1>; break;
+    case kWeightInt8: kern = two ? woq_pair_kernel<kWeightInt8, 2> : woq_pair_kernel<kWeightInt8, 1>; break;
+    case kWeightNf4: kern = two ? woq_pair_kernel<kWeightNf4, 2> : woq_pair_kernel<kWeightNf4, 1>; break;
     default: return cudaErrorInvalidValue;
   }
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
