@@ -1152,8 +1152,10 @@ static int run_pair(const woq_b200_ctx* c, const void* x, int64_t m, int64_t ldx
                     cudaStream_t stream) {
   woq::PairParams p{};
   fill_pair(c, &p, w8);
-  int tok_tiles;
-  woq::pair_token_tiles(m, &p.n_tok, &tok_tiles);
+  const woq::PairCut cut = woq::pair_cut(m, p.w_tiles, p.kb_per_tile, c->num_sms / 2, p.kind);
+  p.n_tok = cut.n_tok;
+  p.whole = cut.whole;
+  p.split = cut.split;
   add_pair_group(c, &p, 0, m, y);
   p.other0 = static_cast<const __nv_bfloat16*>(o0);
   p.other1 = static_cast<const __nv_bfloat16*>(o1);
@@ -1341,11 +1343,15 @@ static int run_int8_gemm(const woq_b200_ctx* c, const int8_t* qa, const float* s
   p.m = (int)m;
   p.n = (int)c->desc.n;
   p.n_out = fusion == WOQ_B200_FUSE_SILU_MUL ? (int)(c->desc.n / 2) : (int)c->desc.n;
-  woq::pair_token_tiles(m, &p.n_tok, &p.tok_tiles);
-  p.part_tok = m < p.n_tok ? (int)m : p.n_tok;
   p.tiles = c->tiles_tc;
   p.w_tiles = (c->tiles_tc + 1) / 2;
   p.kc_per_tile = c->kc_per_tile;
+  const woq::PairCut cut = woq::pair_cut(m, p.w_tiles, p.kc_per_tile, c->num_sms / 2, woq::kPairCutInt8);
+  p.n_tok = cut.n_tok;
+  p.tok_tiles = cut.tok_tiles;
+  p.unit = cut.whole ? p.kc_per_tile : 1;
+  p.split = cut.split;
+  p.part_tok = m < p.n_tok ? (int)m : p.n_tok;
   p.fusion = fusion;
   p.gate_up = c->gate_up;
   p.vec = ldy % 8 == 0 && aligned16(y) && (!o0 || aligned16(o0)) && (!o1 || aligned16(o1));

@@ -14,6 +14,9 @@
 //   warps 4-11  epilogue: int32 -> scales, bias -> bf16 tile of 64 tokens in shared memory -> post-op -> y.  Two
 //               accumulator buffers, so the next tile's MMAs run meanwhile.
 //
+// SPLIT: few tiles; the p.split pairs of a tile form a cluster, take a part of k each and add their int32
+// accumulators over distributed shared memory (as in woq_pair_tc.cu).
+//
 // What bounds it: with 256 columns the tensor cores (16 KB weights + 16 KB codes per SM and 512 cycles of MMAs;
 // one CTA per tile and launch of 256 tokens moved 48 KB); with few columns the weights' HBM traffic.
 #include "woq_pair_epilogue.cuh"
@@ -54,6 +57,15 @@ __device__ __forceinline__ void pair_mma_i8_ss(uint32_t d_tmem, uint64_t a_desc,
       : "memory");
 }
 
+// bias + (float(acc - compensation * zp) * scale_a) * scale_w, the integer part exact
+// (csrc/cpu/aten/utils/woq.h:2310-2321)
+__device__ __forceinline__ __nv_bfloat16 ip_result(int acc, int comp, int zp, float sa, float sw, const float* bias, float b) {
+  float f = (static_cast<float>(acc - comp * zp) * sa) * sw;
+  if (bias) f = b + f;
+  return __float2bfloat16_rn(f);
+}
+
+template <bool SPLIT>
 __global__ void __launch_bounds__(kIpThreads, 1)
     woq_i8_pair_kernel(const __grid_constant__ I8PairParams p, const __grid_constant__ CUtensorMap wmap,
                        const __grid_constant__ CUtensorMap qamap) {
@@ -71,13 +83,23 @@ __global__ void __launch_bounds__(kIpThreads, 1)
   uint8_t* b_stages = a_stages + n_stages * kIpABytes;
   uint8_t* out_tile = b_stages + n_stages * b_bytes;
 
-  const uint32_t rank = pair_cta_rank();
+  const uint32_t crank = pair_cta_rank(), rank = crank & 1, leader = crank - rank;  // rank in cluster / pair
+  const uint16_t pair_mask = static_cast<uint16_t>(3u << leader);
   const int pair = blockIdx.x >> 1, kcpt = p.kc_per_tile;
-  const int64_t pairs = gridDim.x >> 1, total = static_cast<int64_t>(p.w_tiles) * p.tok_tiles * kcpt;
-  const int64_t b_begin = pair * total / pairs, b_end = (pair + 1) * total / pairs;
-  const int item0 = static_cast<int>(b_begin / kcpt);  // item = weight tile * tok_tiles + token tile
-  const int kc00 = static_cast<int>(b_begin % kcpt);
-  const int rem0 = static_cast<int>(b_end - b_begin);
+  // shares are dealt in units of p.unit chunks
+  const int64_t pairs = gridDim.x >> 1, total = static_cast<int64_t>(p.w_tiles) * p.tok_tiles * kcpt / p.unit;
+  int item0, kc00, rem0;  // item = weight tile * tok_tiles + token tile
+  if (SPLIT) {
+    const int sub = crank >> 1;
+    item0 = pair / p.split;
+    kc00 = sub * kcpt / p.split;
+    rem0 = (sub + 1) * kcpt / p.split - kc00;
+  } else {
+    const int64_t b_begin = pair * total / pairs * p.unit, b_end = (pair + 1) * total / pairs * p.unit;
+    item0 = static_cast<int>(b_begin / kcpt);
+    kc00 = static_cast<int>(b_begin % kcpt);
+    rem0 = static_cast<int>(b_end - b_begin);
+  }
 
   if (tid == 0) {
     for (int s = 0; s < n_stages; ++s) {
@@ -108,7 +130,7 @@ __global__ void __launch_bounds__(kIpThreads, 1)
       if (warp == 1) grid_dependency_wait();  // the quantiser's codes
       int item = item0, kc = kc00, rem = rem0, slot = 0;
       uint32_t phase = 0;
-      const uint32_t full0 = pair_map(&hdr->full[0], 0);
+      const uint32_t full0 = pair_map(&hdr->full[0], leader);
       while (rem > 0) {
         int tile = item / p.tok_tiles * 2 + static_cast<int>(rank);
         if (tile >= p.tiles) tile = p.tiles - 1;  // odd tile count: the last pair's second half repeats it
@@ -158,8 +180,8 @@ __global__ void __launch_bounds__(kIpThreads, 1)
               pair_mma_i8_ss(tmem_base + buf * p.n_tok, a + ks * 2, b + ks * 2, idesc, accumulate);
               accumulate = 1;
             }
-            pair_commit(&hdr->free_[slot]);
-            if (seg == 1) pair_commit(&hdr->d_full[buf]);
+            pair_commit(&hdr->free_[slot], pair_mask);
+            if (seg == 1) pair_commit(&hdr->d_full[buf], pair_mask);
           }
           __syncwarp();
           accumulate = 1;
@@ -182,7 +204,7 @@ __global__ void __launch_bounds__(kIpThreads, 1)
       const bool whole = seg_len == kcpt;
       const uint32_t buf = seg_no & 1;
       const uint32_t d_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * p.n_tok;
-      const uint32_t d_empty0 = pair_map(&hdr->d_empty[buf], 0);
+      const uint32_t d_empty0 = pair_map(&hdr->d_empty[buf], leader);
       const int tile = item / p.tok_tiles * 2 + static_cast<int>(rank);
       const int tok0 = item % p.tok_tiles * p.n_tok;
       const int mv = p.m - tok0 < p.n_tok ? p.m - tok0 : p.n_tok;
@@ -199,6 +221,17 @@ __global__ void __launch_bounds__(kIpThreads, 1)
       mbar_wait(&hdr->d_full[buf], (seg_no >> 1) & 1, abort_flag, p.status, 55);
       tc_fence_after_sync();
       __syncwarp();
+      if (SPLIT) {  // this pair's part of the tile, for the CTAs that add it up
+        int* part = reinterpret_cast<int*>(a_stages) + row;
+        for (int c0 = eg * 16; c0 < mv; c0 += 32) {
+          uint32_t t[16];
+          tmem_ld_x16(d_lane + c0, t);
+          tc_wait_ld();
+#pragma unroll
+          for (int e = 0; e < 16; ++e) part[(c0 + e) * kTcTileN] = static_cast<int>(t[e]);
+        }
+        break;
+      }
       auto accumulators_read = [&]() {
         tc_fence_before_sync();
         __syncwarp();
@@ -206,7 +239,7 @@ __global__ void __launch_bounds__(kIpThreads, 1)
       };
       bool finish = whole && real, from_tmem = finish;
       int c_first = pair, c_last = pair;
-      const int64_t tb0 = static_cast<int64_t>(item) * kcpt;  // the tile's first chunk
+      const int64_t tb0 = static_cast<int64_t>(item) * kcpt;  // the tile's first chunk (units of one where tiles are shared)
       auto slot_of = [&](int c) {  // partial tile of pair c, this CTA's rows
         const int s = (c == c_first && c * total / pairs < tb0) ? 1 : 0;
         return p.partials + static_cast<size_t>((c * 2 + static_cast<int>(rank)) * 2 + s) * p.part_tok * kTcTileN + row;
@@ -269,30 +302,31 @@ __global__ void __launch_bounds__(kIpThreads, 1)
 #pragma unroll
               for (int e = 0; e < 16; ++e) v[e] = 0;
             }
+            // three parts in flight together: a round trip to L2 per part was most of a shared tile's cost
             if (!whole)
-              for (; c <= c_last; ++c) {
-                const int* src = slot_of(c) + static_cast<size_t>(c0) * kTcTileN;
-                int t[16];
+              for (; c <= c_last; c += 3) {
+                int t[3][16];
 #pragma unroll
-                for (int e = 0; e < 16; ++e) t[e] = c0 + e < mv ? __ldcg(src + e * kTcTileN) : 0;
+                for (int u = 0; u < 3; ++u) {
+                  const bool some = c + u <= c_last;
+                  const int* src = slot_of(some ? c + u : c) + static_cast<size_t>(c0) * kTcTileN;
 #pragma unroll
-                for (int e = 0; e < 16; ++e) v[e] += t[e];
+                  for (int e = 0; e < 16; ++e) t[u][e] = some && c0 + e < mv ? __ldcg(src + e * kTcTileN) : 0;
+                }
+#pragma unroll
+                for (int e = 0; e < 16; ++e) v[e] += t[0][e] + t[1][e] + t[2][e];
               }
             if (p.acc_out && row_ok) {
 #pragma unroll
               for (int e = 0; e < 16; ++e)
                 if (c0 + e < mv) p.acc_out[static_cast<size_t>(tok0 + c0 + e) * p.n + n] = v[e];
             }
-            // bias + (float(acc - compensation * zp) * scale_a) * scale_w, the integer part exact
-            // (csrc/cpu/aten/utils/woq.h:2310-2321); columns past the last token hold anything
+            // (columns past the last token hold anything)
             uint8_t* dst = out_tile + (c0 - t0) * kOutPitch + row * 2;
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-              const int acc = v[e] - comp * s_zp[c0 + e];
-              float f = (static_cast<float>(acc) * s_sa[c0 + e]) * sw;
-              if (p.bias) f = bias + f;
-              *reinterpret_cast<__nv_bfloat16*>(dst + e * kOutPitch) = __float2bfloat16_rn(f);
-            }
+            for (int e = 0; e < 16; ++e)
+              *reinterpret_cast<__nv_bfloat16*>(dst + e * kOutPitch) =
+                  ip_result(v[e], comp, s_zp[c0 + e], s_sa[c0 + e], sw, p.bias, bias);
           }
           if (from_tmem && t1 == mv) accumulators_read();
           named_bar_sync(1, kEpiThreads);
@@ -305,6 +339,49 @@ __global__ void __launch_bounds__(kIpThreads, 1)
       ++item;
       ++seg_no;
       named_bar_sync(1, kEpiThreads);  // scales and `decision` have been read
+    }
+  }
+
+  if (SPLIT) {
+    __syncwarp();
+    pair_sync();  // every pair's part is in its shared memory
+    const int tile = item0 / p.tok_tiles * 2 + static_cast<int>(rank), tok0 = item0 % p.tok_tiles * p.n_tok;
+    const int mv = p.m - tok0 < p.n_tok ? p.m - tok0 : p.n_tok;
+    const int slice = (mv + p.split - 1) / p.split, t0 = static_cast<int>(crank >> 1) * slice;
+    const int nt = tile >= p.tiles ? 0 : mv - t0 < slice ? mv - t0 : slice;  // this CTA's tokens t0 .. t0 + nt
+    const int row = (warp & 3) * 32 + lane, n = tc_tile_row_to_n(p.n, p.gate_up, tile < p.tiles ? tile : 0, row);
+    const bool row_ok = n < p.n;
+    const float sw = row_ok ? p.sw[n] : 0.f, bias = row_ok && p.bias ? p.bias[n] : 0.f;
+    const int comp = row_ok && p.zpa ? p.comp[n] : 0;
+    const uint32_t part0 = pair_map(reinterpret_cast<const int*>(a_stages) + row, rank);
+    const uint32_t part_step = pair_map(a_stages, 2) - pair_map(a_stages, 0);  // to the next pair's part
+    for (int s0 = 0; s0 < nt; s0 += kIpPassTok) {
+      const int ns = nt - s0 < kIpPassTok ? nt - s0 : kIpPassTok;
+      // a warp: 32 rows of a token; four tokens' reads in flight together
+      constexpr int kGroups = kIpThreads / 128, kBatch = 4;
+      for (int t = warp >> 2; t < ns; t += kGroups * kBatch) {
+        int v[kBatch][4];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+          const int tok = t + u * kGroups;
+#pragma unroll
+          for (int s = 0; s < 4; ++s)
+            v[u][s] = tok < ns && s < p.split
+                          ? __float_as_int(pair_ld_f32(part0 + s * part_step + (t0 + s0 + tok) * (kTcTileN * 4)))
+                          : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+          const int tok = t + u * kGroups, col = t0 + s0 + tok, acc = v[u][0] + v[u][1] + v[u][2] + v[u][3];
+          if (tok >= ns) break;
+          if (p.acc_out && row_ok) p.acc_out[static_cast<size_t>(tok0 + col) * p.n + n] = acc;
+          *reinterpret_cast<__nv_bfloat16*>(out_tile + tok * kOutPitch + row * 2) =
+              ip_result(acc, comp, s_zp[col], s_sa[col], sw, p.bias, bias);
+        }
+      }
+      __syncthreads();
+      if (p.y && warp >= 4) pair_copy_out<false>(p, p.y, out_tile, tile, tok0 + t0 + s0, ns, tid - 4 * 32);
+      __syncthreads();
     }
   }
 
@@ -330,9 +407,14 @@ cudaError_t launch_i8_pair(I8PairParams p, const CUtensorMap& wmap, const CUtens
   p.stages = (227 * 1024 - kIpHeaderBytes - kIpOutBytes) / stage;
   if (p.stages > kIpMaxStages) p.stages = kIpMaxStages;
   const size_t smem = kIpHeaderBytes + static_cast<size_t>(p.stages) * stage + kIpOutBytes;
-  const int64_t total = static_cast<int64_t>(p.w_tiles) * p.tok_tiles * p.kc_per_tile;
-  const int64_t pairs = total < num_sms / 2 ? total : num_sms / 2;
-  cudaError_t e = cudaFuncSetAttribute(woq_i8_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  const int64_t total = static_cast<int64_t>(p.w_tiles) * p.tok_tiles * p.kc_per_tile / p.unit;
+  if (p.split > 1 && (p.kc_per_tile < p.split || static_cast<size_t>(p.n_tok) * kTcTileN * 4 >
+                                                     static_cast<size_t>(p.stages) * stage))
+    return cudaErrorInvalidValue;  // (pair_cut does not ask for these)
+  const int64_t pairs = p.split > 1 ? static_cast<int64_t>(p.w_tiles) * p.tok_tiles * p.split
+                        : total < num_sms / 2 ? total : num_sms / 2;
+  auto* kern = p.split > 1 ? woq_i8_pair_kernel<true> : woq_i8_pair_kernel<false>;
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem));
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
@@ -342,7 +424,7 @@ cudaError_t launch_i8_pair(I8PairParams p, const CUtensorMap& wmap, const CUtens
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.x = p.split > 1 ? 2 * p.split : 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
@@ -352,7 +434,7 @@ cudaError_t launch_i8_pair(I8PairParams p, const CUtensorMap& wmap, const CUtens
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.numAttrs = 2;
   }
-  return cudaLaunchKernelEx(&cfg, woq_i8_pair_kernel, p, wmap, qamap);
+  return cudaLaunchKernelEx(&cfg, kern, p, wmap, qamap);
 }
 
 }  // namespace woq

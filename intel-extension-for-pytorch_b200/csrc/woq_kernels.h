@@ -186,13 +186,20 @@ struct PairParams {
   int tiles, w_tiles;           // 128-row tiles; pairs of them (rounded up)
   int kb_per_tile, kbpg_shift, groups;
   int kbs, kpw, stages, w_ring; // k-blocks per stage, and of them per warpgroup; slots of the two rings
+  int whole, split;             // pairs take whole tiles; pairs of a cluster that share a tile (0, 1: none)
   int unit;                     // shares are multiples of this many k-blocks
   int fusion, gate_up;
   int kind;      // WeightKind
   int part_tok;  // tokens of a partial tile: min(most tokens of a group, n_tok)
   int vec;  // y and the extra operands can be accessed 16 bytes at a time
 };
-void pair_token_tiles(int64_t m, int* n_tok, int* tok_tiles);
+// How a launch is cut: token columns, tiles of tokens, and whether pairs take whole tiles (or equal shares of
+// the k sequence).  `kind`: a WeightKind, or kPairCutInt8 for the INT8 compute kernel (k steps of 128, not 64).
+constexpr int kPairCutInt8 = -1;
+struct PairCut {
+  int n_tok, tok_tiles, whole, split;  // split > 1: so many pairs, a cluster, share each tile
+};
+PairCut pair_cut(int64_t m, int w_tiles, int k_steps, int pairs, int kind);
 int pair_group_columns(const int64_t* rows, int groups);
 size_t pair_plan(PairParams& p);  // fills kbs, stages, w_ring, unit; dynamic shared memory (0: none)
 size_t pair_partial_bytes(int num_sms, int part_tok);
@@ -240,9 +247,10 @@ struct I8PairParams {
   int* status;
   int64_t ldy;
   int m, n, n_out;
-  int n_tok, tok_tiles;  // as pair_token_tiles
+  int n_tok, tok_tiles, unit;  // as pair_cut; shares are multiples of `unit` k-chunks
   int tiles, w_tiles;    // 128-row tiles; pairs of them (rounded up)
   int kc_per_tile, part_tok, stages, fusion, gate_up;
+  int split;  // pairs of a cluster that share a tile (0, 1: none)
   int vec;  // y and the extra operands can be accessed 16 bytes at a time
 };
 size_t i8_pair_partial_bytes(int num_sms, int part_tok);

@@ -26,6 +26,11 @@ __device__ __forceinline__ uint32_t pair_map(const void* p, uint32_t rank) {
 __device__ __forceinline__ void pair_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+__device__ __forceinline__ float pair_ld_f32(uint32_t a) {  // from a shared::cluster address
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
 // true in exactly one lane of a converged warp
 __device__ __forceinline__ bool elect_one() {
   uint32_t ok;
@@ -62,12 +67,13 @@ __device__ __forceinline__ void pair_mma_f16_ts(uint32_t d_tmem, uint32_t a_tmem
       : "r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// arrive on the barrier at this offset in both CTAs once everything this thread has issued is done
-__device__ __forceinline__ void pair_commit(uint64_t* bar) {
+// arrive on the barrier at this offset in both CTAs of the pair (`mask`: their ranks in the cluster) once
+// everything this thread has issued is done
+__device__ __forceinline__ void pair_commit(uint64_t* bar, uint16_t mask = 3) {
   asm volatile(
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
           smem_u32(bar)),
-      "h"(static_cast<uint16_t>(3))
+      "h"(mask)
       : "memory");
 }
 // Instruction descriptor of a pair's MMA (M = 256); formats as umma_idesc.

@@ -23,6 +23,12 @@
 // share, when the others are normally done, and then adds its accumulators straight from TMEM).
 // Nobody waits for an arrival, and the order of the sum does not depend on timing.
 //
+// SPLIT: few tiles (p.split = S = 2 .. 4 pairs each).  The S pairs of a tile form one cluster and take a
+// contiguous part of k each; they leave their fp32 accumulators in shared memory, and after a cluster barrier
+// each CTA adds 1 / S of the tokens over distributed shared memory, in k order.  With shares of the k sequence
+// the same tiles pay three trips through L2 and one CTA per tile reads all the parts: 4096 x 4096, 128 tokens
+// took 26 us for 4 us of MMAs.
+//
 // What bounds it: at 256 token columns the tensor cores under the power limit (57344 x 8192, 512
 // tokens: 339 us, 1420 TFLOP/s, against 501 us for one CTA per tile and 256 tokens per launch); at 32
 // columns the dequantiser's issue slots and the hand-overs between roles (91 us, 2.7 TB/s of weights,
@@ -33,6 +39,8 @@
 // Weights: INT4, INT8 and NF4 in the row layout of their kind (WeightKind); only the dequantiser and
 // the bytes of a k-block differ.
 #include "woq_kernels.h"
+#include <atomic>
+
 #include "woq_pair_epilogue.cuh"
 
 namespace woq {
@@ -157,7 +165,7 @@ __device__ __forceinline__ void pair_dequant(const uint8_t* ws, int row, uint32_
   if (KIND == kWeightNf4) pair_dequant_nf4(ws, row, szw, lut_lane, r);
 }
 
-template <int KIND, int KPW>
+template <int KIND, int KPW, bool SPLIT>
 __global__ void __launch_bounds__(kPairThreads, 1)
     woq_pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtensorMap xmap) {
   extern __shared__ __align__(1024) uint8_t smem[];
@@ -178,16 +186,26 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   uint8_t* lut = out_tile + p.n_tok * kOutPitch;  // NF4 only
   if (KIND == kWeightNf4 && tid < 512) reinterpret_cast<float*>(lut)[tid] = kNf4Table[tid >> 5];
 
-  const uint32_t rank = pair_cta_rank();
+  const uint32_t crank = pair_cta_rank(), rank = crank & 1, leader = crank - rank;  // rank in cluster / pair
+  const uint16_t pair_mask = static_cast<uint16_t>(3u << leader);
   const int pair = blockIdx.x >> 1;
   const int64_t pairs = gridDim.x >> 1;
   const int kbpt = p.kb_per_tile, kbs = p.kbs, n_stages = p.stages, n_wring = p.w_ring;
   // shares are dealt in units of p.unit k-blocks
   const int64_t units = static_cast<int64_t>(p.items) * kbpt / p.unit;
-  const int64_t b_begin = pair * units / pairs * p.unit, b_end = (pair + 1) * units / pairs * p.unit;
-  const int item0 = static_cast<int>(b_begin / kbpt);  // item - group.item0 = weight tile * tok_tiles + token tile
-  const int kb00 = static_cast<int>(b_begin % kbpt);
-  const int rem0 = static_cast<int>(b_end - b_begin);
+  int item0, kb00, rem0;  // item0 - group.item0 = weight tile * tok_tiles + token tile
+  if (SPLIT) {
+    const int sub = crank >> 1, n_st = (kbpt + kbs - 1) / kbs;  // whole stages, at least one each
+    item0 = pair / p.split;
+    kb00 = sub * n_st / p.split * kbs;
+    const int kb_end = (sub + 1) * n_st / p.split * kbs;
+    rem0 = (kb_end < kbpt ? kb_end : kbpt) - kb00;
+  } else {
+    const int64_t b_begin = pair * units / pairs * p.unit, b_end = (pair + 1) * units / pairs * p.unit;
+    item0 = static_cast<int>(b_begin / kbpt);
+    kb00 = static_cast<int>(b_begin % kbpt);
+    rem0 = static_cast<int>(b_end - b_begin);
+  }
 
   if (tid == 0) {
     for (int s = 0; s < n_stages; ++s) {
@@ -258,7 +276,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       grid_dependency_wait();
       int item = item0, kb0 = kb00, rem = rem0, slot = 0, g = pair_group_of(p, item0);
       uint32_t phase = 0;
-      const uint32_t full0 = pair_map(&hdr->full[0], 0);
+      const uint32_t full0 = pair_map(&hdr->full[0], leader);
       while (rem > 0) {
         if (g + 1 < p.n_groups && item >= p.group[g + 1].item0) ++g;
         // (rows past the group's last belong to another group or to nobody: their columns are not used)
@@ -311,8 +329,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
               a += 32;
               b += x_blk16;
             }
-            pair_commit(&hdr->free_[slot]);
-            if (seg <= kbs) pair_commit(&hdr->d_full);
+            pair_commit(&hdr->free_[slot], pair_mask);
+            if (seg <= kbs) pair_commit(&hdr->d_full, pair_mask);
           }
           __syncwarp();
           accumulate = 1;
@@ -332,7 +350,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     const int wgs = kbs / KPW, step = kDeqGroups / wgs;
     const int j0 = wg % wgs * KPW;  // first k-block within the stage
     const uint32_t a_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + p.n_tok + j0 * 32;
-    const uint32_t full0 = pair_map(&hdr->full[0], 0);
+    const uint32_t full0 = pair_map(&hdr->full[0], leader);
     int kb_seg = kb00, rem = rem0;
     int own = wg / wgs, slot = own, wslot = own;  // `own`: this warpgroup's next stage, counted over all segments
     int st = 0;
@@ -391,7 +409,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     const int q = warp & 3, eg = (warp - kRoleWarps) >> 2, et = tid - kRoleWarps * 32;
     const int row = q * 32 + lane;
     const uint32_t d_lane = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
-    const uint32_t d_empty0 = pair_map(&hdr->d_empty, 0);
+    const uint32_t d_empty0 = pair_map(&hdr->d_empty, leader);
     grid_dependency_wait();  // y, the fused operands and the workspace belong to this grid now
     int item = item0, kb0 = kb00, rem = rem0, g = pair_group_of(p, item0);
     uint32_t seg_no = 0;
@@ -425,6 +443,17 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       mbar_wait<true>(&hdr->d_full, seg_no & 1, abort_flag, p.status, 37);
       tc_fence_after_sync();
       __syncwarp();
+      if (SPLIT) {  // this pair's part of the tile, for the CTAs that add it up
+        float* part = reinterpret_cast<float*>(x_stages) + row;
+        for (int c0 = eg * 16; c0 < mv; c0 += 32) {
+          uint32_t t[16];
+          tmem_ld_x16(d_lane + c0, t);
+          tc_wait_ld();
+#pragma unroll
+          for (int e = 0; e < 16; ++e) part[(c0 + e) * kTcTileN] = __uint_as_float(t[e]);
+        }
+        break;
+      }
       bool finish = whole && real;
       if (whole || !real) {
         if (real)
@@ -498,13 +527,18 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 #pragma unroll
               for (int e = 0; e < 16; ++e) v[e] = 0.f;
             }
-            for (; c <= c_last; ++c) {
+            // two parts in flight together: a round trip to L2 per part was most of a shared tile's cost
+            for (; c <= c_last; c += 2) {
+              const bool two = c < c_last;
               const float* src = slot_of(c) + static_cast<size_t>(c0) * kTcTileN;
-              float t[16];
+              const float* src2 = slot_of(two ? c + 1 : c) + static_cast<size_t>(c0) * kTcTileN;
+              float t[16], t2[16];
 #pragma unroll
               for (int e = 0; e < 16; ++e) t[e] = c0 + e < mv ? __ldcg(src + e * kTcTileN) : 0.f;
 #pragma unroll
-              for (int e = 0; e < 16; ++e) v[e] += t[e];
+              for (int e = 0; e < 16; ++e) t2[e] = two && c0 + e < mv ? __ldcg(src2 + e * kTcTileN) : 0.f;
+#pragma unroll
+              for (int e = 0; e < 16; ++e) v[e] = two ? v[e] + t[e] + t2[e] : v[e] + t[e];
             }
             to_tile(c0, v, bias);
           }
@@ -520,6 +554,44 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     }
   }
 
+  if (SPLIT) {
+    __syncwarp();
+    pair_sync();  // every pair's part is in its shared memory
+    const PairGroup& grp = p.group[0];
+    const int tile = item0 / grp.tok_tiles * 2 + static_cast<int>(rank), tok0 = item0 % grp.tok_tiles * p.n_tok;
+    const int mv = grp.m - tok0 < p.n_tok ? grp.m - tok0 : p.n_tok;
+    const int slice = (mv + p.split - 1) / p.split, t0 = static_cast<int>(crank >> 1) * slice;
+    const int nt = mv - t0 < slice ? mv - t0 : slice;  // this CTA's tokens t0 .. t0 + nt (none: <= 0)
+    if (tile < p.tiles) {
+      // a warp: 32 rows of a token; four tokens' reads in flight together
+      constexpr int kWarps = kPairThreads / 32, kBatch = 4;
+      const int row = (warp & 3) * 32 + lane, n = tc_tile_row_to_n(p.n, p.gate_up, tile, row);
+      const float bias = grp.bias && n < p.n ? grp.bias[n] : 0.f;
+      const uint32_t part0 = pair_map(reinterpret_cast<const float*>(x_stages) + row, rank);
+      const uint32_t part_step = pair_map(x_stages, 2) - pair_map(x_stages, 0);  // to the next pair's part
+      for (int t = warp >> 2; t < nt; t += kWarps / 4 * kBatch) {
+        float v[kBatch][4];
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+          const int tok = t + u * (kWarps / 4);
+#pragma unroll
+          for (int s = 0; s < 4; ++s)
+            v[u][s] = tok < nt && s < p.split ? pair_ld_f32(part0 + s * part_step + (t0 + tok) * (kTcTileN * 4)) : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < kBatch; ++u) {
+          const int tok = t + u * (kWarps / 4);
+          if (tok < nt)
+            *reinterpret_cast<__nv_bfloat16*>(out_tile + tok * kOutPitch + row * 2) =
+                __float2bfloat16_rn(((v[u][0] + v[u][1]) + v[u][2]) + v[u][3] + bias);
+        }
+      }
+    }
+    __syncthreads();
+    if (tile < p.tiles && nt > 0 && warp >= kRoleWarps && warp < kDeqWarp0)
+      pair_copy_out<true>(p, grp.y, out_tile, tile, tok0 + t0, nt, tid - kRoleWarps * 32);
+  }
+
   __syncwarp();
   tc_fence_before_sync();
   __syncthreads();
@@ -532,13 +604,45 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 
 }  // namespace
 
-// Token tiles of a call: as few as 256 columns allow, then as narrow as they can be (a multiple of 32,
-// which is what a pair's MMA takes), so that 300 tokens are two tiles of 160, not of 256.
-void pair_token_tiles(int64_t m, int* n_tok, int* tok_tiles) {
-  const int t = static_cast<int>((m + 255) / 256);
-  *tok_tiles = t < 1 ? 1 : t;
-  *n_tok = static_cast<int>(((m + *tok_tiles - 1) / *tok_tiles + 31) / 32 * 32);
-  if (*n_tok < 32) *n_tok = 32;
+// Token tiles of a call, and how its tiles are dealt, by estimated time in us.  A k step costs a tile of n
+// columns the larger of its dequantisation and hand-overs (or, for INT8 compute, its L2 traffic) and its MMAs:
+// fitted to 57344 x 8192 INT4 (72 / 77 / 89 / 101 / 176 / 333 us at 32 / 64 / 96 / 128 / 256 / 512 tokens),
+// 57344 x 4096 INT8 with bf16 compute (44 / 52 / 68 us at 8 / 64 / 128) and INT8 compute on 28672 x 4096
+// (121 / 220 us at 1024 / 2048).  Whole tiles take as many rounds as the fullest pair has tiles.  Equal shares of the k sequence
+// keep every pair busy to the end, but then the parts of shared tiles go through the workspace, one after
+// another and behind the last MMA: 4096 x 4096, 1000 tokens took 46 us with shares for 25 us of MMAs.  With few
+// tiles, clusters of pairs split k (see SPLIT).
+static int pair_cluster_capacity(int ctas);
+PairCut pair_cut(int64_t m, int w_tiles, int k_steps, int pairs, int kind) {
+  PairCut best{};
+  double best_cost = -1;
+  const int t0 = static_cast<int>(m > 256 ? (m + 255) / 256 : 1);
+  for (int t = t0; t <= 2 * t0 + 1; ++t) {
+    int n = static_cast<int>(((m + t - 1) / t + 31) / 32 * 32);
+    if (n < 32) n = 32;
+    if ((m + n - 1) / n != t) continue;  // fewer tiles of this width do
+    const double mma = (kind == kPairCutInt8 ? 0.0011 : 0.0017) * n;
+    double step = kind == kPairCutInt8                                    ? 0.26 + 0.001 * n
+                  : kind == kWeightInt4 || kind == kWeightInt4InPlace     ? 0.165 + 0.00075 * n
+                  : kind == kWeightNf4                                    ? 0.25 + 0.001 * n
+                                                                          : 0.19 + 0.00125 * n;
+    if (step < mma) step = mma;
+    const int64_t items = static_cast<int64_t>(w_tiles) * t;
+    const double shares = step * k_steps * items / pairs + 4 + 0.04 * n + 2.0 * pairs / items;
+    const double rounds = step * k_steps * static_cast<double>((items + pairs - 1) / pairs);
+    auto consider = [&](double cost, int whole, int split) {
+      if (best_cost >= 0 && cost >= best_cost) return;
+      best_cost = cost;
+      best = PairCut{n, t, whole, split};
+    };
+    consider(shares, 0, 1);
+    consider(rounds, 1, 1);
+    // (a part has at least one stage of four k-blocks)
+    for (int s = 2; s <= 4; ++s)
+      if (k_steps >= 4 * s && items <= pair_cluster_capacity(2 * s))
+        consider(step * ((k_steps + s - 1) / s) + 2 + 0.01 * n, 0, s);
+  }
+  return best;
 }
 
 // Token columns for several linears in one launch, by the number of tokens each has: the width with the least
@@ -594,47 +698,87 @@ size_t pair_plan(PairParams& p) {
   p.w_ring = ring;
   // shares in whole stages where they are long enough for the rounding not to matter
   const int64_t total = static_cast<int64_t>(p.items) * p.kb_per_tile;
-  p.unit = p.kb_per_tile % p.kbs == 0 && total >= static_cast<int64_t>(74) * 8 * p.kbs ? p.kbs : 1;
+  p.unit = p.whole ? p.kb_per_tile : p.kb_per_tile % p.kbs == 0 && total >= static_cast<int64_t>(74) * 8 * p.kbs ? p.kbs : 1;
   return kPairHeaderBytes + static_cast<size_t>(stages) * x_stage + static_cast<size_t>(ring) * w_stage +
          static_cast<size_t>(p.n_tok) * kOutPitch + lut;
 }
 
-// Pairs of a launch: all SMs, or one per k-block when there are fewer.
+// Pairs of a launch: all SMs, or one per unit of work when there are fewer.
 int pair_grid(const PairParams& p, int num_sms) {
-  const int64_t total = static_cast<int64_t>(p.items) * p.kb_per_tile;
+  const int64_t total = static_cast<int64_t>(p.items) * p.kb_per_tile / p.unit;
   int64_t pairs = num_sms / 2;
   if (pairs > total) pairs = total;
   return static_cast<int>(pairs < 1 ? 1 : pairs) * 2;
+}
+
+// Clusters of that many CTAs of this kernel's size that the current device runs at a time: a split whose
+// clusters need a second round takes twice as long (16 clusters of 8: 27 us for a 4096 x 14336 layer that 20 us
+// of shares do).  Asked once per device and size; an error counts as none.
+static int pair_cluster_capacity(int ctas) {
+  static std::atomic<int> known[64][9];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) return 0;
+  int n = known[dev][ctas].load(std::memory_order_relaxed);
+  if (n) return n - 1;
+  auto* kern = woq_pair_kernel<kWeightInt4, 1, true>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(static_cast<unsigned>(ctas * 32));
+  cfg.blockDim = dim3(kPairThreads);
+  cfg.dynamicSmemBytes = 227 * 1024;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = ctas;
+  attr.val.clusterDim.y = 1;
+  attr.val.clusterDim.z = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    clusters = 0;
+  }
+  known[dev][ctas].store(clusters + 1, std::memory_order_relaxed);
+  return clusters;
 }
 
 size_t pair_partial_bytes(int num_sms, int part_tok) {
   return static_cast<size_t>(num_sms) * 2 * part_tok * kTcTileN * sizeof(float);
 }
 
+template <int KIND>
+static void (*pick_pair_kernel(const PairParams& p))(const PairParams, const CUtensorMap) {
+  if (p.split > 1) return p.kpw == 2 ? woq_pair_kernel<KIND, 2, true> : woq_pair_kernel<KIND, 1, true>;
+  return p.kpw == 2 ? woq_pair_kernel<KIND, 2, false> : woq_pair_kernel<KIND, 1, false>;
+}
+
 cudaError_t launch_pair(PairParams p, const CUtensorMap& xmap, int num_sms, cudaStream_t stream) {
   const size_t smem = pair_plan(p);
   if (smem == 0) return cudaErrorInvalidConfiguration;
   void (*kern)(const PairParams, const CUtensorMap) = nullptr;
-  const bool two = p.kpw == 2;
   switch (p.kind) {
-    case kWeightInt4InPlace: kern = two ? woq_pair_kernel<kWeightInt4InPlace, 2> : woq_pair_kernel<kWeightInt4InPlace, 1>; break;
-    case kWeightInt4: kern = two ? woq_pair_kernel<kWeightInt4, 2> : woq_pair_kernel<kWeightInt4, 1>; break;
-    case kWeightInt8InPlace: kern = two ? woq_pair_kernel<kWeightInt8InPlace, 2> : woq_pair_kernel<kWeightInt8InPlace, 1>; break;
-    case kWeightInt8: kern = two ? woq_pair_kernel<kWeightInt8, 2> : woq_pair_kernel<kWeightInt8, 1>; break;
-    case kWeightNf4: kern = two ? woq_pair_kernel<kWeightNf4, 2> : woq_pair_kernel<kWeightNf4, 1>; break;
+    case kWeightInt4InPlace: kern = pick_pair_kernel<kWeightInt4InPlace>(p); break;
+    case kWeightInt4: kern = pick_pair_kernel<kWeightInt4>(p); break;
+    case kWeightInt8InPlace: kern = pick_pair_kernel<kWeightInt8InPlace>(p); break;
+    case kWeightInt8: kern = pick_pair_kernel<kWeightInt8>(p); break;
+    case kWeightNf4: kern = pick_pair_kernel<kWeightNf4>(p); break;
     default: return cudaErrorInvalidValue;
   }
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem));
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(pair_grid(p, num_sms));
+  if (p.split > 1 && (p.n_groups != 1 || (p.kb_per_tile + p.kbs - 1) / p.kbs < p.split ||
+                      static_cast<size_t>(p.n_tok) * kTcTileN * 4 >
+                          smem - kPairHeaderBytes - static_cast<size_t>(p.n_tok) * kOutPitch - kNf4LutBytes))
+    return cudaErrorInvalidValue;  // (pair_cut does not ask for these)
+  cfg.gridDim = dim3(p.split > 1 ? p.items * p.split * 2 : pair_grid(p, num_sms));
   cfg.blockDim = dim3(kPairThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.x = p.split > 1 ? 2 * p.split : 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
