@@ -16,6 +16,7 @@
 
 #include "../../include/woq_b200.h"
 #include "woq_kernels.h"
+#include "woq_nf4.cuh"
 
 namespace woq {
 
@@ -24,6 +25,8 @@ namespace {
 constexpr int kRows = 4;    // output rows per warp
 constexpr int kTok = 8;     // tokens per pass
 constexpr int kWarps = 4;   // warps per CTA
+
+__constant__ float kNf4Table[16] = WOQ_NF4_VALUES;
 
 // FP8 e4m3 byte -> fp32, bit for bit the reference's conversion
 // (csrc/cpu/aten/utils/woq.h:465-483): exponent rebias by 120, three mantissa bits, zero when

@@ -141,23 +141,6 @@ enum WeightKind { kWeightInt4InPlace = 0, kWeightInt4, kWeightInt8InPlace, kWeig
 __host__ __device__ constexpr int pair_block_bytes(int kind) {
   return kind == kWeightInt8InPlace || kind == kWeightInt8 ? 2 * kTcBlockBytes : kTcBlockBytes;
 }
-// NF4 code -> value (reference: csrc/cpu/aten/utils/woq_utils.h:34-51)
-__constant__ const float kNf4Table[16] = {-1.0f,
-                                          -0.6961928009986877f,
-                                          -0.5250730514526367f,
-                                          -0.39491748809814453f,
-                                          -0.28444138169288635f,
-                                          -0.18477343022823334f,
-                                          -0.09105003625154495f,
-                                          0.0f,
-                                          0.07958029955625534f,
-                                          0.16093020141124725f,
-                                          0.24611230194568634f,
-                                          0.33791524171829224f,
-                                          0.44070982933044434f,
-                                          0.5626170039176941f,
-                                          0.7229568362236023f,
-                                          1.0f};
 // A launch runs one linear, or several of one shape on consecutive row ranges of x (the experts of a
 // mixture): `groups` of them, their items one after the other.
 constexpr int kMaxPairGroups = 32;
@@ -173,6 +156,7 @@ struct PairGroup {
 struct PairParams {
   PairGroup group[kMaxPairGroups];
   int n_groups, items;
+  float nf4[16];       // NF4: the table
   const __nv_bfloat16* other0;  // extra operands: one group only
   const __nv_bfloat16* other1;
   const int32_t* row_idx;

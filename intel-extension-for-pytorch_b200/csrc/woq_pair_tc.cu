@@ -41,6 +41,7 @@
 #include "woq_kernels.h"
 #include <atomic>
 
+#include "woq_nf4.cuh"
 #include "woq_pair_epilogue.cuh"
 
 namespace woq {
@@ -184,7 +185,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   uint8_t* w_stages = x_stages + static_cast<size_t>(p.stages) * x_stage_bytes;
   uint8_t* out_tile = w_stages + static_cast<size_t>(p.w_ring) * w_stage_bytes;
   uint8_t* lut = out_tile + p.n_tok * kOutPitch;  // NF4 only
-  if (KIND == kWeightNf4 && tid < 512) reinterpret_cast<float*>(lut)[tid] = kNf4Table[tid >> 5];
+  if (KIND == kWeightNf4 && tid < 512) reinterpret_cast<float*>(lut)[tid] = p.nf4[tid >> 5];
 
   const uint32_t crank = pair_cta_rank(), rank = crank & 1, leader = crank - rank;  // rank in cluster / pair
   const uint16_t pair_mask = static_cast<uint16_t>(3u << leader);
@@ -755,6 +756,10 @@ static void (*pick_pair_kernel(const PairParams& p))(const PairParams, const CUt
 cudaError_t launch_pair(PairParams p, const CUtensorMap& xmap, int num_sms, cudaStream_t stream) {
   const size_t smem = pair_plan(p);
   if (smem == 0) return cudaErrorInvalidConfiguration;
+  if (p.kind == kWeightNf4) {
+    static constexpr float values[16] = WOQ_NF4_VALUES;
+    for (int i = 0; i < 16; ++i) p.nf4[i] = values[i];
+  }
   void (*kern)(const PairParams, const CUtensorMap) = nullptr;
   switch (p.kind) {
     case kWeightInt4InPlace: kern = pick_pair_kernel<kWeightInt4InPlace>(p); break;
