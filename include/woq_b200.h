@@ -106,11 +106,13 @@ extern "C" {
  * loader can create hundreds of contexts back to back.  The inputs must stay alive until the
  * stream has passed the create call either way.  Plain-format INT4 contexts only. */
 #define WOQ_B200_LAYOUT_DEFER_CHECK 0x10
-/* Keep the weight in its plain layout and run it through the general kernel (any weight dtype,
+/* Run the layer on the general route: the general kernel (any weight dtype,
  * fp32 / fp16 / bf16 compute, any K, group sizes that are multiples of 8).  Descriptions the
  * tuned kernels do not take (NF4 / FP8 weights, INT8 weights without INT8 compute, lowp FP16,
  * K not a multiple of 64, group sizes below 64) get this route without the flag; set it to run
- * an INT4 layer on fp32 or fp16 activations under lowp NONE. */
+ * an INT4 layer on fp32 or fp16 activations under lowp NONE.  INT8 and NF4 layers of this route whose shape
+ * allows it (K a multiple of 64, one group or power-of-two groups of at least 64, zero points -128..127) run
+ * bf16 activations with bf16 compute on the tensor-core kernel, given woq_b200_workspace_bytes of workspace. */
 #define WOQ_B200_LAYOUT_GENERIC 0x20
 
 /* kernel selection for INT4 weights.  AUTO, TENSOR_CORE and STREAM all multiply by the

@@ -230,7 +230,7 @@ Int8Workspace int8_ws_layout(const woq_b200_ctx* c, int64_t m) {
   n_tok = (n_tok + 15) / 16 * 16;
   if (n_tok < 16) n_tok = 16;
   w.partial_off = kWsHeaderBytes;
-  size_t off = w.partial_off + woq::int8_partial_bytes(c->num_sms, n_tok);
+  size_t off = w.partial_off + woq::i8_pair_partial_bytes(c->num_sms, n_tok);
   w.sa_off = (off + 255) / 256 * 256;
   const size_t m_pad = static_cast<size_t>((m + 63) / 64 * 64);
   w.zpa_off = w.sa_off + m_pad * sizeof(float);

@@ -195,27 +195,6 @@ __host__ __device__ inline int tc_tile_row_to_n(int n_total, int gate_up, int ti
 }
 
 // ---- INT8 compute path ----------------------------------------------------------------------
-struct I8Params {
-  const int8_t* wq;     // operand images [tiles64][kc_per_tile][8192]
-  const float* sw;      // per-channel weight scales [n_pad]
-  const float* sa;      // per-token activation scales [m]
-  const int32_t* zpa;   // per-token activation zero points [m] (asymmetric codes are u8), or null
-  const int32_t* comp;  // with zpa: per-row sums of the weight codes [n_pad]
-  const float* bias;
-  __nv_bfloat16* y;     // may be null when only the accumulators are wanted
-  const __nv_bfloat16* other0;
-  const __nv_bfloat16* other1;
-  int* acc_out;         // optional [m][n] int32 accumulators
-  void* partials;       // int32 [2 * grid][n_tok][128]
-  uint32_t* counters;
-  int* status;
-  int64_t ldy;
-  int m, n, n_out;
-  int m0, n_tok;
-  int tiles, kc_per_tile;  // 128-row tiles, 128-k chunks
-  int stages, fusion, gate_up;
-};
-// the same on CTA pairs (woq_i8_pair.cu)
 struct I8PairParams {
   const float* sw;      // per-channel weight scales [n_pad]
   const float* sa;      // per-token activation scales [m]
@@ -252,8 +231,6 @@ cudaError_t launch_rmsnorm_quant(const __nv_bfloat16* x, int64_t ldx, const __nv
                                  int k, int asym, __nv_bfloat16* y, int64_t ldy, int8_t* qa, float* sa, int32_t* zpa,
                                  cudaStream_t stream);
 cudaError_t launch_weight_row_sum(const int8_t* plain, int n, int k, int32_t* comp, cudaStream_t stream);
-size_t int8_partial_bytes(int grid, int n_tok);
-cudaError_t launch_int8_tc(I8Params p, const CUtensorMap& qamap, int grid, cudaStream_t stream);
 
 // ---- INT8 compute with K-block scaling (woq_int8_block.cu) --------------------------------
 struct I8BlockParams {
