@@ -305,9 +305,9 @@ int woq_b200_comm_status(woq_b200_comm* comm, void* stream);
 /* No counterpart in the reference.  Same computation as woq_b200_linear for at most 16 tokens,
  * for callers that may not allocate device memory (memory-planned graphs, servers that forbid
  * allocation after start-up, sandboxes without a re-entrant allocator): the scratch lives in a
- * 4 MiB array inside the library's device image, held by every GPU that loads the library
+ * 8 MiB array inside the library's device image, held by every GPU that loads the library
  * until the process exits.  Calls no cudaMalloc / cudaFree.  Returns WOQ_B200_ERR_INVALID_ARG
- * for m > 16 and WOQ_B200_ERR_WORKSPACE when the GPU would need more than the 4 MiB (more than
+ * for m > 16 and WOQ_B200_ERR_WORKSPACE when the GPU would need more than the 8 MiB (more than
  * 252 SMs).  The first call on each device looks up the array's address; make that call
  * outside any stream capture.  All calls on one GPU share the array: they must be
  * stream-ordered, two that overlap on the device race on the partial tiles and counters.  The
