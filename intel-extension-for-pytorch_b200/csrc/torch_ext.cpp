@@ -14,12 +14,17 @@
 #include <ATen/ATen.h>
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/custom_class.h>
 #include <torch/library.h>
 
+#include <algorithm>
+#include <atomic>
 #include <map>
 #include <mutex>
+#include <utility>
+#include <vector>
 
 #include "../../include/woq_b200.h"
 
@@ -45,38 +50,131 @@ int dtype_code(const at::Tensor& t) {
     TORCH_CHECK(rc__ == WOQ_B200_OK, "WOQ: ", woq_b200_last_error(), " (status ", rc__, ")"); \
   } while (0)
 
-// One zeroed workspace per (device, stream); grows on demand.  Calls on one stream are ordered,
-// which is what a shared workspace needs.
-std::mutex g_ws_mu;
-std::map<std::pair<int, cudaStream_t>, at::Tensor> g_ws_pool;
+// ---- workspaces -----------------------------------------------------------------------------
+// A call needs scratch whose header is zero and that no call running beside it uses (woq_b200_workspace_bytes).
+//
+// Eager calls on one stream are ordered: one workspace per (device, stream), replaced by a larger one on demand.
+//
+// A captured call runs again with every replay: on any stream, beside eager calls and other graphs, and after
+// the eager workspace of the capturing stream has been replaced.  So each stream of a capture has a workspace of its
+// own.  It is zeroed outside the graph (no node of one graph that another would rely on) and owned by the graph:
+// CUDA calls release_graph_workspaces when the graph and all that was instantiated from it are gone.
+struct GraphWorkspaces {
+  unsigned long long capture;  // unique over the lifetime of the process
+  struct Buffers {
+    int dev;
+    std::vector<at::Tensor> all;  // the last one is in use; calls captured earlier hold the smaller ones before it
+  };
+  std::map<cudaStream_t, Buffers> of_stream;
+};
 
-at::Tensor& workspace_for(c10::DeviceIndex dev, cudaStream_t stream, size_t bytes) {
-  // the same (device, stream) as the previous call of this thread: no lock, no look-up
-  thread_local int last_dev = -1;
-  thread_local cudaStream_t last_stream = nullptr;
-  thread_local at::Tensor* last = nullptr;
-  if (last && last_dev == dev && last_stream == stream && static_cast<size_t>(last->numel()) >= bytes) return *last;
-  std::lock_guard<std::mutex> lock(g_ws_mu);
-  auto& t = g_ws_pool[{dev, stream}];
-  if (!t.defined() || static_cast<size_t>(t.numel()) < bytes) {
-    t = at::zeros({static_cast<int64_t>(bytes)},
-                  at::TensorOptions().dtype(at::kByte).device(at::Device(at::kCUDA, dev)));
+struct WorkspacePool {
+  std::mutex mu;
+  std::map<std::pair<int, cudaStream_t>, at::Tensor> eager;
+  std::map<unsigned long long, GraphWorkspaces*> captured;  // by capture id
+  std::map<int, cudaStream_t> side;  // per device: a stream that is never captured
+  // what release_graph_workspaces leaves for the next call.  A lock of its own, under which nothing calls CUDA.
+  std::mutex released_mu;
+  std::atomic<bool> any_released{false};
+  std::vector<GraphWorkspaces*> released;
+};
+WorkspacePool& workspace_pool() {
+  static auto* pool = new WorkspacePool;  // never destroyed: a graph may be released while the process exits
+  return *pool;
+}
+
+// Runs where CUDA may not be called, so the buffers go back to the allocator from the next call.
+void CUDART_CB release_graph_workspaces(void* graph_workspaces) {
+  WorkspacePool& pool = workspace_pool();
+  std::lock_guard<std::mutex> lock(pool.released_mu);
+  pool.released.push_back(static_cast<GraphWorkspaces*>(graph_workspaces));
+  pool.any_released = true;
+}
+
+// (with pool.mu held)
+void free_released(WorkspacePool& pool) {
+  if (!pool.any_released) return;
+  std::vector<GraphWorkspaces*> dead;
+  {
+    std::lock_guard<std::mutex> lock(pool.released_mu);
+    dead.swap(pool.released);
+    pool.any_released = false;
   }
-  last_dev = dev;
-  last_stream = stream;
-  last = &t;  // std::map never moves its elements
+  for (auto* g : dead) {
+    pool.captured.erase(g->capture);
+    delete g;
+  }
+}
+
+// (with pool.mu held) A buffer with a zero header, made on a stream that takes no part in any capture.
+at::Tensor workspace_outside_captures(WorkspacePool& pool, c10::DeviceIndex dev, size_t bytes) {
+  c10::cuda::CUDAStreamCaptureModeGuard allow{cudaStreamCaptureModeRelaxed};
+  cudaStream_t& side = pool.side[dev];
+  if (!side) C10_CUDA_CHECK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+  c10::cuda::CUDAStreamGuard on_side(c10::cuda::getStreamFromExternal(side, dev));
+  at::Tensor t = at::empty({static_cast<int64_t>(bytes)},
+                           at::TensorOptions().dtype(at::kByte).device(at::Device(at::kCUDA, dev)));
+  C10_CUDA_CHECK(cudaMemsetAsync(t.data_ptr(), 0, woq_b200_workspace_header_bytes(), side));
+  C10_CUDA_CHECK(cudaStreamSynchronize(side));
   return t;
 }
 
-// Synchronises every stream that has run a WOQ op and raises if a kernel gave up one of its
-// bounded waits (its output is then not valid).  The ops themselves never synchronise.
+at::Tensor workspace_for(c10::DeviceIndex dev, cudaStream_t stream, size_t bytes) {
+  WorkspacePool& pool = workspace_pool();
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long capture = 0;
+  cudaGraph_t graph = nullptr;
+  if (stream) C10_CUDA_CHECK(cudaStreamGetCaptureInfo(stream, &status, &capture, &graph));  // (the legacy stream is never captured)
+  std::lock_guard<std::mutex> lock(pool.mu);
+  free_released(pool);
+  if (status != cudaStreamCaptureStatusActive) {
+    at::Tensor& t = pool.eager[{dev, stream}];
+    if (!t.defined() || static_cast<size_t>(t.numel()) < bytes)
+      t = at::zeros({static_cast<int64_t>(bytes)},
+                    at::TensorOptions().dtype(at::kByte).device(at::Device(at::kCUDA, dev)));
+    return t;
+  }
+  GraphWorkspaces*& g = pool.captured[capture];
+  if (!g) {
+    g = new GraphWorkspaces{capture, {}};
+    cudaUserObject_t owner = nullptr;
+    cudaError_t e = cudaUserObjectCreate(&owner, g, release_graph_workspaces, 1, cudaUserObjectNoDestructorSync);
+    if (e != cudaSuccess) {
+      delete g;
+      pool.captured.erase(capture);
+      C10_CUDA_CHECK(e);
+    }
+    e = cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove);
+    if (e != cudaSuccess) {
+      pool.captured.erase(capture);
+      cudaUserObjectRelease(owner, 1);  // hands the object to release_graph_workspaces
+      C10_CUDA_CHECK(e);
+    }
+  }
+  auto& bufs = g->of_stream[stream];
+  bufs.dev = dev;
+  const size_t last = bufs.all.empty() ? 0 : static_cast<size_t>(bufs.all.back().numel());
+  if (last < bytes) bufs.all.push_back(workspace_outside_captures(pool, dev, std::max(bytes, last + last / 2)));
+  return bufs.all.back();
+}
+
+// Synchronises every stream that has run a WOQ op, and the devices of captured ones, and raises if a kernel gave
+// up one of its bounded waits (its output is then not valid).  The ops themselves never synchronise.
 void woq_check_status() {
-  std::lock_guard<std::mutex> lock(g_ws_mu);
-  for (auto& kv : g_ws_pool) {
+  WorkspacePool& pool = workspace_pool();
+  std::lock_guard<std::mutex> lock(pool.mu);
+  free_released(pool);
+  for (auto& kv : pool.eager) {
     if (!kv.second.defined()) continue;
     c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(kv.first.first));
     WOQ_CHECK(woq_b200_workspace_status(kv.second.data_ptr(), kv.first.second));
   }
+  for (auto& g : pool.captured)
+    for (auto& kv : g.second->of_stream) {
+      c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(kv.second.dev));
+      C10_CUDA_CHECK(cudaDeviceSynchronize());  // replays run on streams that are not known here
+      for (auto& t : kv.second.all) WOQ_CHECK(woq_b200_workspace_status(t.data_ptr(), pool.side[kv.second.dev]));
+    }
 }
 
 // plain INT4 weight [N, K/2] (k even in the low nibble) with its input channels re-ordered
@@ -351,7 +449,7 @@ at::Tensor run(WoqLinearOpContext* c, const at::Tensor& input, int32_t fusion,
   if (M > 0) {
     woq_b200_ctx* k = general ? c->ctx_general() : c->ctx_for(M);
     const size_t need = woq_b200_workspace_bytes(k, M);
-    at::Tensor& ws = workspace_for(c->device, stream.stream(), need);
+    at::Tensor ws = workspace_for(c->device, stream.stream(), need);
     if (general) {
       const int io = x.scalar_type() == at::kBFloat16 ? WOQ_B200_T_BF16
                      : x.scalar_type() == at::kHalf   ? WOQ_B200_T_F16
@@ -445,7 +543,7 @@ at::Tensor woq_linear_prequant(const at::Tensor& qa, const at::Tensor& sa, const
   auto stream = at::cuda::getCurrentCUDAStream(c->device);
   if (M > 0) {
     woq_b200_ctx* k = c->ctx_for(M);
-    at::Tensor& ws = workspace_for(c->device, stream.stream(), woq_b200_workspace_bytes(k, M));
+    at::Tensor ws = workspace_for(c->device, stream.stream(), woq_b200_workspace_bytes(k, M));
     WOQ_CHECK(woq_b200_linear_prequant(k, q2.data_ptr(), sa.data_ptr(), zpa.numel() ? zpa.data_ptr() : nullptr, M,
                                        static_cast<int32_t>(fusion), optr.empty() ? nullptr : optr.data(),
                                        static_cast<int32_t>(optr.size()), y.data_ptr(), y.stride(0), ws.data_ptr(),
@@ -479,7 +577,7 @@ at::Tensor mixtral_moe_woq(const at::Tensor& hidden_states, const at::Tensor& to
   const int64_t M = a.size(0);
   auto stream = at::cuda::getCurrentCUDAStream(d->device);
   woq_b200_ctx* dk = d->ctx_for(M);
-  at::Tensor& ws = workspace_for(d->device, stream.stream(), woq_b200_workspace_bytes(dk, M));
+  at::Tensor ws = workspace_for(d->device, stream.stream(), woq_b200_workspace_bytes(dk, M));
   WOQ_CHECK(woq_b200_linear_scatter(dk, a.data_ptr(), M, a.stride(0), ti.data_ptr<int32_t>(), w.data_ptr(),
                                     output.data_ptr(), output.stride(0), ws.data_ptr(), ws.numel(),
                                     stream.stream()));
@@ -571,7 +669,7 @@ at::Tensor deepseek_moe_woq(const at::Tensor& hidden_states, const at::Tensor& t
         yd.push_back(row(res, off));
         off += cnt[e];
       }
-      at::Tensor& ws = workspace_for(dev, stream, woq_b200_workspace_bytes(gu[0], std::max<int64_t>(17, most)));
+      at::Tensor ws = workspace_for(dev, stream, woq_b200_workspace_bytes(gu[0], std::max<int64_t>(17, most)));
       WOQ_CHECK(woq_b200_linear_grouped(gu.data(), row0.data(), rows.data(), y.data(), static_cast<int32_t>(gu.size()),
                                         x.data_ptr(), pairs, hidden, ffn, ws.data_ptr(), ws.numel(), stream));
       WOQ_CHECK(woq_b200_silu_mul(gate.data_ptr(), up.data_ptr(), act.data_ptr(), pairs * ffn, stream));
@@ -585,7 +683,7 @@ at::Tensor deepseek_moe_woq(const at::Tensor& hidden_states, const at::Tensor& t
         auto linear = [&](const c10::intrusive_ptr<WoqLinearOpContext>& c, const at::Tensor& in, int32_t fusion,
                           const void* other, const at::Tensor& out) {
           woq_b200_ctx* k = c->ctx_for(cnt[e]);
-          at::Tensor& ws = workspace_for(dev, stream, woq_b200_workspace_bytes(k, cnt[e]));
+          at::Tensor ws = workspace_for(dev, stream, woq_b200_workspace_bytes(k, cnt[e]));
           WOQ_CHECK(woq_b200_linear(k, row(in, off), cnt[e], in.size(1), fusion, other ? &other : nullptr,
                                     other ? 1 : 0, row(out, off), out.size(1), ws.data_ptr(), ws.numel(), stream));
         };

@@ -352,6 +352,7 @@ class WoqContext:
                 )
             )
         self._ws: Optional[Workspace] = None
+        self._smaller = []  # workspaces that a larger one replaced: a captured call may still use them
 
     # -- lifetime ---------------------------------------------------------------------
     def close(self):
@@ -382,8 +383,13 @@ class WoqContext:
         return {"grid": out[0], "cluster": out[1], "kblocks_per_warp": out[2], "smem_budget": out[3]}
 
     def workspace(self, m: int) -> Workspace:
+        """The context's own workspace, for calls that are ordered by their stream.  It must not be made inside
+        a capture (its zeroing would belong to that graph): ask for it before, or pass `workspace` to the call."""
         need = self.workspace_bytes(m)
         if self._ws is None or self._ws.nbytes < need:
+            if self._ws is not None:
+                self._smaller.append(self._ws)
+                need = max(need, 2 * self._ws.nbytes)  # so that the replaced ones stay below the present one
             self._ws = Workspace(need, self.device)
         return self._ws
 

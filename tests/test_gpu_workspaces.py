@@ -1,0 +1,165 @@
+"""Scratch of captured calls: a CUDA graph stays valid whatever the capturing stream does afterwards, on whatever
+stream it is replayed, and beside other graphs captured on that stream."""
+import time
+
+import pytest
+import torch
+from torch import nn
+
+pytestmark = pytest.mark.gpu
+
+# 80 tiles of 256 rows: more than an SM pair each, so that the tensor-core kernels cut k and sum partial tiles
+# in the workspace (8 tokens of INT4 weights do that in the streaming kernel)
+N, K = 20480, 4096
+
+
+@pytest.fixture(scope="module")
+def linears():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    import ipex_b200  # noqa: F401
+    from ipex_b200 import quantization as Q
+    from ipex_b200.nn.modules import WeightOnlyQuantizedLinear
+
+    modes = Q.WoqActQuantMode
+    recipes = {
+        "default": (Q.WoqWeightDtype.INT8, Q.WoqLowpMode.NONE, modes.NONE, -1),
+        "nf4": (Q.WoqWeightDtype.NF4, Q.WoqLowpMode.NONE, modes.NONE, 64),
+        "int4": (Q.WoqWeightDtype.INT4, Q.WoqLowpMode.BF16, modes.NONE, 128),
+        "int8_int8": (Q.WoqWeightDtype.INT8, Q.WoqLowpMode.INT8, modes.PER_BATCH_SYM, -1),
+        "int4_int8": (Q.WoqWeightDtype.INT4, Q.WoqLowpMode.INT8, modes.PER_BATCH_IC_BLOCK_SYM, 128),
+    }
+    made = {}
+
+    def get(name):
+        if name not in made:
+            wd, lowp, act, g = recipes[name]
+            gen = torch.Generator(device="cuda").manual_seed(1)
+            lin = nn.Linear(K, N, bias=False, device="cuda", dtype=torch.bfloat16)
+            with torch.no_grad():
+                lin.weight.copy_(torch.randn(N, K, generator=gen, device="cuda", dtype=torch.bfloat16).mul_(0.02))
+            lin.qconfig = Q.get_weight_only_quant_qconfig_mapping(
+                weight_dtype=wd, lowp_mode=lowp, act_quant_mode=act, group_size=g).global_qconfig
+            made[name] = WeightOnlyQuantizedLinear.from_float(lin)
+            made[name].weight = None
+        return made[name]
+
+    return get
+
+
+def acts(m, seed=0):
+    return torch.randn(m, K, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda").bfloat16()
+
+
+def expected(lin, x):
+    y = lin(x)
+    torch.cuda.synchronize()
+    return y
+
+
+def capture(lin, x, stream):
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        y = lin(x)
+    return graph, y
+
+
+RECIPES = ["default", "nf4", "int4", "int8_int8", "int4_int8"]
+
+
+@pytest.mark.parametrize("recipe", RECIPES)
+@pytest.mark.parametrize("m", [8, 24])
+def test_replay_after_a_larger_eager_call(linears, recipe, m):
+    lin, x = linears(recipe), acts(m)
+    ref = expected(lin, x)
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        lin(x)  # the stream's eager workspace, as large as this call needs
+    graph, y = capture(lin, x, stream)
+    with torch.cuda.stream(stream):
+        lin(acts(512, 1))  # replaces it
+        fresh = [torch.full((1 << 20,), 0x5A, dtype=torch.uint8, device="cuda") for _ in range(64)]
+        y.zero_()
+        graph.replay()
+        graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, ref)
+    assert all(bool((t == 0x5A).all()) for t in fresh)
+    torch.ops.torch_ipex.woq_check_status()
+
+
+@pytest.mark.parametrize("recipe", RECIPES)
+def test_first_use_under_capture(linears, recipe):
+    """Nothing has run on the stream before it is captured, and the second graph is replayed first."""
+    lin, x = linears(recipe), acts(24)
+    ref = expected(lin, x)
+    stream = torch.cuda.Stream()
+    g1, y1 = capture(lin, x, stream)
+    g2, y2 = capture(lin, x, stream)
+    for g in (g2, g1, g2):
+        g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y1, ref) and torch.equal(y2, ref)
+
+
+@pytest.mark.parametrize("recipe", RECIPES)
+def test_growth_within_a_capture(linears, recipe):
+    lin = linears(recipe)
+    xs = [acts(m, m) for m in (3, 40, 300)]
+    refs = [expected(lin, x) for x in xs]
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        ys = [lin(x) for x in xs + xs[:1]]
+    for _ in range(2):
+        for y in ys:
+            y.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        for y, ref in zip(ys, refs + refs[:1]):
+            assert torch.equal(y, ref)
+
+
+@pytest.mark.parametrize("recipe", RECIPES)
+def test_replays_beside_eager_calls_and_another_graph(linears, recipe):
+    """Two graphs captured on one stream are replayed on two others while eager calls run on the capturing one."""
+    lin, x, xe = linears(recipe), acts(24), acts(20, 2)
+    ref, ref_e = expected(lin, x), expected(lin, xe)
+    stream, sides = torch.cuda.Stream(), [torch.cuda.Stream(), torch.cuda.Stream()]
+    graphs = [capture(lin, x, stream) for _ in sides]
+    torch.cuda.synchronize()
+    eager, replayed = [], []
+    for _ in range(30):
+        for (g, y), side in zip(graphs, sides):
+            with torch.cuda.stream(side):
+                g.replay()
+                replayed.append(y.clone())
+        with torch.cuda.stream(stream):
+            eager.append(lin(xe))
+    torch.cuda.synchronize()
+    assert all(torch.equal(y, ref) for y in replayed)
+    assert all(torch.equal(y, ref_e) for y in eager)
+    torch.ops.torch_ipex.woq_check_status()
+
+
+def test_a_graphs_workspace_is_given_back(linears):
+    lin, x = linears("default"), acts(200)
+    expected(lin, x)
+    one = acts(1)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    for _ in range(3):
+        graph, y = capture(lin, x, torch.cuda.Stream())
+        graph.replay()
+        torch.cuda.synchronize()
+        del graph, y
+    end = time.time() + 10
+    while time.time() < end:  # the graph's resources are released asynchronously
+        lin(one)
+        torch.cuda.synchronize()
+        if torch.cuda.memory_allocated() <= before:
+            break
+        time.sleep(0.05)
+    assert torch.cuda.memory_allocated() <= before
