@@ -303,9 +303,11 @@ I8BlockWs i8block_ws(const woq_b200_ctx* c, int64_t m) {
     w.n_tok = woq::i8_block_tc_columns(m);
     w.tok_tiles = static_cast<int>((m + w.n_tok - 1) / w.n_tok);
     w.part_tok = m < w.n_tok ? static_cast<int>(m) : w.n_tok;
-    off += (static_cast<size_t>(w.tok_tiles) * c->kc * w.n_tok * 4 + 255) / 256 * 256;
+    // (by the widest tile, so that a workspace made for m tokens serves any smaller call as well: the width does
+    // not grow with m)
+    off += (static_cast<size_t>((m + 127) / 128 * 128) * c->kc * 4 + 255) / 256 * 256;
     w.partials = off;
-    off += woq::i8_block_tc_partial_bytes(c->num_sms, w.part_tok);
+    off += woq::i8_block_tc_partial_bytes(c->num_sms, m < 128 ? static_cast<int>(m) : 128);
   }
   w.total = off;
   return w;

@@ -163,3 +163,62 @@ def test_a_graphs_workspace_is_given_back(linears):
             break
         time.sleep(0.05)
     assert torch.cuda.memory_allocated() <= before
+
+
+# ---- C ABI: the size of a workspace -------------------------------------------------------------------------
+def layer_ctx(recipe):
+    import numpy as np
+
+    from ipex_b200 import _capi
+    from oracle import woq_oracle as O
+
+    n, k = 384, 4096
+    wd, lowp, act, g = {
+        "int4": (O.WOQ_DTYPE_INT4, _capi.LOWP_BF16, -1, 128),
+        "int8_general": (O.WOQ_DTYPE_INT8, _capi.LOWP_NONE, -1, -1),
+        "nf4_general": (O.WOQ_DTYPE_NF4, _capi.LOWP_NONE, -1, 64),
+        "fp16_activations": (O.WOQ_DTYPE_INT8, _capi.LOWP_FP16, -1, -1),
+        "int8_per_token": (O.WOQ_DTYPE_INT8, _capi.LOWP_INT8, 2, -1),
+        "int8_per_token_sym": (O.WOQ_DTYPE_INT8, _capi.LOWP_INT8, 6, -1),
+        "int4_k_blocks": (O.WOQ_DTYPE_INT4, _capi.LOWP_INT8, 7, 128),
+        "int4_k_blocks_asym": (O.WOQ_DTYPE_INT4, _capi.LOWP_INT8, 3, 128),
+        "int8_k_blocks": (O.WOQ_DTYPE_INT8, _capi.LOWP_INT8, 7, -1),
+    }[recipe]
+    w = (np.random.default_rng(0).standard_normal((n, k)) * 0.02).astype(np.float32)
+    sym = wd == O.WOQ_DTYPE_NF4 or (lowp == _capi.LOWP_INT8 and wd == O.WOQ_DTYPE_INT8)
+    if g > 0:
+        qw, s, z = O.quantize_per_block(w, wd, g, sym)
+    else:
+        qw, s, z = O.quantize_per_channel(w, wd, sym)
+        s, z = s[:, None], None if z is None else z[:, None]
+    t = lambda a: None if a is None else torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    return _capi, _capi.WoqContext(t(qw), t(s), t(None if sym else z), None, n, k, wd, g, lowp, act_quant_mode=act)
+
+
+ROUTES = ["int4", "int8_general", "nf4_general", "fp16_activations", "int8_per_token", "int8_per_token_sym", "int4_k_blocks",
+          "int4_k_blocks_asym", "int8_k_blocks"]
+
+
+@pytest.mark.parametrize("recipe", ROUTES)
+def test_workspace_bytes_never_shrink_with_the_tokens(recipe):
+    _, ctx = layer_ctx(recipe)
+    sizes = [ctx.workspace_bytes(m) for m in range(1, 1300)]
+    assert all(a <= b for a, b in zip(sizes, sizes[1:]))
+
+
+@pytest.mark.parametrize("recipe", ROUTES)
+def test_a_workspace_serves_every_smaller_call(recipe):
+    capi, ctx = layer_ctx(recipe)
+    ws = capi.Workspace(ctx.workspace_bytes(160), "cuda")
+    ctx._ws = ws
+    for m in (1, 16, 17, 65, 100, 127, 128, 129, 160):
+        x = acts(m, m)
+        y = ctx.linear_any(x)
+        assert ctx._ws is ws
+        own = capi.Workspace(ctx.workspace_bytes(m), "cuda")
+        ctx._ws = own
+        assert torch.equal(y, ctx.linear_any(x))
+        assert ctx._ws is own
+        own.status()
+        ctx._ws = ws
+    ws.status()
