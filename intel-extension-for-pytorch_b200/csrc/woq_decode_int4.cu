@@ -1183,10 +1183,9 @@ const ClusterCapacity& cluster_capacity(int num_sms) {
   static ClusterCapacity cc = [num_sms] {
     ClusterCapacity v{};
     void (*kern)(const DecodeParams) = woq_int4_decode_kernel<1, kExactInPlace, 1, false, true>;
+    const bool attr_ok = allow_max_smem(kern) == cudaSuccess;
     for (int big = 0; big < 2; ++big) {
       const int smem = big ? 2 * kBudgetTwoCtas - 8 * 1024 : kBudgetTwoCtas;
-      const bool attr_ok =
-          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess;
       for (int c = 1; c <= 8; ++c) {
         int n = 0;
         cudaLaunchConfig_t cfg = {};
@@ -1303,8 +1302,7 @@ cudaError_t launch_decode_int4(DecodeParams p, const DecodePlan& plan, cudaStrea
   void (*kern)(const DecodeParams) = tb == 2     ? pick_kernel<2, 1>(p.exact, comm, cl)
                                      : kpw == 2 ? pick_kernel<1, 2>(p.exact, comm, cl)
                                                 : pick_kernel<1, 1>(p.exact, comm, cl);
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem));
+  cudaError_t e = allow_max_smem(kern);
   if (e != cudaSuccess) return e;
   // Programmatic dependent launch: this grid may start streaming weights while the previous
   // kernel in the stream drains (it waits for that kernel before it touches x, y or the

@@ -565,7 +565,7 @@ cudaError_t launch_i8_block_tc(I8BlockTcParams p, const CUtensorMap& qamap, int 
     case 128: kern = woq_i8_block_tc_kernel<4>; break;
     default: return cudaErrorInvalidValue;
   }
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+  cudaError_t e = allow_max_smem(kern);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(total < num_sms ? total : num_sms));

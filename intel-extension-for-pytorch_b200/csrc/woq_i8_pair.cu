@@ -404,7 +404,7 @@ size_t i8_pair_partial_bytes(int num_sms, int part_tok) {
 cudaError_t launch_i8_pair(I8PairParams p, const CUtensorMap& wmap, const CUtensorMap& qamap, int num_sms,
                            cudaStream_t stream) {
   const int stage = kIpABytes + p.n_tok / 2 * 128;
-  p.stages = (227 * 1024 - kIpHeaderBytes - kIpOutBytes) / stage;
+  p.stages = (kMaxSmemBytes - kIpHeaderBytes - kIpOutBytes) / stage;
   if (p.stages > kIpMaxStages) p.stages = kIpMaxStages;
   const size_t smem = kIpHeaderBytes + static_cast<size_t>(p.stages) * stage + kIpOutBytes;
   const int64_t total = static_cast<int64_t>(p.w_tiles) * p.tok_tiles * p.kc_per_tile / p.unit;
@@ -414,8 +414,7 @@ cudaError_t launch_i8_pair(I8PairParams p, const CUtensorMap& wmap, const CUtens
   const int64_t pairs = p.split > 1 ? static_cast<int64_t>(p.w_tiles) * p.tok_tiles * p.split
                         : total < num_sms / 2 ? total : num_sms / 2;
   auto* kern = p.split > 1 ? woq_i8_pair_kernel<true> : woq_i8_pair_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem));
+  cudaError_t e = allow_max_smem(kern);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(pairs * 2));

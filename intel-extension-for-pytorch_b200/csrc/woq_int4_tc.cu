@@ -630,9 +630,7 @@ size_t tc_plan(TcParams& p) {
 cudaError_t launch_int4_tc(TcParams p, const CUtensorMap& xmap, int grid, cudaStream_t stream) {
   const size_t smem = tc_plan(p);
   if (smem == 0) return cudaErrorInvalidConfiguration;
-  cudaError_t e = cudaFuncSetAttribute(woq_int4_tc_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem));
+  cudaError_t e = allow_max_smem(woq_int4_tc_kernel);
   if (e != cudaSuccess) return e;
   woq_int4_tc_kernel<<<grid, kTcThreads, smem, stream>>>(p, xmap);
   return cudaGetLastError();

@@ -127,6 +127,14 @@ struct TcParams {
 // the M <= 16 kernel's launches opt into programmatic dependent launch unless WOQ_B200_PDL=0 was
 // set before first use (the tcgen05 kernels launch plainly)
 bool dependent_launch_enabled();
+// Lets `kern` (no static shared memory) be launched with all the shared memory a block can have.  Always the same
+// limit, set before each launch: with the launch's own size, two host threads with different token counts could
+// interleave so that one launches above the limit the other has just set.
+constexpr int kMaxSmemBytes = 227 * 1024;
+template <class K>
+inline cudaError_t allow_max_smem(K* kern) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmemBytes);
+}
 int tc_pick_grid(int tiles, int kb_per_tile, int num_sms);
 size_t tc_partial_bytes(int grid, int n_tok);
 size_t tc_plan(TcParams& p);  // fills a_col0, kbs, stages, w_ring from n_tok; returns the dynamic shared memory (0: none)

@@ -680,7 +680,7 @@ int pair_group_columns(const int64_t* rows, int groups) {
 //     at least step stages.
 size_t pair_plan(PairParams& p) {
   const int lut = p.kind == kWeightNf4 ? kNf4LutBytes : 0;
-  const int budget = 227 * 1024 - kPairHeaderBytes - lut - p.n_tok * kOutPitch;
+  const int budget = kMaxSmemBytes - kPairHeaderBytes - lut - p.n_tok * kOutPitch;
   p.kbs = p.n_tok <= 128 ? 4 : 2;
   p.kpw = p.kbs == 4 && (p.n_tok < 128 || pair_block_bytes(p.kind) == kTcBlockBytes) ? 2 : 1;
   const int step = kDeqGroups * p.kpw / p.kbs;
@@ -725,7 +725,7 @@ static int pair_cluster_capacity(int ctas) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(ctas * 32));
   cfg.blockDim = dim3(kPairThreads);
-  cfg.dynamicSmemBytes = 227 * 1024;
+  cfg.dynamicSmemBytes = kMaxSmemBytes;
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
   attr.val.clusterDim.x = ctas;
@@ -734,7 +734,7 @@ static int pair_cluster_capacity(int ctas) {
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
   int clusters = 0;
-  if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
+  if (allow_max_smem(kern) != cudaSuccess ||
       cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
     cudaGetLastError();
     clusters = 0;
@@ -769,8 +769,7 @@ cudaError_t launch_pair(PairParams p, const CUtensorMap& xmap, int num_sms, cuda
     case kWeightNf4: kern = pick_pair_kernel<kWeightNf4>(p); break;
     default: return cudaErrorInvalidValue;
   }
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem));
+  cudaError_t e = allow_max_smem(kern);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   if (p.split > 1 && (p.n_groups != 1 || (p.kb_per_tile + p.kbs - 1) / p.kbs < p.split ||
