@@ -596,6 +596,12 @@ bool moe_grouped(const std::vector<c10::intrusive_ptr<WoqLinearOpContext>>& ctxs
   return true;
 }
 
+int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
+
+// Scratch of a mixture-of-experts call: three tensors with a row for every (token, slot) pair.  Long batches go
+// through in slabs of tokens that stay below this (8192 pairs of Mixtral-8x7B's layer, 1024 for each expert).
+constexpr int64_t kMoeScratchBytes = 512ll << 20;
+
 // reference: csrc/cpu/aten/MoE.cpp:290-330.  topk_ids [tokens, top_k] names each token's experts; every
 // selected expert runs gate, up, silu * up and down on its tokens, and the results are added to the output
 // in expert order with their routing weights.
@@ -632,70 +638,78 @@ at::Tensor deepseek_moe_woq(const at::Tensor& hidden_states, const at::Tensor& t
     c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(dev));
     cudaStream_t stream = at::cuda::getCurrentCUDAStream(dev).stream();
     flat = flat.contiguous();
-    const auto ints = flat.options().dtype(at::kInt);
-    at::Tensor dcounts = at::empty({experts + 1}, ints), token_of = at::empty({pairs}, ints);
-    at::Tensor pos_of = at::empty({pairs}, ints);
-    WOQ_CHECK(woq_b200_moe_route(flat.data_ptr<int64_t>(), tokens, static_cast<int32_t>(top_k),
-                                 static_cast<int32_t>(experts), dcounts.data_ptr<int32_t>(),
-                                 token_of.data_ptr<int32_t>(), pos_of.data_ptr<int32_t>(), stream));
     at::Tensor w = routing_weights.to(hidden_states.device(), at::kBFloat16).contiguous();
-    at::Tensor counts = dcounts.cpu();
-    const int32_t* cnt = counts.data_ptr<int32_t>();
-    TORCH_CHECK(cnt[experts] == 0, "WOQ: topk_ids names an expert beyond the contexts given");
-    auto rows_of = [&](int64_t width) { return at::empty({pairs, width}, hidden_states.options()); };
-    at::Tensor x = rows_of(hidden), gate = rows_of(ffn), act = rows_of(ffn), res = rows_of(hidden);
-    WOQ_CHECK(woq_b200_gather_rows(hidden_states.data_ptr(), hidden, token_of.data_ptr<int32_t>(), pairs, hidden,
-                                   x.data_ptr(), stream));
-    int32_t most = 0;
-    for (int64_t e = 0; e < experts; ++e) most = std::max(most, cnt[e]);
-    auto row = [](const at::Tensor& t, int64_t r) { return static_cast<uint8_t*>(t.data_ptr()) + r * t.size(1) * 2; };
-    if (most > 16) {
-      at::Tensor up = rows_of(ffn);
-      std::vector<const woq_b200_ctx*> gu, d;
-      std::vector<int64_t> row0, rows, row0d, rowsd;
-      std::vector<void*> y, yd;
-      int64_t off = 0;
-      for (int64_t e = 0; e < experts; ++e) {
-        if (cnt[e] == 0) continue;
-        for (const auto* c : {&gate_ctx[e], &up_ctx[e]}) {
-          gu.push_back((*c)->ctx_for(17));  // the tensor-core tiling
-          row0.push_back(off);
-          rows.push_back(cnt[e]);
-          y.push_back(row(c == &gate_ctx[e] ? gate : up, off));
-        }
-        d.push_back(down_ctx[e]->ctx_for(17));
-        row0d.push_back(off);
-        rowsd.push_back(cnt[e]);
-        yd.push_back(row(res, off));
-        off += cnt[e];
-      }
-      at::Tensor ws = workspace_for(dev, stream, woq_b200_workspace_bytes(gu[0], std::max<int64_t>(17, most)));
-      WOQ_CHECK(woq_b200_linear_grouped(gu.data(), row0.data(), rows.data(), y.data(), static_cast<int32_t>(gu.size()),
-                                        x.data_ptr(), pairs, hidden, ffn, ws.data_ptr(), ws.numel(), stream));
-      WOQ_CHECK(woq_b200_silu_mul(gate.data_ptr(), up.data_ptr(), act.data_ptr(), pairs * ffn, stream));
-      WOQ_CHECK(woq_b200_linear_grouped(d.data(), row0d.data(), rowsd.data(), yd.data(),
-                                        static_cast<int32_t>(d.size()), act.data_ptr(), pairs, ffn, hidden,
-                                        ws.data_ptr(), ws.numel(), stream));
-    } else {
-      int64_t off = 0;
-      for (int64_t e = 0; e < experts; ++e) {
-        if (cnt[e] == 0) continue;
-        auto linear = [&](const c10::intrusive_ptr<WoqLinearOpContext>& c, const at::Tensor& in, int32_t fusion,
-                          const void* other, const at::Tensor& out) {
-          woq_b200_ctx* k = c->ctx_for(cnt[e]);
-          at::Tensor ws = workspace_for(dev, stream, woq_b200_workspace_bytes(k, cnt[e]));
-          WOQ_CHECK(woq_b200_linear(k, row(in, off), cnt[e], in.size(1), fusion, other ? &other : nullptr,
-                                    other ? 1 : 0, row(out, off), out.size(1), ws.data_ptr(), ws.numel(), stream));
-        };
-        linear(gate_ctx[e], x, WOQ_B200_FUSE_SILU, nullptr, gate);
-        linear(up_ctx[e], x, WOQ_B200_FUSE_MUL, row(gate, off), act);
-        linear(down_ctx[e], act, WOQ_B200_FUSE_NONE, nullptr, res);
-        off += cnt[e];
-      }
-    }
     at::Tensor output = at::empty_like(hidden_states);
-    WOQ_CHECK(woq_b200_moe_combine(res.data_ptr(), flat.data_ptr<int64_t>(), pos_of.data_ptr<int32_t>(), w.data_ptr(),
-                                   tokens, static_cast<int32_t>(top_k), hidden, output.data_ptr(), stream));
+    // equal slabs of tokens whose rows below fit the scratch bound
+    const int64_t fit = std::max<int64_t>(1, kMoeScratchBytes / (2 * (hidden + 2 * ffn) * top_k));
+    const int64_t slab = ceil_div(tokens, ceil_div(tokens, fit));
+    const auto ints = flat.options().dtype(at::kInt);
+    at::Tensor dcounts = at::empty({experts + 1}, ints), token_of = at::empty({slab * top_k}, ints);
+    at::Tensor pos_of = at::empty({slab * top_k}, ints);
+    auto rows_of = [&](int64_t width) { return at::empty({slab * top_k, width}, hidden_states.options()); };
+    // the gathered tokens, then the experts' results; gate; up, then silu(gate) * up
+    at::Tensor x = rows_of(hidden), gate = rows_of(ffn), act = rows_of(ffn);
+    auto row = [](const at::Tensor& t, int64_t r) { return static_cast<uint8_t*>(t.data_ptr()) + r * t.size(1) * 2; };
+    for (int64_t t0 = 0; t0 < tokens; t0 += slab) {
+      const int64_t nt = std::min(slab, tokens - t0), np = nt * top_k;
+      const int64_t* ids = flat.data_ptr<int64_t>() + t0 * top_k;
+      WOQ_CHECK(woq_b200_moe_route(ids, nt, static_cast<int32_t>(top_k), static_cast<int32_t>(experts),
+                                   dcounts.data_ptr<int32_t>(), token_of.data_ptr<int32_t>(),
+                                   pos_of.data_ptr<int32_t>(), stream));
+      at::Tensor counts = dcounts.cpu();
+      const int32_t* cnt = counts.data_ptr<int32_t>();
+      TORCH_CHECK(cnt[experts] == 0, "WOQ: topk_ids names an expert beyond the contexts given");
+      WOQ_CHECK(woq_b200_gather_rows(row(hidden_states, t0), hidden, token_of.data_ptr<int32_t>(), np, hidden,
+                                     x.data_ptr(), stream));
+      int32_t most = 0;
+      for (int64_t e = 0; e < experts; ++e) most = std::max(most, cnt[e]);
+      if (most > 16) {
+        std::vector<const woq_b200_ctx*> gu, d;
+        std::vector<int64_t> row0, rows, row0d, rowsd;
+        std::vector<void*> y, yd;
+        int64_t off = 0;
+        for (int64_t e = 0; e < experts; ++e) {
+          if (cnt[e] == 0) continue;
+          for (const auto* c : {&gate_ctx[e], &up_ctx[e]}) {
+            gu.push_back((*c)->ctx_for(17));  // the tensor-core tiling
+            row0.push_back(off);
+            rows.push_back(cnt[e]);
+            y.push_back(row(c == &gate_ctx[e] ? gate : act, off));
+          }
+          d.push_back(down_ctx[e]->ctx_for(17));
+          row0d.push_back(off);
+          rowsd.push_back(cnt[e]);
+          yd.push_back(row(x, off));
+          off += cnt[e];
+        }
+        at::Tensor ws = workspace_for(dev, stream, woq_b200_workspace_bytes(gu[0], std::max<int64_t>(17, most)));
+        WOQ_CHECK(woq_b200_linear_grouped(gu.data(), row0.data(), rows.data(), y.data(),
+                                          static_cast<int32_t>(gu.size()), x.data_ptr(), np, hidden, ffn,
+                                          ws.data_ptr(), ws.numel(), stream));
+        WOQ_CHECK(woq_b200_silu_mul(gate.data_ptr(), act.data_ptr(), act.data_ptr(), np * ffn, stream));
+        WOQ_CHECK(woq_b200_linear_grouped(d.data(), row0d.data(), rowsd.data(), yd.data(),
+                                          static_cast<int32_t>(d.size()), act.data_ptr(), np, ffn, hidden,
+                                          ws.data_ptr(), ws.numel(), stream));
+      } else {
+        int64_t off = 0;
+        for (int64_t e = 0; e < experts; ++e) {
+          if (cnt[e] == 0) continue;
+          auto linear = [&](const c10::intrusive_ptr<WoqLinearOpContext>& c, const at::Tensor& in, int32_t fusion,
+                            const void* other, const at::Tensor& out) {
+            woq_b200_ctx* k = c->ctx_for(cnt[e]);
+            at::Tensor ws = workspace_for(dev, stream, woq_b200_workspace_bytes(k, cnt[e]));
+            WOQ_CHECK(woq_b200_linear(k, row(in, off), cnt[e], in.size(1), fusion, other ? &other : nullptr,
+                                      other ? 1 : 0, row(out, off), out.size(1), ws.data_ptr(), ws.numel(), stream));
+          };
+          linear(gate_ctx[e], x, WOQ_B200_FUSE_SILU, nullptr, gate);
+          linear(up_ctx[e], x, WOQ_B200_FUSE_MUL, row(gate, off), act);
+          linear(down_ctx[e], act, WOQ_B200_FUSE_NONE, nullptr, x);
+          off += cnt[e];
+        }
+      }
+      WOQ_CHECK(woq_b200_moe_combine(x.data_ptr(), ids, pos_of.data_ptr<int32_t>(),
+                                     row(w, t0), nt, static_cast<int32_t>(top_k), hidden, row(output, t0), stream));
+    }
     return output;
   }
 

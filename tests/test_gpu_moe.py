@@ -206,3 +206,36 @@ def test_deepseek_moe_expert_counts(env, tokens, experts, top_k):
     bad[tokens // 2, 0] = experts
     with pytest.raises(RuntimeError):
         torch.ops.torch_ipex.deepseek_moe_woq(x, bad, gate, up, down, w, False)
+
+
+def moe_layer(env, hidden, ffn, g, experts, gen):
+    def ctx(n, k):
+        w = torch.randn((n, k), device="cuda", generator=gen) * 0.05
+        q, s, z = env.quantization.quantize_per_block(w, 2, g)
+        return torch.ops.ipex_prepack.weight_only_qlinear_prepack(q, 2, [n, k], s, z, None, None, None, g, 2, -1)
+
+    return [[ctx(n, k) for _ in range(experts)] for n, k in ((ffn, hidden), (ffn, hidden), (hidden, ffn))]
+
+
+def test_deepseek_moe_scratch_is_bounded(env):
+    """A long batch goes through in slabs: 1.5 GB of rows, 512 MiB of scratch; every token gets what it gets in a
+    batch of its own (another cut of the sums at most)."""
+    hidden, ffn, experts, tokens = 1024, 4096, 4, 40000
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    gate, up, down = moe_layer(env, hidden, ffn, 128, experts, gen)
+    x = torch.randn((tokens, hidden), device="cuda", generator=gen).bfloat16()
+    w, ids = torch.topk(torch.softmax(torch.randn((tokens, experts), device="cuda", generator=gen), -1), 2, -1)
+    w = w.bfloat16()
+    parts = [torch.ops.torch_ipex.deepseek_moe_woq(x[t:t + 999], ids[t:t + 999], gate, up, down, w[t:t + 999], False)
+             for t in range(0, tokens, 999)]
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    out = torch.ops.torch_ipex.deepseek_moe_woq(x, ids, gate, up, down, w, False)
+    torch.cuda.synchronize()
+    # the output, 12 bytes of routing for each pair, and the scratch
+    assert torch.cuda.max_memory_allocated() - before <= (512 << 20) + out.numel() * 2 + tokens * 2 * 12 + (2 << 20)
+    ref = torch.cat(parts).float()
+    # a sum that rounds to the neighbouring bf16 value moves a product and an addition by one unit each
+    assert (out.float() - ref).norm() <= 4e-3 * ref.norm()
+    assert ((out.float() - ref).norm(dim=1) <= 2e-2 * ref.norm(dim=1)).all()
