@@ -607,12 +607,12 @@ constexpr int64_t kMoeScratchBytes = 512ll << 20;
 // in expert order with their routing weights.
 //
 // The (token, slot) pairs are sorted by expert on the device; the per-expert counts come to the host, which
-// shapes the launches with them (and refuses ids that name no expert).  When an expert has more than 16
-// tokens, all gate and up projections are one launch and all down projections another: an expert's linear
+// shapes the launches with them (and refuses ids that name no expert).  All gate and up projections of the
+// experts with more than 16 tokens are one launch and all their down projections another: an expert's linear
 // alone is too small to fill the GPU for long (Mixtral-8x7B's layer, 256 tokens: 996 us expert by expert, 350 in
-// two grouped launches).  Up to 16 tokens the streaming kernel runs expert by expert, so that a model that only decodes
-// keeps one copy of its weights.  Everything else (other weight types, act-order, ...) goes through the
-// per-expert operator above.
+// two grouped launches).  The experts with up to 16 tokens run one after another on the streaming kernel: the
+// grouped launch needs the second tiling of a weight, which only an expert that has had more than 16 tokens gets.
+// Everything else (other weight types, act-order, ...) goes through the per-expert operator above.
 at::Tensor deepseek_moe_woq(const at::Tensor& hidden_states, const at::Tensor& topk_ids,
                             const std::vector<c10::intrusive_ptr<WoqLinearOpContext>>& gate_ctx,
                             const std::vector<c10::intrusive_ptr<WoqLinearOpContext>>& up_ctx,
@@ -661,52 +661,56 @@ at::Tensor deepseek_moe_woq(const at::Tensor& hidden_states, const at::Tensor& t
       TORCH_CHECK(cnt[experts] == 0, "WOQ: topk_ids names an expert beyond the contexts given");
       WOQ_CHECK(woq_b200_gather_rows(row(hidden_states, t0), hidden, token_of.data_ptr<int32_t>(), np, hidden,
                                      x.data_ptr(), stream));
+      std::vector<const woq_b200_ctx*> gu, d;
+      std::vector<int64_t> row0, rows, row0d, rowsd, few, few_row;  // few: experts of at most 16 tokens
+      std::vector<void*> y, yd;
       int32_t most = 0;
-      for (int64_t e = 0; e < experts; ++e) most = std::max(most, cnt[e]);
-      if (most > 16) {
-        std::vector<const woq_b200_ctx*> gu, d;
-        std::vector<int64_t> row0, rows, row0d, rowsd;
-        std::vector<void*> y, yd;
-        int64_t off = 0;
-        for (int64_t e = 0; e < experts; ++e) {
-          if (cnt[e] == 0) continue;
-          for (const auto* c : {&gate_ctx[e], &up_ctx[e]}) {
-            gu.push_back((*c)->ctx_for(17));  // the tensor-core tiling
-            row0.push_back(off);
-            rows.push_back(cnt[e]);
-            y.push_back(row(c == &gate_ctx[e] ? gate : act, off));
-          }
-          d.push_back(down_ctx[e]->ctx_for(17));
-          row0d.push_back(off);
-          rowsd.push_back(cnt[e]);
-          yd.push_back(row(x, off));
-          off += cnt[e];
+      for (int64_t e = 0, off = 0; e < experts; off += cnt[e++]) {
+        if (cnt[e] == 0) continue;
+        if (cnt[e] <= 16) {
+          few.push_back(e);
+          few_row.push_back(off);
+          continue;
         }
-        at::Tensor ws = workspace_for(dev, stream, woq_b200_workspace_bytes(gu[0], std::max<int64_t>(17, most)));
+        most = std::max(most, cnt[e]);
+        for (const auto* c : {&gate_ctx[e], &up_ctx[e]}) {
+          gu.push_back((*c)->ctx_for(cnt[e]));
+          row0.push_back(off);
+          rows.push_back(cnt[e]);
+          y.push_back(row(c == &gate_ctx[e] ? gate : act, off));
+        }
+        d.push_back(down_ctx[e]->ctx_for(cnt[e]));
+        row0d.push_back(off);
+        rowsd.push_back(cnt[e]);
+        yd.push_back(row(x, off));
+      }
+      at::Tensor ws;
+      if (most > 0) {
+        ws = workspace_for(dev, stream, woq_b200_workspace_bytes(gu[0], most));
         WOQ_CHECK(woq_b200_linear_grouped(gu.data(), row0.data(), rows.data(), y.data(),
                                           static_cast<int32_t>(gu.size()), x.data_ptr(), np, hidden, ffn,
                                           ws.data_ptr(), ws.numel(), stream));
+        // (all rows: those of the other experts hold nothing yet)
         WOQ_CHECK(woq_b200_silu_mul(gate.data_ptr(), act.data_ptr(), act.data_ptr(), np * ffn, stream));
+      }
+      for (size_t i = 0; i < few.size(); ++i) {
+        const int64_t e = few[i], off = few_row[i];
+        auto linear = [&](const c10::intrusive_ptr<WoqLinearOpContext>& c, const at::Tensor& in, int32_t fusion,
+                          const void* other, const at::Tensor& out) {
+          woq_b200_ctx* k = c->ctx_for(cnt[e]);
+          at::Tensor scratch = workspace_for(dev, stream, woq_b200_workspace_bytes(k, cnt[e]));
+          WOQ_CHECK(woq_b200_linear(k, row(in, off), cnt[e], in.size(1), fusion, other ? &other : nullptr,
+                                    other ? 1 : 0, row(out, off), out.size(1), scratch.data_ptr(), scratch.numel(),
+                                    stream));
+        };
+        linear(gate_ctx[e], x, WOQ_B200_FUSE_SILU, nullptr, gate);
+        linear(up_ctx[e], x, WOQ_B200_FUSE_MUL, row(gate, off), act);
+        linear(down_ctx[e], act, WOQ_B200_FUSE_NONE, nullptr, x);
+      }
+      if (most > 0)
         WOQ_CHECK(woq_b200_linear_grouped(d.data(), row0d.data(), rowsd.data(), yd.data(),
                                           static_cast<int32_t>(d.size()), act.data_ptr(), np, ffn, hidden,
                                           ws.data_ptr(), ws.numel(), stream));
-      } else {
-        int64_t off = 0;
-        for (int64_t e = 0; e < experts; ++e) {
-          if (cnt[e] == 0) continue;
-          auto linear = [&](const c10::intrusive_ptr<WoqLinearOpContext>& c, const at::Tensor& in, int32_t fusion,
-                            const void* other, const at::Tensor& out) {
-            woq_b200_ctx* k = c->ctx_for(cnt[e]);
-            at::Tensor ws = workspace_for(dev, stream, woq_b200_workspace_bytes(k, cnt[e]));
-            WOQ_CHECK(woq_b200_linear(k, row(in, off), cnt[e], in.size(1), fusion, other ? &other : nullptr,
-                                      other ? 1 : 0, row(out, off), out.size(1), ws.data_ptr(), ws.numel(), stream));
-          };
-          linear(gate_ctx[e], x, WOQ_B200_FUSE_SILU, nullptr, gate);
-          linear(up_ctx[e], x, WOQ_B200_FUSE_MUL, row(gate, off), act);
-          linear(down_ctx[e], act, WOQ_B200_FUSE_NONE, nullptr, x);
-          off += cnt[e];
-        }
-      }
       WOQ_CHECK(woq_b200_moe_combine(x.data_ptr(), ids, pos_of.data_ptr<int32_t>(),
                                      row(w, t0), nt, static_cast<int32_t>(top_k), hidden, row(output, t0), stream));
     }

@@ -239,3 +239,30 @@ def test_deepseek_moe_scratch_is_bounded(env):
     # a sum that rounds to the neighbouring bf16 value moves a product and an addition by one unit each
     assert (out.float() - ref).norm() <= 4e-3 * ref.norm()
     assert ((out.float() - ref).norm(dim=1) <= 2e-2 * ref.norm(dim=1)).all()
+
+
+def test_deepseek_moe_second_tiling_only_where_needed(env):
+    """One expert with 40 tokens among experts with 8: only its three weights are packed a second time."""
+    hidden, ffn, experts = 2048, 4096, 4
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    gate, up, down = moe_layer(env, hidden, ffn, 128, experts, gen)
+    x = torch.randn((64, hidden), device="cuda", generator=gen).bfloat16()
+    w = torch.ones((64, 1), device="cuda").bfloat16()
+
+    def call(ids):
+        n = len(ids)
+        out = torch.ops.torch_ipex.deepseek_moe_woq(x[:n], torch.tensor(ids, device="cuda")[:, None], gate, up, down,
+                                                    w[:n], False)
+        torch.cuda.synchronize()
+        free, total = torch.cuda.mem_get_info()
+        return out, total - free - torch.cuda.memory_reserved()
+
+    few = [e for e in range(experts) for _ in range(8)]
+    out0, before = call(few)
+    out1, after = call(few + [2] * 32)
+    copy = sum((c.get_weight().numel() + (1 << 21)) for c in (gate[2], up[2], down[2]))  # (cudaMalloc granularity)
+    assert copy // 2 < after - before <= 2 * copy
+    # the other experts' tokens are untouched by how expert 2 runs
+    keep = [i for i, e in enumerate(few) if e != 2]
+    assert torch.equal(out0[keep], out1[keep])
+    assert (out0.float() - out1[:32].float()).norm() <= 4e-3 * out0.float().norm()
