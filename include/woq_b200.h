@@ -444,6 +444,17 @@ int woq_b200_decode_plan(const woq_b200_ctx* ctx, int64_t m, int32_t* out);
  * shared memory in bytes. */
 int woq_b200_tc_plan(int32_t n_tok, int32_t* out);
 
+/* The pipeline shape of a launch of the CTA-pair kernel (more than 16 tokens of INT4 weights; INT8 and NF4 weights
+ * with bf16 compute) with `columns` token columns (32..256, a multiple of 32) on `tiles` (256 rows x columns) of K
+ * each.  A diagnostic that needs no GPU: out[0] k-blocks per stage, out[1] k-blocks a dequantising warpgroup
+ * takes per visit, out[2] slots of the A-operand / activation ring, out[3] slots of the packed-weight ring (a
+ * multiple of the stages between two visits of a warpgroup, 4 * out[1] / out[0]; the A ring is at least as long), out[4]
+ * k-blocks that shares of the k sequence are multiples of, out[5] dynamic shared memory in bytes. */
+int woq_b200_pair_plan(int32_t weight_dtype, int32_t columns, int64_t tiles, int64_t k, int32_t num_sms, int32_t* out);
+
+/* The token columns woq_b200_linear_grouped takes for groups of these many rows (a diagnostic; needs no GPU). */
+int woq_b200_grouped_columns(const int64_t* rows, int32_t groups, int32_t* columns);
+
 /* Reads the status word of a workspace (synchronises the stream).  WOQ_B200_OK, or
  * WOQ_B200_ERR_DEVICE_WAIT when a bounded wait inside a kernel gave up; the word is cleared. */
 int woq_b200_workspace_status(void* workspace, void* stream);

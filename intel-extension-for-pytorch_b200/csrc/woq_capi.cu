@@ -1167,7 +1167,7 @@ static int run_pair(const woq_b200_ctx* c, const void* x, int64_t m, int64_t ldx
   if (fusion == WOQ_B200_FUSE_SILU_MUL) p.n_out = (int)(c->desc.n / 2);
   p.fusion = fusion;
   p.vec = ldy % 8 == 0 && aligned16(y) && (!o0 || aligned16(o0)) && (!o1 || aligned16(o1));
-  if (woq::pair_plan(p) == 0) return fail(WOQ_B200_ERR_UNSUPPORTED, "no pipeline shape for %d token columns", p.n_tok);
+  if (woq::pair_plan(p, c->num_sms) == 0) return fail(WOQ_B200_ERR_UNSUPPORTED, "no pipeline shape for %d token columns", p.n_tok);
   CUtensorMap xmap;
   if (int rc = make_kblock_map(&xmap, x, m, c->desc.k, ldx, 2, p.n_tok / 2, p.kbs)) return rc;
   CUDA_TRY(woq::launch_pair(p, xmap, c->num_sms, stream));
@@ -1204,7 +1204,7 @@ int woq_b200_linear_grouped(const woq_b200_ctx* const* ctxs, const int64_t* row0
   if (total_rows > (1ll << 30) || ldx < c0->desc.k || (ldx % 8) != 0 || !aligned16(x))
     return fail(WOQ_B200_ERR_INVALID_ARG, "x must be 16-byte aligned with ldx >= K and ldx %% 8 == 0");
   if (ldy < c0->desc.n) return fail(WOQ_B200_ERR_INVALID_ARG, "ldy smaller than the output width");
-  const int n_tok = woq::pair_group_columns(rows, groups);
+  const int n_tok = woq::pair_group_columns(rows, groups, in_place ? woq::kWeightInt4InPlace : woq::kWeightInt4);
   const size_t need = kWsHeaderBytes + woq::pair_partial_bytes(c0->num_sms, most < n_tok ? (int)most : n_tok);
   if (workspace_bytes < need) return fail(WOQ_B200_ERR_WORKSPACE, "workspace has %zu bytes, need %zu", workspace_bytes, need);
   CUtensorMap xmap;
@@ -1219,7 +1219,7 @@ int woq_b200_linear_grouped(const woq_b200_ctx* const* ctxs, const int64_t* row0
       add_pair_group(ctxs[g], &p, row0[g], rows[g], y[g]);
       p.vec = p.vec && aligned16(y[g]);
     }
-    if (woq::pair_plan(p) == 0) return fail(WOQ_B200_ERR_UNSUPPORTED, "no pipeline shape for %d token columns", n_tok);
+    if (woq::pair_plan(p, c0->num_sms) == 0) return fail(WOQ_B200_ERR_UNSUPPORTED, "no pipeline shape for %d token columns", n_tok);
     if (g0 == 0)
       if (int rc = make_kblock_map(&xmap, x, total_rows, c0->desc.k, ldx, 2, n_tok / 2, p.kbs)) return rc;
     CUDA_TRY(woq::launch_pair(p, xmap, c0->num_sms, static_cast<cudaStream_t>(stream_)));
@@ -1986,6 +1986,39 @@ int woq_b200_tc_plan(int32_t n_tok, int32_t* out) {
   out[2] = p.w_ring;
   out[3] = p.a_col0;
   out[4] = static_cast<int32_t>(smem);
+  return WOQ_B200_OK;
+}
+
+int woq_b200_pair_plan(int32_t weight_dtype, int32_t columns, int64_t tiles, int64_t k, int32_t num_sms, int32_t* out) {
+  int kind = -1;
+  switch (weight_dtype) {
+    case WOQ_B200_DTYPE_INT4: kind = woq::kWeightInt4; break;
+    case WOQ_B200_DTYPE_INT8: kind = woq::kWeightInt8; break;
+    case WOQ_B200_DTYPE_NF4: kind = woq::kWeightNf4; break;
+  }
+  if (!out || kind < 0 || columns < 32 || columns > 256 || (columns & 31) || tiles < 1 || tiles >= (1ll << 31) ||
+      k < 64 || k % 64 || num_sms < 2)
+    return fail(WOQ_B200_ERR_INVALID_ARG, "CTA-pair plan: INT4, INT8 or NF4 weights, token columns 32..256, a multiple "
+                "of 32, at least one tile, K a multiple of 64");
+  woq::PairParams p{};
+  p.kind = kind;
+  p.n_tok = columns;
+  p.items = (int)tiles;
+  p.kb_per_tile = (int)(k / 64);
+  const size_t smem = woq::pair_plan(p, num_sms);
+  if (smem == 0) return fail(WOQ_B200_ERR_UNSUPPORTED, "no pipeline shape for %d token columns", (int)columns);
+  out[0] = p.kbs;
+  out[1] = p.kpw;
+  out[2] = p.stages;
+  out[3] = p.w_ring;
+  out[4] = p.unit;
+  out[5] = static_cast<int32_t>(smem);
+  return WOQ_B200_OK;
+}
+
+int woq_b200_grouped_columns(const int64_t* rows, int32_t groups, int32_t* columns) {
+  if (!rows || !columns || groups < 1) return fail(WOQ_B200_ERR_INVALID_ARG, "grouped columns: null pointer or no group");
+  *columns = woq::pair_group_columns(rows, groups, woq::kWeightInt4InPlace);
   return WOQ_B200_OK;
 }
 

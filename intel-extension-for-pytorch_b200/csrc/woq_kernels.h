@@ -192,8 +192,8 @@ struct PairCut {
   int n_tok, tok_tiles, whole, split;  // split > 1: so many pairs, a cluster, share each tile
 };
 PairCut pair_cut(int64_t m, int w_tiles, int k_steps, int pairs, int kind);
-int pair_group_columns(const int64_t* rows, int groups);
-size_t pair_plan(PairParams& p);  // fills kbs, stages, w_ring, unit; dynamic shared memory (0: none)
+int pair_group_columns(const int64_t* rows, int groups, int kind);
+size_t pair_plan(PairParams& p, int num_sms);  // fills kbs, stages, w_ring, unit; dynamic shared memory (0: none)
 size_t pair_partial_bytes(int num_sms, int part_tok);
 cudaError_t launch_pair(PairParams p, const CUtensorMap& xmap, int num_sms, cudaStream_t stream);
 

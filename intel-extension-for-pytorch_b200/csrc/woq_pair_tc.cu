@@ -605,11 +605,21 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 
 }  // namespace
 
-// Token tiles of a call, and how its tiles are dealt, by estimated time in us.  A k step costs a tile of n
-// columns the larger of its dequantisation and hand-overs (or, for INT8 compute, its L2 traffic) and its MMAs:
-// fitted to 57344 x 8192 INT4 (72 / 77 / 89 / 101 / 176 / 333 us at 32 / 64 / 96 / 128 / 256 / 512 tokens),
-// 57344 x 4096 INT8 with bf16 compute (44 / 52 / 68 us at 8 / 64 / 128) and INT8 compute on 28672 x 4096
-// (121 / 220 us at 1024 / 2048).  Whole tiles take as many rounds as the fullest pair has tiles.  Equal shares of the k sequence
+// What a k step costs a tile of n columns, in us: the larger of its dequantisation and hand-overs (or, for INT8
+// compute, its L2 traffic) and its MMAs.  Fitted to 57344 x 8192 INT4 (72 / 77 / 89 / 101 / 176 / 333 us at
+// 32 / 64 / 96 / 128 / 256 / 512 tokens), 57344 x 4096 INT8 with bf16 compute (44 / 52 / 68 us at 8 / 64 / 128) and
+// INT8 compute on 28672 x 4096 (121 / 220 us at 1024 / 2048).
+static double pair_step_us(int kind, int n) {
+  const double mma = (kind == kPairCutInt8 ? 0.0011 : 0.0017) * n;
+  const double step = kind == kPairCutInt8                                    ? 0.26 + 0.001 * n
+                      : kind == kWeightInt4 || kind == kWeightInt4InPlace     ? 0.165 + 0.00075 * n
+                      : kind == kWeightNf4                                    ? 0.25 + 0.001 * n
+                                                                              : 0.19 + 0.00125 * n;
+  return step < mma ? mma : step;
+}
+
+// Token tiles of a call, and how its tiles are dealt, by estimated time.  Whole tiles take as many rounds as the
+// fullest pair has tiles.  Equal shares of the k sequence
 // keep every pair busy to the end, but then the parts of shared tiles go through the workspace, one after
 // another and behind the last MMA: 4096 x 4096, 1000 tokens took 46 us with shares for 25 us of MMAs.  With few
 // tiles, clusters of pairs split k (see SPLIT).
@@ -622,12 +632,7 @@ PairCut pair_cut(int64_t m, int w_tiles, int k_steps, int pairs, int kind) {
     int n = static_cast<int>(((m + t - 1) / t + 31) / 32 * 32);
     if (n < 32) n = 32;
     if ((m + n - 1) / n != t) continue;  // fewer tiles of this width do
-    const double mma = (kind == kPairCutInt8 ? 0.0011 : 0.0017) * n;
-    double step = kind == kPairCutInt8                                    ? 0.26 + 0.001 * n
-                  : kind == kWeightInt4 || kind == kWeightInt4InPlace     ? 0.165 + 0.00075 * n
-                  : kind == kWeightNf4                                    ? 0.25 + 0.001 * n
-                                                                          : 0.19 + 0.00125 * n;
-    if (step < mma) step = mma;
+    const double step = pair_step_us(kind, n);
     const int64_t items = static_cast<int64_t>(w_tiles) * t;
     const double shares = step * k_steps * items / pairs + 4 + 0.04 * n + 2.0 * pairs / items;
     const double rounds = step * k_steps * static_cast<double>((items + pairs - 1) / pairs);
@@ -647,14 +652,14 @@ PairCut pair_cut(int64_t m, int w_tiles, int k_steps, int pairs, int kind) {
 }
 
 // Token columns for several linears in one launch, by the number of tokens each has: the width with the least
-// sum over their tiles.  A k-block costs a tile about 120 + columns in units of a column's MMAs (8192 x 57344
-// weights: 91 us at 32 columns, 150 at 128, one tile each).
-int pair_group_columns(const int64_t* rows, int groups) {
+// sum over their tiles.
+int pair_group_columns(const int64_t* rows, int groups, int kind) {
   int best = 256;
-  int64_t best_cost = -1;
+  double best_cost = -1;
   for (int n = 256; n >= 32; n -= 32) {
-    int64_t cost = 0;
-    for (int g = 0; g < groups; ++g) cost += (rows[g] + n - 1) / n * (120 + n);
+    int64_t tiles = 0;
+    for (int g = 0; g < groups; ++g) tiles += (rows[g] + n - 1) / n;
+    const double cost = static_cast<double>(tiles) * pair_step_us(kind, n);
     if (best_cost < 0 || cost < best_cost) {
       best_cost = cost;
       best = n;
@@ -678,7 +683,7 @@ int pair_group_columns(const int64_t* rows, int groups) {
 //     slot to the same warpgroups every time; on the A / activation ring the wait for stage s - step (the
 //     MMAs of stage s - step - stages, which complete in order) covers stage s - 2 * stages when there are
 //     at least step stages.
-size_t pair_plan(PairParams& p) {
+size_t pair_plan(PairParams& p, int num_sms) {
   const int lut = p.kind == kWeightNf4 ? kNf4LutBytes : 0;
   const int budget = kMaxSmemBytes - kPairHeaderBytes - lut - p.n_tok * kOutPitch;
   p.kbs = p.n_tok <= 128 ? 4 : 2;
@@ -699,7 +704,7 @@ size_t pair_plan(PairParams& p) {
   p.w_ring = ring;
   // shares in whole stages where they are long enough for the rounding not to matter
   const int64_t total = static_cast<int64_t>(p.items) * p.kb_per_tile;
-  p.unit = p.whole ? p.kb_per_tile : p.kb_per_tile % p.kbs == 0 && total >= static_cast<int64_t>(74) * 8 * p.kbs ? p.kbs : 1;
+  p.unit = p.whole ? p.kb_per_tile : p.kb_per_tile % p.kbs == 0 && total >= static_cast<int64_t>(num_sms / 2) * 8 * p.kbs ? p.kbs : 1;
   return kPairHeaderBytes + static_cast<size_t>(stages) * x_stage + static_cast<size_t>(ring) * w_stage +
          static_cast<size_t>(p.n_tok) * kOutPitch + lut;
 }
@@ -754,7 +759,7 @@ static void (*pick_pair_kernel(const PairParams& p))(const PairParams, const CUt
 }
 
 cudaError_t launch_pair(PairParams p, const CUtensorMap& xmap, int num_sms, cudaStream_t stream) {
-  const size_t smem = pair_plan(p);
+  const size_t smem = pair_plan(p, num_sms);
   if (smem == 0) return cudaErrorInvalidConfiguration;
   if (p.kind == kWeightNf4) {
     static constexpr float values[16] = WOQ_NF4_VALUES;

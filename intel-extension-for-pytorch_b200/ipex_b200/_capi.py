@@ -51,6 +51,8 @@ EXPORTS = [
     "woq_b200_moe_workspace_bytes",
     "woq_b200_moe_expert",
     "woq_b200_linear_grouped",
+    "woq_b200_grouped_columns",
+    "woq_b200_pair_plan",
     "woq_b200_moe_route",
     "woq_b200_gather_rows",
     "woq_b200_silu_mul",
@@ -154,6 +156,8 @@ def lib() -> ctypes.CDLL:
     L.woq_b200_workspace_status.argtypes = [vp, vp]
     L.woq_b200_decode_plan.argtypes = [vp, i64, ctypes.POINTER(i32)]
     L.woq_b200_tc_plan.argtypes = [i32, ctypes.POINTER(i32)]
+    L.woq_b200_pair_plan.argtypes = [i32, i32, i64, i64, i32, ctypes.POINTER(i32)]
+    L.woq_b200_grouped_columns.argtypes = [ctypes.POINTER(i64), i32, ctypes.POINTER(i32)]
     L.woq_b200_comm_create.argtypes = [i32, i32, i64, sz, ctypes.POINTER(vp)]
     L.woq_b200_comm_export.argtypes = [vp, vp]
     L.woq_b200_comm_connect.argtypes = [vp, vp]
@@ -196,6 +200,20 @@ def tc_plan(n_tok: int) -> dict:
     out = (ctypes.c_int32 * 5)()
     _check(lib().woq_b200_tc_plan(n_tok, out))
     return {"kbs": out[0], "stages": out[1], "w_ring": out[2], "a_col0": out[3], "smem_bytes": out[4]}
+
+
+def pair_plan(weight_dtype: int, columns: int, tiles: int, k: int, num_sms: int = 148) -> dict:
+    """Pipeline shape of a launch of the CTA-pair kernel (woq_b200_pair_plan; no GPU needed)."""
+    out = (ctypes.c_int32 * 6)()
+    _check(lib().woq_b200_pair_plan(weight_dtype, columns, tiles, k, num_sms, out))
+    return dict(zip(("kbs", "kpw", "stages", "w_ring", "unit", "smem_bytes"), out))
+
+
+def grouped_columns(rows) -> int:
+    """Token columns of a grouped launch for groups of these many rows (woq_b200_grouped_columns; no GPU needed)."""
+    out = ctypes.c_int32()
+    _check(lib().woq_b200_grouped_columns((ctypes.c_int64 * len(rows))(*rows), len(rows), ctypes.byref(out)))
+    return out.value
 
 
 def static_scratch_status():

@@ -96,3 +96,46 @@ def test_tensor_core_pipeline_shapes_keep_the_ring_rules(built_lib):
     out = (ctypes.c_int32 * 5)()
     for bad in (0, 8, 24, 272):
         assert L.woq_b200_tc_plan(bad, out) == 1
+
+
+def test_pair_pipeline_shapes_keep_the_ring_rules(built_lib):
+    """woq_b200_pair_plan for every width and weight type: a packed-weight ring that is a multiple of the stages
+    between two visits of a warpgroup (each slot belongs to the same warpgroups), an A ring at least that long
+    (in-order MMAs then order its uses), A operands beside the accumulators in 512 TMEM columns, shared memory
+    within a CTA's 227 KB, and room for the partial tile of a cluster split over the rings."""
+    from ipex_b200 import _capi
+
+    for dtype, block in ((_capi.DTYPE_INT4, 4096), (_capi.DTYPE_NF4, 4096), (_capi.DTYPE_INT8, 8192)):
+        for n in range(32, 257, 32):
+            p = _capi.pair_plan(dtype, n, 1, 4096)
+            step = 4 * p["kpw"] // p["kbs"]
+            assert p["kbs"] == (4 if n <= 128 else 2) and 4 * p["kpw"] % p["kbs"] == 0, (n, p)
+            assert p["stages"] >= max(2, step) and p["w_ring"] >= 2 and p["w_ring"] % step == 0, (n, p)
+            assert n + 32 * p["kbs"] * p["stages"] <= 512, (n, p)
+            out_tile, lut = n * 272, 2048 if dtype == _capi.DTYPE_NF4 else 0
+            rings = p["stages"] * p["kbs"] * n // 2 * 128 + p["w_ring"] * p["kbs"] * (block + 512)
+            assert p["smem_bytes"] == 1024 + rings + out_tile + lut <= 227 * 1024, (n, p)
+            assert p["stages"] <= 8 and p["w_ring"] <= 24, (n, p)
+            assert n * 512 <= rings - 2048 + lut, (n, p)
+
+
+def test_pair_shares_follow_the_number_of_sms(built_lib):
+    """Shares are dealt in whole stages where every pair gets eight of them, on a GPU of any size."""
+    from ipex_b200 import _capi
+
+    for sms in (148, 132, 60):
+        pairs = sms // 2
+        tiles = pairs * 8 * 4 // 32  # of 32 k-blocks: eight stages of four for each pair
+        assert _capi.pair_plan(_capi.DTYPE_INT4, 64, tiles, 2048, sms)["unit"] == 4
+        assert _capi.pair_plan(_capi.DTYPE_INT4, 64, tiles - 1, 2048, sms)["unit"] == 1
+
+
+def test_grouped_columns_weigh_tiles_by_their_measured_cost(built_lib):
+    """A tile of 128 columns costs 101 / 72 of one of 32 (57344 x 8192, one tile each): four experts with 40 tokens
+    and one with 200 are six tiles of 128 columns, not eight of 64."""
+    from ipex_b200 import _capi
+
+    assert _capi.grouped_columns([40] * 4 + [200]) == 128
+    assert _capi.grouped_columns([20] * 8) == 32
+    assert _capi.grouped_columns([64] * 8) == 64
+    assert _capi.grouped_columns([1024] * 8) == 256
