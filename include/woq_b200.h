@@ -131,6 +131,14 @@ extern "C" {
 #define WOQ_B200_HINT_STREAM 2      /* register-dequant streaming kernel, 16 tokens a pass     */
 #define WOQ_B200_HINT_STREAM_FAST 3 /* streaming kernel, scale applied after the k-block sum   */
 
+/* OR-ed into kernel_hint, a diagnostic: every call of the context that runs on a CTA-pair kernel takes `columns` token
+ * columns per tile (a multiple of 32 up to 256; 0: chosen) and deals its tiles in a fixed way, where the library
+ * otherwise chooses by its estimate of the time.  `cut`: 0 chosen (with `columns`: equal shares), 1 equal shares of the
+ * k sequence (shared tiles are summed through the workspace), 2 whole tiles, 3 .. 5 clusters of 2 .. 4 pairs that
+ * split k (K of at least four k steps per pair; a k step is 64, INT8 compute 128).  Results differ in the order of the
+ * fp32 sums only. */
+#define WOQ_B200_HINT_PAIR(columns, cut) (((columns) << 16) | ((cut) << 8))
+
 /* Description of one quantised linear layer: the arguments of
  * ipex_prepack::weight_only_qlinear_prepack
  * (csrc/cpu/jit/cpu/kernels/RegisterOpContextClass.cpp:192-205). */
@@ -147,7 +155,7 @@ typedef struct woq_b200_desc {
                              int32 words (same packing as the weight) for GPTQ/AWQ         */
   int32_t bias_dtype;     /* NONE, F32 or BF16; bias is [N]                                 */
   int32_t layout_flags;   /* WOQ_B200_LAYOUT_*                                              */
-  int32_t kernel_hint;    /* WOQ_B200_HINT_*: 0 lets the library choose per call              */
+  int32_t kernel_hint;    /* WOQ_B200_HINT_*: 0 lets the library choose per call; | WOQ_B200_HINT_PAIR(..) */
 } woq_b200_desc;
 
 typedef struct woq_b200_ctx woq_b200_ctx; /* opaque; host memory owning device buffers */

@@ -968,7 +968,7 @@ static int run_decode(const woq_b200_ctx* c, const void* x, int64_t m, int64_t l
   // The scale-after-sum form only on request: it stays within the output tolerance for one
   // linear (mean relative deviation 1.2e-3 .. 1.7e-3 from the per-weight form, bar 2e-3) but
   // a product of two such linears (gate/up, woq_linear_silu followed by woq_linear_mul) does not.
-  const bool after_sum = c->desc.kernel_hint == WOQ_B200_HINT_STREAM_FAST;
+  const bool after_sum = (c->desc.kernel_hint & 0xff) == WOQ_B200_HINT_STREAM_FAST;
   p.exact = after_sum ? 0 : c->plain_scales ? 2 : 1;
 #ifdef WOQ_B200_TIMELINE
   {
@@ -1148,13 +1148,30 @@ static void add_pair_group(const woq_b200_ctx* c, woq::PairParams* p, int64_t ro
   if (part > p->part_tok) p->part_tok = part;
 }
 
+// How a call of `m` tokens is cut: by estimate, or as the context's WOQ_B200_HINT_PAIR asks.
+static int choose_pair_cut(const woq_b200_ctx* c, int64_t m, int w_tiles, int k_steps, int kind, woq::PairCut* cut) {
+  *cut = woq::pair_cut(m, w_tiles, k_steps, c->num_sms / 2, kind);
+  const int forced = (c->desc.kernel_hint >> 8) & 0xff, columns = (c->desc.kernel_hint >> 16) & 0xffff;
+  if (!forced && !columns) return WOQ_B200_OK;
+  if (forced > 5 || columns > 256 || columns % 32 || (forced > 2 && k_steps < 4 * (forced - 1)))
+    return fail(WOQ_B200_ERR_INVALID_ARG, "WOQ_B200_HINT_PAIR(%d, %d) does not fit K = %lld", columns, forced,
+                (long long)c->desc.k);
+  if (columns) *cut = woq::PairCut{columns, static_cast<int>((m + columns - 1) / columns), 0, 1};
+  if (forced) {
+    cut->whole = forced == 2;
+    cut->split = forced > 2 ? forced - 1 : 1;
+  }
+  return WOQ_B200_OK;
+}
+
 // One launch on CTA pairs, whatever the token count.
 static int run_pair(const woq_b200_ctx* c, const void* x, int64_t m, int64_t ldx, int32_t fusion, const void* o0,
                     const void* o1, const int32_t* row_idx, const void* row_w, void* y, int64_t ldy, uint8_t* w8,
                     cudaStream_t stream) {
   woq::PairParams p{};
   fill_pair(c, &p, w8);
-  const woq::PairCut cut = woq::pair_cut(m, p.w_tiles, p.kb_per_tile, c->num_sms / 2, p.kind);
+  woq::PairCut cut;
+  if (int rc = choose_pair_cut(c, m, p.w_tiles, p.kb_per_tile, p.kind, &cut)) return rc;
   p.n_tok = cut.n_tok;
   p.whole = cut.whole;
   p.split = cut.split;
@@ -1348,7 +1365,8 @@ static int run_int8_gemm(const woq_b200_ctx* c, const int8_t* qa, const float* s
   p.tiles = c->tiles_tc;
   p.w_tiles = (c->tiles_tc + 1) / 2;
   p.kc_per_tile = c->kc_per_tile;
-  const woq::PairCut cut = woq::pair_cut(m, p.w_tiles, p.kc_per_tile, c->num_sms / 2, woq::kPairCutInt8);
+  woq::PairCut cut;
+  if (int rc = choose_pair_cut(c, m, p.w_tiles, p.kc_per_tile, woq::kPairCutInt8, &cut)) return rc;
   p.n_tok = cut.n_tok;
   p.tok_tiles = cut.tok_tiles;
   p.unit = cut.whole ? p.kc_per_tile : 1;
@@ -1398,7 +1416,7 @@ static bool use_tc_path(const woq_b200_ctx* c, int64_t m) {
   }
   if (!c->wq_tc) return false;  // context packed for the streaming kernel only
   if (!c->wq) return true;      // context packed for the tensor-core kernel only
-  const int hint = c->desc.kernel_hint ? c->desc.kernel_hint : env;
+  const int own = c->desc.kernel_hint & 0xff, hint = own ? own : env;
   if (hint == WOQ_B200_HINT_TENSOR_CORE) return true;
   if (hint == WOQ_B200_HINT_STREAM || hint == WOQ_B200_HINT_STREAM_FAST) return false;
   return m > 16;

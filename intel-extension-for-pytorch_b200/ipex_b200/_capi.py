@@ -202,6 +202,15 @@ def tc_plan(n_tok: int) -> dict:
     return {"kbs": out[0], "stages": out[1], "w_ring": out[2], "a_col0": out[3], "smem_bytes": out[4]}
 
 
+# how a launch of a CTA-pair kernel deals its tiles (HINT_PAIR)
+PAIR_CUT_SHARES, PAIR_CUT_WHOLE, PAIR_CUT_SPLIT2, PAIR_CUT_SPLIT3, PAIR_CUT_SPLIT4 = 1, 2, 3, 4, 5
+
+
+def HINT_PAIR(columns: int, cut: int) -> int:
+    """WOQ_B200_HINT_PAIR of include/woq_b200.h."""
+    return columns << 16 | cut << 8
+
+
 def pair_plan(weight_dtype: int, columns: int, tiles: int, k: int, num_sms: int = 148) -> dict:
     """Pipeline shape of a launch of the CTA-pair kernel (woq_b200_pair_plan; no GPU needed)."""
     out = (ctypes.c_int32 * 6)()

@@ -190,3 +190,19 @@ def test_launches_back_to_back(capi, m):
         stream.synchronize()
     assert torch.equal(bufs[-1], want)
     ws.status()
+
+
+@pytest.mark.parametrize("m", [4, 16])
+def test_many_pipeline_stages_per_cta_up_to_16_tokens(capi, m):
+    """The same for the token counts at which this context's calls run on the one-CTA kernel (above 16 tokens they
+    run on CTA pairs: tests/test_gpu_pair_kernel.py)."""
+    layer = make_int4_layer(1152, 16384, 128, seed=4242)
+    ctx = make_ctx(capi, layer, flags=capi.LAYOUT_TC_ONLY)
+    x = make_acts(m, 16384, seed=m)
+    y0 = None
+    for _ in range(4):
+        y = ctx.linear(bf16_tensor(x, "cuda"))
+        y0 = y if y0 is None else y0
+        assert torch.equal(y, y0)
+    ctx.workspace(m).status()
+    check(bf16_numpy(y0), oracle_y(layer, x))

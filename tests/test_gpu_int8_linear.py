@@ -244,3 +244,57 @@ def test_rmsnorm_quant_rejects_what_it_cannot_do(capi):
     sa = torch.ones((2,), dtype=torch.float32, device="cuda")
     with pytest.raises(capi.WoqError, match="tcgen05 INT8 route"):
         blk.linear_prequant(qa, sa)
+
+
+# --------------------------------------------------------------------------------------------
+# The CTA-pair kernel and the quantiser at the edges of their tiles
+
+
+@pytest.mark.parametrize("act_mode", [6, 2])
+@pytest.mark.parametrize("n,k", [(129, 128), (331, 640), (1000, 1920), (331, 2048), (129, 16512)])
+@pytest.mark.parametrize("m", [31, 33, 63, 65, 127, 129, 257, 513])
+def test_tile_edges(capi, act_mode, n, k, m):
+    """Token counts around a 32-column step, the 64-token output pass, the 256-column tile and the quantiser's
+    128 tokens; rows that are not 16-byte aligned; one k-chunk; K on both sides of the quantiser's limits (2048 for
+    four CTAs a row, 16384 for a row in registers)."""
+    layer = make_layer(n, k, seed=n + k, bias=True)
+    ctx = make_ctx(capi, layer, act_mode=act_mode)
+    x = O.rne_bf16(make_acts(m, k, seed=m) + (0.3 if act_mode == 2 else 0.0))
+    x[m // 2] = 0.0
+    xb = bf16_tensor(x, "cuda")
+    qa, sa, acc = ctx.int8_internals(xb)
+    qa_ref, sa_ref, _ = O.dynamic_quant(x, act_mode)
+    np.testing.assert_array_equal(qa.cpu().numpy().view(qa_ref.dtype), qa_ref)
+    np.testing.assert_array_equal(sa.cpu().numpy(), sa_ref)
+    np.testing.assert_array_equal(acc.cpu().numpy(), O.int8_accumulators(qa_ref, layer["qw"]))
+    resid = make_acts(m, n, seed=m + 1)
+    y = bf16_numpy(ctx.linear(xb, capi.FUSE_ADD, [bf16_tensor(resid, "cuda")]))
+    ctx.workspace(m).status()
+    ref = O.woq_linear_int8(x, layer["qw"], layer["s"], layer["bias"], O.FUSE_ADD, [resid], act_mode=act_mode)
+    mx, mr = O.parity_metrics(y, ref)
+    # exact integer sums: the order of bias, scales and rounding is all that may differ
+    assert mx <= O.MAX_ABS_TOL and mr <= O.MEAN_REL_TOL, (mx, mr)
+    assert (y == ref).mean() > 0.99
+
+
+@pytest.mark.parametrize("act_mode", [6, 2])
+@pytest.mark.parametrize("n,k,m,columns", [(331, 1920, 290, 32), (331, 2048, 161, 160), (129, 640, 33, 64),
+                                           (2304, 2048, 513, 32), (2304, 2048, 513, 256)])
+def test_every_cut_gives_the_same_bits(capi, act_mode, n, k, m, columns):
+    """Integer sums: shared tiles, whole tiles and splits agree exactly, with the accumulators of the oracle."""
+    layer = make_layer(n, k, seed=n + m, bias=True)
+    x = O.rne_bf16(make_acts(m, k, seed=m) + (0.3 if act_mode == 2 else 0.0))
+    xb, resid = bf16_tensor(x, "cuda"), bf16_tensor(make_acts(m, n, seed=5), "cuda")
+    qa_ref, _, _ = O.dynamic_quant(x, act_mode)
+    acc_ref = O.int8_accumulators(qa_ref, layer["qw"])
+    want = make_ctx(capi, layer, act_mode=act_mode).linear(xb, capi.FUSE_ADD, [resid])
+    for cut in (capi.PAIR_CUT_SHARES, capi.PAIR_CUT_WHOLE, capi.PAIR_CUT_SPLIT2, capi.PAIR_CUT_SPLIT3, capi.PAIR_CUT_SPLIT4):
+        if cut > 2 and k // 128 < 4 * (cut - 1):
+            continue
+        ctx = capi.WoqContext(torch.from_numpy(layer["qw"]).cuda(), torch.from_numpy(layer["s"]).cuda(), None,
+                              torch.from_numpy(layer["bias"]).cuda(), n, k, capi.DTYPE_INT8, -1, capi.LOWP_INT8,
+                              act_quant_mode=act_mode, kernel_hint=capi.HINT_PAIR(columns, cut))
+        for _ in range(3):
+            assert torch.equal(ctx.linear(xb, capi.FUSE_ADD, [resid]), want), cut
+        np.testing.assert_array_equal(ctx.int8_internals(xb)[2].cpu().numpy(), acc_ref)
+        ctx.workspace(m).status()
