@@ -14,15 +14,16 @@
 #include <ATen/ATen.h>
 #include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/custom_class.h>
 #include <torch/library.h>
 
 #include <algorithm>
-#include <atomic>
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <utility>
 #include <vector>
 
@@ -55,107 +56,125 @@ int dtype_code(const at::Tensor& t) {
 //
 // Eager calls on one stream are ordered: one workspace per (device, stream), replaced by a larger one on demand.
 //
-// A captured call runs again with every replay: on any stream, beside eager calls and other graphs, and after
-// the eager workspace of the capturing stream has been replaced.  So each stream of a capture has a workspace of its
-// own.  It is zeroed outside the graph (no node of one graph that another would rely on) and owned by the graph:
-// CUDA calls release_graph_workspaces when the graph and all that was instantiated from it are gone.
-struct GraphWorkspaces {
-  unsigned long long capture;  // unique over the lifetime of the process
-  struct Buffers {
-    int dev;
-    std::vector<at::Tensor> all;  // the last one is in use; calls captured earlier hold the smaller ones before it
-  };
-  std::map<cudaStream_t, Buffers> of_stream;
+// A captured call runs again with every replay: on any stream, beside eager calls and other graphs, and after the
+// eager workspace of the capturing stream has been replaced.  So captures have workspaces of their own: one per
+// memory pool of the graph and capturing stream.  (PyTorch's graphs have a pool each, or share one when they are
+// never replayed at the same time.)  They are zeroed outside the graph, so that no graph relies on a node of another, lie
+// outside the pools, whose memory other graphs may write, and are given back when the pool has no user left.
+// Captures that PyTorch's allocator knows nothing of count as one pool that is never without a user.
+// (A user object of the graph would tell when the graph is gone, but made every replay 4.5 us longer.)
+struct Workspace {
+  void* ptr = nullptr;
+  size_t bytes = 0;
+  at::Tensor owner;  // eager ones: keeps the buffer for the call when another thread replaces it
 };
 
 struct WorkspacePool {
+  struct GraphKey {
+    int dev;
+    c10::MempoolId_t pool;
+    cudaStream_t stream;
+    bool operator<(const GraphKey& o) const {
+      return std::tie(dev, pool, stream) < std::tie(o.dev, o.pool, o.stream);
+    }
+  };
   std::mutex mu;
   std::map<std::pair<int, cudaStream_t>, at::Tensor> eager;
-  std::map<unsigned long long, GraphWorkspaces*> captured;  // by capture id
+  // the last one of a key is in use; calls captured earlier hold the smaller ones before it
+  std::map<GraphKey, std::vector<Workspace>> graphs;
+  std::map<cudaStream_t, std::pair<unsigned long long, c10::MempoolId_t>> capture;  // latest of a stream: id, pool
   std::map<int, cudaStream_t> side;  // per device: a stream that is never captured
-  // what release_graph_workspaces leaves for the next call.  A lock of its own, under which nothing calls CUDA.
-  std::mutex released_mu;
-  std::atomic<bool> any_released{false};
-  std::vector<GraphWorkspaces*> released;
+  std::vector<std::pair<int, Workspace>> dead;
 };
 WorkspacePool& workspace_pool() {
-  static auto* pool = new WorkspacePool;  // never destroyed: a graph may be released while the process exits
+  static auto* pool = new WorkspacePool;  // never destroyed: the process may exit in any order
   return *pool;
 }
 
-// Runs where CUDA may not be called, so the buffers go back to the allocator from the next call.
-void CUDART_CB release_graph_workspaces(void* graph_workspaces) {
-  WorkspacePool& pool = workspace_pool();
-  std::lock_guard<std::mutex> lock(pool.released_mu);
-  pool.released.push_back(static_cast<GraphWorkspaces*>(graph_workspaces));
-  pool.any_released = true;
+// The memory pool that `p`, allocated during a capture, belongs to; {0, 0}: none of a graph, or an allocator that
+// does not say.
+c10::MempoolId_t pool_of(int dev, const void* p) {
+  const auto at = reinterpret_cast<uintptr_t>(p);
+  try {
+    for (const auto& seg : c10::cuda::CUDACachingAllocator::snapshot({0, 0}, false).segments)
+      if (seg.device == dev && at >= seg.address && at < seg.address + seg.total_size) return seg.owner_private_pool_id;
+  } catch (const c10::Error&) {
+  }
+  return {0, 0};
 }
 
-// (with pool.mu held)
-void free_released(WorkspacePool& pool) {
-  if (!pool.any_released) return;
-  std::vector<GraphWorkspaces*> dead;
-  {
-    std::lock_guard<std::mutex> lock(pool.released_mu);
-    dead.swap(pool.released);
-    pool.any_released = false;
-  }
-  for (auto* g : dead) {
-    pool.captured.erase(g->capture);
-    delete g;
+// (an allocator that has told the pool's id above: it fails for an id that it has no pool of any more)
+bool pool_has_users(int dev, c10::MempoolId_t id) {
+  try {
+    return c10::cuda::CUDACachingAllocator::getPoolUseCount(static_cast<c10::DeviceIndex>(dev), id) > 0;
+  } catch (const c10::Error&) {
+    return false;
   }
 }
 
-// (with pool.mu held) A buffer with a zero header, made on a stream that takes no part in any capture.
-at::Tensor workspace_outside_captures(WorkspacePool& pool, c10::DeviceIndex dev, size_t bytes) {
+// (with pool.mu held) Finds the workspaces whose graphs are gone.
+void collect_dead(WorkspacePool& pool) {
+  for (auto it = pool.graphs.begin(); it != pool.graphs.end();) {
+    const auto& key = it->first;
+    if (key.pool == c10::MempoolId_t{0, 0} || pool_has_users(key.dev, key.pool)) {
+      ++it;
+      continue;
+    }
+    for (auto& w : it->second) pool.dead.emplace_back(key.dev, std::move(w));
+    it = pool.graphs.erase(it);
+  }
+}
+
+// (with pool.mu held, not under capture) cudaFree waits for a last replay that may still be running.
+void free_dead(WorkspacePool& pool) {
+  if (pool.dead.empty()) return;
+  c10::cuda::CUDAStreamCaptureModeGuard allow{cudaStreamCaptureModeRelaxed};  // (another thread may be capturing)
+  for (auto& d : pool.dead) {
+    c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(d.first));
+    C10_CUDA_CHECK(cudaFree(d.second.ptr));
+  }
+  pool.dead.clear();
+}
+
+// (with pool.mu held) A buffer with a zero header that belongs to no graph and no stream.
+Workspace graph_workspace(WorkspacePool& pool, c10::DeviceIndex dev, size_t bytes) {
   c10::cuda::CUDAStreamCaptureModeGuard allow{cudaStreamCaptureModeRelaxed};
   cudaStream_t& side = pool.side[dev];
   if (!side) C10_CUDA_CHECK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
-  c10::cuda::CUDAStreamGuard on_side(c10::cuda::getStreamFromExternal(side, dev));
-  at::Tensor t = at::empty({static_cast<int64_t>(bytes)},
-                           at::TensorOptions().dtype(at::kByte).device(at::Device(at::kCUDA, dev)));
-  C10_CUDA_CHECK(cudaMemsetAsync(t.data_ptr(), 0, woq_b200_workspace_header_bytes(), side));
+  Workspace w;
+  C10_CUDA_CHECK(cudaMalloc(&w.ptr, bytes));
+  w.bytes = bytes;
+  C10_CUDA_CHECK(cudaMemsetAsync(w.ptr, 0, woq_b200_workspace_header_bytes(), side));
   C10_CUDA_CHECK(cudaStreamSynchronize(side));
-  return t;
+  return w;
 }
 
-at::Tensor workspace_for(c10::DeviceIndex dev, cudaStream_t stream, size_t bytes) {
+// `out`: a tensor that this call has allocated.
+Workspace workspace_for(c10::DeviceIndex dev, cudaStream_t stream, size_t bytes, const at::Tensor& out) {
   WorkspacePool& pool = workspace_pool();
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   unsigned long long capture = 0;
-  cudaGraph_t graph = nullptr;
-  if (stream) C10_CUDA_CHECK(cudaStreamGetCaptureInfo(stream, &status, &capture, &graph));  // (the legacy stream is never captured)
+  if (stream) C10_CUDA_CHECK(cudaStreamGetCaptureInfo(stream, &status, &capture));  // (the legacy stream is never captured)
   std::lock_guard<std::mutex> lock(pool.mu);
-  free_released(pool);
   if (status != cudaStreamCaptureStatusActive) {
     at::Tensor& t = pool.eager[{dev, stream}];
-    if (!t.defined() || static_cast<size_t>(t.numel()) < bytes)
+    if (!t.defined() || static_cast<size_t>(t.numel()) < bytes) {
       t = at::zeros({static_cast<int64_t>(bytes)},
                     at::TensorOptions().dtype(at::kByte).device(at::Device(at::kCUDA, dev)));
-    return t;
-  }
-  GraphWorkspaces*& g = pool.captured[capture];
-  if (!g) {
-    g = new GraphWorkspaces{capture, {}};
-    cudaUserObject_t owner = nullptr;
-    cudaError_t e = cudaUserObjectCreate(&owner, g, release_graph_workspaces, 1, cudaUserObjectNoDestructorSync);
-    if (e != cudaSuccess) {
-      delete g;
-      pool.captured.erase(capture);
-      C10_CUDA_CHECK(e);
+      collect_dead(pool);
     }
-    e = cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove);
-    if (e != cudaSuccess) {
-      pool.captured.erase(capture);
-      cudaUserObjectRelease(owner, 1);  // hands the object to release_graph_workspaces
-      C10_CUDA_CHECK(e);
-    }
+    free_dead(pool);
+    return {t.data_ptr(), static_cast<size_t>(t.numel()), t};
   }
-  auto& bufs = g->of_stream[stream];
-  bufs.dev = dev;
-  const size_t last = bufs.all.empty() ? 0 : static_cast<size_t>(bufs.all.back().numel());
-  if (last < bytes) bufs.all.push_back(workspace_outside_captures(pool, dev, std::max(bytes, last + last / 2)));
-  return bufs.all.back();
+  auto& latest = pool.capture[stream];
+  if (latest.first != capture) {
+    collect_dead(pool);
+    latest = {capture, pool_of(dev, out.data_ptr())};
+  }
+  auto& bufs = pool.graphs[{dev, latest.second, stream}];
+  const size_t last = bufs.empty() ? 0 : bufs.back().bytes;
+  if (last < bytes) bufs.push_back(graph_workspace(pool, dev, std::max(bytes, last + last / 2)));
+  return bufs.back();
 }
 
 // Synchronises every stream that has run a WOQ op, and the devices of captured ones, and raises if a kernel gave
@@ -163,18 +182,18 @@ at::Tensor workspace_for(c10::DeviceIndex dev, cudaStream_t stream, size_t bytes
 void woq_check_status() {
   WorkspacePool& pool = workspace_pool();
   std::lock_guard<std::mutex> lock(pool.mu);
-  free_released(pool);
+  collect_dead(pool);
+  free_dead(pool);
   for (auto& kv : pool.eager) {
     if (!kv.second.defined()) continue;
     c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(kv.first.first));
     WOQ_CHECK(woq_b200_workspace_status(kv.second.data_ptr(), kv.first.second));
   }
-  for (auto& g : pool.captured)
-    for (auto& kv : g.second->of_stream) {
-      c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(kv.second.dev));
-      C10_CUDA_CHECK(cudaDeviceSynchronize());  // replays run on streams that are not known here
-      for (auto& t : kv.second.all) WOQ_CHECK(woq_b200_workspace_status(t.data_ptr(), pool.side[kv.second.dev]));
-    }
+  for (auto& g : pool.graphs) {
+    c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(g.first.dev));
+    C10_CUDA_CHECK(cudaDeviceSynchronize());  // replays run on streams that are not known here
+    for (auto& w : g.second) WOQ_CHECK(woq_b200_workspace_status(w.ptr, pool.side[g.first.dev]));
+  }
 }
 
 // plain INT4 weight [N, K/2] (k even in the low nibble) with its input channels re-ordered
@@ -449,18 +468,18 @@ at::Tensor run(WoqLinearOpContext* c, const at::Tensor& input, int32_t fusion,
   if (M > 0) {
     woq_b200_ctx* k = general ? c->ctx_general() : c->ctx_for(M);
     const size_t need = woq_b200_workspace_bytes(k, M);
-    at::Tensor ws = workspace_for(c->device, stream.stream(), need);
+    const Workspace ws = workspace_for(c->device, stream.stream(), need, y);
     if (general) {
       const int io = x.scalar_type() == at::kBFloat16 ? WOQ_B200_T_BF16
                      : x.scalar_type() == at::kHalf   ? WOQ_B200_T_F16
                                                       : WOQ_B200_T_F32;
       WOQ_CHECK(woq_b200_linear_any(k, x.data_ptr(), io, M, x.stride(0), fusion,
                                     optr.empty() ? nullptr : optr.data(), static_cast<int32_t>(optr.size()),
-                                    y.data_ptr(), y.stride(0), ws.data_ptr(), ws.numel(), stream.stream()));
+                                    y.data_ptr(), y.stride(0), ws.ptr, ws.bytes, stream.stream()));
     } else {
       WOQ_CHECK(woq_b200_linear(k, x.data_ptr(), M, x.stride(0), fusion,
                                 optr.empty() ? nullptr : optr.data(), static_cast<int32_t>(optr.size()),
-                                y.data_ptr(), y.stride(0), ws.data_ptr(), ws.numel(), stream.stream()));
+                                y.data_ptr(), y.stride(0), ws.ptr, ws.bytes, stream.stream()));
     }
   }
   auto sizes = input.sizes().vec();
@@ -543,11 +562,11 @@ at::Tensor woq_linear_prequant(const at::Tensor& qa, const at::Tensor& sa, const
   auto stream = at::cuda::getCurrentCUDAStream(c->device);
   if (M > 0) {
     woq_b200_ctx* k = c->ctx_for(M);
-    at::Tensor ws = workspace_for(c->device, stream.stream(), woq_b200_workspace_bytes(k, M));
+    const Workspace ws = workspace_for(c->device, stream.stream(), woq_b200_workspace_bytes(k, M), y);
     WOQ_CHECK(woq_b200_linear_prequant(k, q2.data_ptr(), sa.data_ptr(), zpa.numel() ? zpa.data_ptr() : nullptr, M,
                                        static_cast<int32_t>(fusion), optr.empty() ? nullptr : optr.data(),
-                                       static_cast<int32_t>(optr.size()), y.data_ptr(), y.stride(0), ws.data_ptr(),
-                                       ws.numel(), stream.stream()));
+                                       static_cast<int32_t>(optr.size()), y.data_ptr(), y.stride(0), ws.ptr,
+                                       ws.bytes, stream.stream()));
   }
   auto sizes = qa.sizes().vec();
   sizes.back() = n_out;
@@ -577,9 +596,9 @@ at::Tensor mixtral_moe_woq(const at::Tensor& hidden_states, const at::Tensor& to
   const int64_t M = a.size(0);
   auto stream = at::cuda::getCurrentCUDAStream(d->device);
   woq_b200_ctx* dk = d->ctx_for(M);
-  at::Tensor ws = workspace_for(d->device, stream.stream(), woq_b200_workspace_bytes(dk, M));
+  const Workspace ws = workspace_for(d->device, stream.stream(), woq_b200_workspace_bytes(dk, M), a);
   WOQ_CHECK(woq_b200_linear_scatter(dk, a.data_ptr(), M, a.stride(0), ti.data_ptr<int32_t>(), w.data_ptr(),
-                                    output.data_ptr(), output.stride(0), ws.data_ptr(), ws.numel(),
+                                    output.data_ptr(), output.stride(0), ws.ptr, ws.bytes,
                                     stream.stream()));
   return output;
 }
@@ -684,12 +703,12 @@ at::Tensor deepseek_moe_woq(const at::Tensor& hidden_states, const at::Tensor& t
         rowsd.push_back(cnt[e]);
         yd.push_back(row(x, off));
       }
-      at::Tensor ws;
+      Workspace ws;
       if (most > 0) {
-        ws = workspace_for(dev, stream, woq_b200_workspace_bytes(gu[0], most));
+        ws = workspace_for(dev, stream, woq_b200_workspace_bytes(gu[0], most), output);
         WOQ_CHECK(woq_b200_linear_grouped(gu.data(), row0.data(), rows.data(), y.data(),
                                           static_cast<int32_t>(gu.size()), x.data_ptr(), np, hidden, ffn,
-                                          ws.data_ptr(), ws.numel(), stream));
+                                          ws.ptr, ws.bytes, stream));
         // (all rows: those of the other experts hold nothing yet)
         WOQ_CHECK(woq_b200_silu_mul(gate.data_ptr(), act.data_ptr(), act.data_ptr(), np * ffn, stream));
       }
@@ -698,9 +717,9 @@ at::Tensor deepseek_moe_woq(const at::Tensor& hidden_states, const at::Tensor& t
         auto linear = [&](const c10::intrusive_ptr<WoqLinearOpContext>& c, const at::Tensor& in, int32_t fusion,
                           const void* other, const at::Tensor& out) {
           woq_b200_ctx* k = c->ctx_for(cnt[e]);
-          at::Tensor scratch = workspace_for(dev, stream, woq_b200_workspace_bytes(k, cnt[e]));
+          const Workspace scratch = workspace_for(dev, stream, woq_b200_workspace_bytes(k, cnt[e]), output);
           WOQ_CHECK(woq_b200_linear(k, row(in, off), cnt[e], in.size(1), fusion, other ? &other : nullptr,
-                                    other ? 1 : 0, row(out, off), out.size(1), scratch.data_ptr(), scratch.numel(),
+                                    other ? 1 : 0, row(out, off), out.size(1), scratch.ptr, scratch.bytes,
                                     stream));
         };
         linear(gate_ctx[e], x, WOQ_B200_FUSE_SILU, nullptr, gate);
@@ -710,7 +729,7 @@ at::Tensor deepseek_moe_woq(const at::Tensor& hidden_states, const at::Tensor& t
       if (most > 0)
         WOQ_CHECK(woq_b200_linear_grouped(d.data(), row0d.data(), rowsd.data(), yd.data(),
                                           static_cast<int32_t>(d.size()), act.data_ptr(), np, ffn, hidden,
-                                          ws.data_ptr(), ws.numel(), stream));
+                                          ws.ptr, ws.bytes, stream));
       WOQ_CHECK(woq_b200_moe_combine(x.data_ptr(), ids, pos_of.data_ptr<int32_t>(),
                                      row(w, t0), nt, static_cast<int32_t>(top_k), hidden, row(output, t0), stream));
     }
