@@ -45,14 +45,20 @@ def test_two_threads(capi, route, tokens):
     def work(i):
         try:
             torch.cuda.set_device(0)
-            ws = capi.Workspace(ctx.workspace_bytes(tokens[i]), "cuda")
+            x, m = xs[i], tokens[i]
+            ws = capi.Workspace(ctx.workspace_bytes(m), "cuda")
             out = [torch.empty_like(refs[i]) for _ in range(4)]
             torch.cuda.synchronize()
-            with torch.cuda.stream(torch.cuda.Stream()):
-                start.wait()
-                for j in range(1500):
-                    ctx.linear(xs[i], out=out[j % 4], workspace=ws)
-                torch.cuda.current_stream().synchronize()
+            stream = torch.cuda.Stream()
+            # bare calls of the C ABI, so that the threads spend their time in the library, beside each other
+            call = capi.lib().woq_b200_linear
+            args = [(ctx.handle, x.data_ptr(), m, x.stride(0), 0, None, 0, y.data_ptr(), y.stride(0), ws.buf.data_ptr(),
+                     ws.nbytes, stream.cuda_stream) for y in out]
+            start.wait()
+            codes = {call(*args[j % 4]) for j in range(20000)}
+            stream.synchronize()
+            assert codes == {0}, (codes, capi.lib().woq_b200_last_error())
+            with torch.cuda.stream(stream):
                 ws.status()
             outs[i] = out
         except Exception as e:  # noqa: BLE001
