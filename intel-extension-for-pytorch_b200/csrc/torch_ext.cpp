@@ -620,18 +620,25 @@ int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 // Scratch of a mixture-of-experts call: three tensors with a row for every (token, slot) pair.  Long batches go
 // through in slabs of tokens that stay below this (8192 pairs of Mixtral-8x7B's layer, 1024 for each expert).
 constexpr int64_t kMoeScratchBytes = 512ll << 20;
+// An expert with more tokens than this joins the grouped launches of a call that has them, and is packed a second time
+// for them (88 MB for one of Mixtral-8x7B's).  One that stays outside costs three launches of the streaming kernel,
+// about 20 us: tokens [40, 30, 20, 8, 6, 4, 2, 2] take 355 us, with all experts grouped 279.  With 9 and more tokens
+// beside others above 16 an expert is in the middle of the crowd and gets its own more than 16 soon enough, and
+// keeping such experts outside costs most: [18, 17, 21, 12, 13, 19, 11, 17] 260 us grouped, 379 with a limit of 16.
+constexpr int32_t kMoeJoinAbove = 8;
 
 // reference: csrc/cpu/aten/MoE.cpp:290-330.  topk_ids [tokens, top_k] names each token's experts; every
 // selected expert runs gate, up, silu * up and down on its tokens, and the results are added to the output
 // in expert order with their routing weights.
 //
 // The (token, slot) pairs are sorted by expert on the device; the per-expert counts come to the host, which
-// shapes the launches with them (and refuses ids that name no expert).  All gate and up projections of the
-// experts with more than 16 tokens are one launch and all their down projections another: an expert's linear
-// alone is too small to fill the GPU for long (Mixtral-8x7B's layer, 256 tokens: 996 us expert by expert, 350 in
-// two grouped launches).  The experts with up to 16 tokens run one after another on the streaming kernel: the
-// grouped launch needs the second tiling of a weight, which only an expert that has had more than 16 tokens gets.
-// Everything else (other weight types, act-order, ...) goes through the per-expert operator above.
+// shapes the launches with them (and refuses ids that name no expert).  Up to 16 tokens for every expert, the
+// streaming kernel runs expert by expert, so that a model that only decodes keeps one copy of its weights.
+// Otherwise all gate and up projections are one launch and all down projections another: an expert's linear alone
+// is too small to fill the GPU for long (Mixtral-8x7B's layer, 256 tokens: 996 us expert by expert, 350 in two
+// grouped launches).  They read a second tiling of the weights, which experts that see only a few tokens beside the
+// others do not get: kMoeJoinAbove.  Everything else (other weight types, act-order, ...) goes through the
+// per-expert operator above.
 at::Tensor deepseek_moe_woq(const at::Tensor& hidden_states, const at::Tensor& topk_ids,
                             const std::vector<c10::intrusive_ptr<WoqLinearOpContext>>& gate_ctx,
                             const std::vector<c10::intrusive_ptr<WoqLinearOpContext>>& up_ctx,
@@ -681,30 +688,29 @@ at::Tensor deepseek_moe_woq(const at::Tensor& hidden_states, const at::Tensor& t
       WOQ_CHECK(woq_b200_gather_rows(row(hidden_states, t0), hidden, token_of.data_ptr<int32_t>(), np, hidden,
                                      x.data_ptr(), stream));
       std::vector<const woq_b200_ctx*> gu, d;
-      std::vector<int64_t> row0, rows, row0d, rowsd, few, few_row;  // few: experts of at most 16 tokens
+      std::vector<int64_t> row0, rows, row0d, rowsd, few, few_row;  // few: experts outside the grouped launches
       std::vector<void*> y, yd;
-      int32_t most = 0;
+      const int32_t most = *std::max_element(cnt, cnt + experts);
       for (int64_t e = 0, off = 0; e < experts; off += cnt[e++]) {
         if (cnt[e] == 0) continue;
-        if (cnt[e] <= 16) {
+        if (most <= 16 || cnt[e] <= kMoeJoinAbove) {
           few.push_back(e);
           few_row.push_back(off);
           continue;
         }
-        most = std::max(most, cnt[e]);
         for (const auto* c : {&gate_ctx[e], &up_ctx[e]}) {
-          gu.push_back((*c)->ctx_for(cnt[e]));
+          gu.push_back((*c)->ctx_for(17));  // the tensor-core tiling
           row0.push_back(off);
           rows.push_back(cnt[e]);
           y.push_back(row(c == &gate_ctx[e] ? gate : act, off));
         }
-        d.push_back(down_ctx[e]->ctx_for(cnt[e]));
+        d.push_back(down_ctx[e]->ctx_for(17));
         row0d.push_back(off);
         rowsd.push_back(cnt[e]);
         yd.push_back(row(x, off));
       }
       Workspace ws;
-      if (most > 0) {
+      if (!gu.empty()) {
         ws = workspace_for(dev, stream, woq_b200_workspace_bytes(gu[0], most), output);
         WOQ_CHECK(woq_b200_linear_grouped(gu.data(), row0.data(), rows.data(), y.data(),
                                           static_cast<int32_t>(gu.size()), x.data_ptr(), np, hidden, ffn,
@@ -726,7 +732,7 @@ at::Tensor deepseek_moe_woq(const at::Tensor& hidden_states, const at::Tensor& t
         linear(up_ctx[e], x, WOQ_B200_FUSE_MUL, row(gate, off), act);
         linear(down_ctx[e], act, WOQ_B200_FUSE_NONE, nullptr, x);
       }
-      if (most > 0)
+      if (!d.empty())
         WOQ_CHECK(woq_b200_linear_grouped(d.data(), row0d.data(), rowsd.data(), yd.data(),
                                           static_cast<int32_t>(d.size()), act.data_ptr(), np, ffn, hidden,
                                           ws.ptr, ws.bytes, stream));
