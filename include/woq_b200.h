@@ -126,8 +126,8 @@ extern "C" {
  * epilogue, woq_linear_silu followed by woq_linear_mul) deviates by about 2.5e-3, over the
  * bar; so it is never chosen automatically.  It expects |x| < 2^40 (larger activations
  * overflow to infinity inside the kernel) and treats |x| < 2^-61 as zero. */
-#define WOQ_B200_HINT_AUTO 0        /* streaming kernel for M <= 16, tcgen05 kernel above      */
-#define WOQ_B200_HINT_TENSOR_CORE 1 /* tcgen05 kernel for every M                              */
+#define WOQ_B200_HINT_AUTO 0        /* streaming kernel for M <= 16, CTA-pair kernel above     */
+#define WOQ_B200_HINT_TENSOR_CORE 1 /* tcgen05 kernels for every M                             */
 #define WOQ_B200_HINT_STREAM 2      /* register-dequant streaming kernel, 16 tokens a pass     */
 #define WOQ_B200_HINT_STREAM_FAST 3 /* streaming kernel, scale applied after the k-block sum   */
 
@@ -444,9 +444,9 @@ int woq_b200_int8_zero_points(const woq_b200_ctx* ctx, int64_t m, int32_t* zp, c
  * shared-memory budget per thread block in bytes. */
 int woq_b200_decode_plan(const woq_b200_ctx* ctx, int64_t m, int32_t* out);
 
-/* The pipeline shape of one launch of the tcgen05 INT4 kernel with n_tok token columns (16..256,
- * a multiple of 16; woq_b200_linear rounds the tokens of a launch up to that).  No reference
- * counterpart; a diagnostic that needs no GPU: out[0] k-blocks per stage, out[1] slots of the
+/* The pipeline shape of one launch of the one-CTA tcgen05 INT4 kernel with n_tok token columns (16..256,
+ * a multiple of 16; woq_b200_linear runs it with 16, for up to 16 tokens of a context that asks for the tensor
+ * cores or holds their tiling only).  No reference counterpart; a diagnostic that needs no GPU: out[0] k-blocks per stage, out[1] slots of the
  * A-group / activation ring (at least 4), out[2] slots of the packed-weight ring (a multiple of 4),
  * out[3] first TMEM column of the A groups (out[3] + 32 * out[0] * out[1] <= 512), out[4] dynamic
  * shared memory in bytes. */

@@ -1300,43 +1300,36 @@ static int run_tc(const woq_b200_ctx* c, const void* x, int64_t m, int64_t ldx, 
   if (int rc = settle_prepack_flag(c)) return rc;
   if (m > 16)
     return run_pair(c, x, m, ldx, fusion, o0, o1, row_idx, row_w, y, ldy, static_cast<uint8_t*>(ws), stream);
+  woq::TcParams p{};
+  p.n_tok = 16;
   CUtensorMap xmap;
-  const int64_t mt = m < 256 ? m : 256;
-  int n_tok = static_cast<int>((mt + 15) / 16 * 16);
-  if (int rc = make_kmajor_map(&xmap, x, m, c->desc.k, ldx, 2, n_tok)) return rc;
+  if (int rc = make_kmajor_map(&xmap, x, m, c->desc.k, ldx, 2, p.n_tok)) return rc;
   uint8_t* w8 = static_cast<uint8_t*>(ws);
-  const bool scatter = fusion == WOQ_B200_FUSE_SCALED_SCATTER_ADD;
-  for (int64_t m0 = 0; m0 < m; m0 += 256) {
-    const int64_t mm = m - m0 < 256 ? m - m0 : 256;
-    woq::TcParams p{};
-    p.wq = c->wq_tc;
-    p.sz = c->sz_tc;
-    p.bias = c->bias;
-    p.y = scatter ? static_cast<__nv_bfloat16*>(y) : static_cast<__nv_bfloat16*>(y) + m0 * ldy;
-    p.other0 = o0 ? static_cast<const __nv_bfloat16*>(o0) + m0 * ldy : nullptr;
-    p.other1 = o1 ? static_cast<const __nv_bfloat16*>(o1) + m0 * ldy : nullptr;
-    p.row_idx = row_idx ? row_idx + m0 : nullptr;
-    p.row_w = row_w ? static_cast<const __nv_bfloat16*>(row_w) + m0 : nullptr;
-    p.status = reinterpret_cast<int*>(w8);
-    p.counters = reinterpret_cast<uint32_t*>(w8 + 256);
-    p.partials = reinterpret_cast<float*>(w8 + kWsHeaderBytes);
-    p.ldy = ldy;
-    p.m = (int)mm;
-    p.n = (int)c->desc.n;
-    p.n_out = fusion == WOQ_B200_FUSE_SILU_MUL ? (int)(c->desc.n / 2) : (int)c->desc.n;
-    p.k = (int)c->desc.k;
-    p.m0 = (int)m0;
-    p.n_tok = n_tok;
-    p.tiles = c->tiles_tc;
-    p.kb_per_tile = c->kb_per_tile;
-    p.kbpg_shift = c->kbpg_shift;
-    p.groups = c->groups;
-    p.fusion = fusion;
-    p.gate_up = c->gate_up;
-    const int grid = woq::tc_pick_grid(c->tiles_tc, c->kb_per_tile, c->num_sms);
-    CUDA_TRY(woq::launch_int4_tc(p, xmap, grid, stream));
-    woq::count_launch();
-  }
+  p.wq = c->wq_tc;
+  p.sz = c->sz_tc;
+  p.bias = c->bias;
+  p.y = static_cast<__nv_bfloat16*>(y);
+  p.other0 = static_cast<const __nv_bfloat16*>(o0);
+  p.other1 = static_cast<const __nv_bfloat16*>(o1);
+  p.row_idx = row_idx;
+  p.row_w = static_cast<const __nv_bfloat16*>(row_w);
+  p.status = reinterpret_cast<int*>(w8);
+  p.counters = reinterpret_cast<uint32_t*>(w8 + 256);
+  p.partials = reinterpret_cast<float*>(w8 + kWsHeaderBytes);
+  p.ldy = ldy;
+  p.m = (int)m;
+  p.n = (int)c->desc.n;
+  p.n_out = fusion == WOQ_B200_FUSE_SILU_MUL ? (int)(c->desc.n / 2) : (int)c->desc.n;
+  p.k = (int)c->desc.k;
+  p.tiles = c->tiles_tc;
+  p.kb_per_tile = c->kb_per_tile;
+  p.kbpg_shift = c->kbpg_shift;
+  p.groups = c->groups;
+  p.fusion = fusion;
+  p.gate_up = c->gate_up;
+  const int grid = woq::tc_pick_grid(c->tiles_tc, c->kb_per_tile, c->num_sms);
+  CUDA_TRY(woq::launch_int4_tc(p, xmap, grid, stream));
+  woq::count_launch();
   return WOQ_B200_OK;
 }
 

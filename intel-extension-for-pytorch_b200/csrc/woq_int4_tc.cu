@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         mbar_wait(&hdr->free_[slot], phase ^ 1, abort_flag, p.status, 12);
         mbar_arrive_expect_tx(&hdr->full[slot], nkb * p.n_tok * 128);
         for (int j = 0; j < nkb; ++j)
-          tma_load_2d(xs + j * p.n_tok * 128, &xmap, (kb0 + j) * kBlockK, p.m0, &hdr->full[slot]);
+          tma_load_2d(xs + j * p.n_tok * 128, &xmap, (kb0 + j) * kBlockK, 0, &hdr->full[slot]);
         kb0 += nkb;
         rem -= nkb;
         if (kb0 == kbpt) kb0 = 0;

@@ -94,7 +94,7 @@ cudaError_t launch_decode_int4(DecodeParams p, const DecodePlan& plan, cudaStrea
 // Receives a pending all-gather without running a linear (status: the workspace-style status word).
 cudaError_t launch_comm_fence(const CommParams& c, int* status, int num_sms, cudaStream_t stream);
 
-// ---- INT4 tensor-core path (any M up to 256 per launch) --------------------------------
+// ---- INT4 tensor-core path, one CTA per tile (M <= 16; above: the CTA-pair path below) -----
 // Row layout: tiles of 128 output rows x 64 k, 4096 bytes each, [tile][k-block][half][row][16 B].
 // Word j' = 4 * half + j of a row holds k = 8 j' + 2 s in nibble s (bits 4s..4s+3) and
 // k = 8 j' + 2 s + 1 in nibble s + 4, so (w >> 4s) & 0x000f000f is the bf16x2 pair (k, k+1).
@@ -116,16 +116,15 @@ struct TcParams {
   int* status;
   int64_t ldy;
   int m, n, n_out, k;
-  int m0;              // first token row of this launch inside the x tensor map
-  int n_tok;           // token columns of the MMA (multiple of 16, <= 256)
+  int n_tok;           // token columns of the MMA: 16 (the pipeline shapes go up to 256)
   int tiles, kb_per_tile, kbpg_shift, groups;
   int kbs, stages;     // k-blocks per stage; slots of the A-group / activation ring
   int w_ring, a_col0;  // slots of the packed-weight ring (a multiple of four); first TMEM column of the A groups
   int fusion, gate_up;
 };
 
-// the M <= 16 kernel's launches opt into programmatic dependent launch unless WOQ_B200_PDL=0 was
-// set before first use (the tcgen05 kernels launch plainly)
+// The decode kernel, the CTA-pair kernels, the K-block tcgen05 kernel and the per-token quantiser opt into
+// programmatic dependent launch unless WOQ_B200_PDL=0 was set before first use (all other kernels launch plainly).
 bool dependent_launch_enabled();
 // Lets `kern` (no static shared memory) be launched with all the shared memory a block can have.  Always the same
 // limit, set before each launch: with the launch's own size, two host threads with different token counts could

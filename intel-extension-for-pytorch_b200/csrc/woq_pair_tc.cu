@@ -29,12 +29,12 @@
 // the same tiles pay three trips through L2 and one CTA per tile reads all the parts: 4096 x 4096, 128 tokens
 // took 26 us for 4 us of MMAs.
 //
-// What bounds it: at 256 token columns the tensor cores under the power limit (57344 x 8192, 512
-// tokens: 339 us, 1420 TFLOP/s, against 501 us for one CTA per tile and 256 tokens per launch); at 32
-// columns the dequantiser's issue slots and the hand-overs between roles (91 us, 2.7 TB/s of weights,
-// was 125 us; 72 us with two k-blocks per visit and idle warps suspended).  A lone thread beside sixteen dequantising warps gets an instruction issued every ten
-// cycles or so, so the roles' work per stage is what has to be small: one activation copy per stage,
-// several k-blocks per stage, no wait or fence that is not needed.
+// What bounds it.  At 256 token columns: the tensor cores under the power limit (57344 x 8192, 512 tokens: 333 us,
+// 1440 TFLOP/s; one CTA per tile and 256 tokens per launch took 501).  At 32 columns: the dequantiser's issue
+// slots and the hand-overs between roles (57344 x 8192, 32 tokens: 72 us, 3.4 TB/s of weights; 91 us with one
+// k-block per visit and polling idle warps, 125 us with one CTA per tile).  A lone thread beside sixteen
+// dequantising warps gets an instruction issued every ten cycles or so, so the roles' work per stage is what has
+// to be small: one activation copy per stage, several k-blocks per stage, no wait or fence that is not needed.
 //
 // Weights: INT4, INT8 and NF4 in the row layout of their kind (WeightKind); only the dequantiser and
 // the bytes of a k-block differ.
@@ -672,11 +672,10 @@ int pair_group_columns(const int64_t* rows, int groups, int kind) {
 //   k-blocks per stage: four up to 128 columns, two above.  Every stage costs each single-thread role
 //     300-400 cycles of waiting, issuing and bookkeeping beside the busy dequantising warps, whatever
 //     the stage holds; a k-block's MMAs take at least 64 cycles, 4 x n_tok / 2 when that is more.
-//   k-blocks per warpgroup and visit: two up to 128 columns, so that the two waits, the store's completion
-//     and the arrival (600 of 1490 cycles, most of it latency) come once per two k-blocks.  57344 x 8192 INT4,
-//     32 / 64 / 128 tokens: 80 / 83 / 105 us with one, 72 / 77 / 101 with two; 57344 x 4096 INT8, 8 tokens:
-//     46 and 44 us.  (Stages of two with one warpgroup each: 89 / 92 / 110 us.)  At 128 columns of 8-bit
-//     weights only three weight slots fit, too few for that: 68 us with one, 73 with two.
+//   k-blocks per warpgroup and visit: two up to 128 columns, because the two waits, the store's completion and
+//     the arrival (600 of 1490 cycles, most of it latency) then come once per two k-blocks (57344 x 8192 INT4, 32 /
+//     64 / 128 tokens: 72 / 77 / 101 us, with one 80 / 83 / 105).  One at 128 columns of 8-bit weights: only three
+//     weight slots fit, too few for two warpgroups to hold one each and a third to land (73 us with two, 68 with one).
 //   Rings: a parity wait cannot tell a barrier that is one completion short from one that is three
 //     short, so whoever waits for use u of a slot must know that use u - 1 has completed.  A warpgroup sees
 //     every step-th stage (step = 4 kpw / kbs: 1 or 2).  A weight ring that is a multiple of step gives each

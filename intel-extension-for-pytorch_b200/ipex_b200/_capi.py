@@ -196,7 +196,7 @@ def _others(others, m: int, n_out: int, out: torch.Tensor):
 
 
 def tc_plan(n_tok: int) -> dict:
-    """Pipeline shape of a tcgen05 INT4 launch with n_tok token columns (woq_b200_tc_plan; no GPU needed)."""
+    """Pipeline shape of a one-CTA tcgen05 INT4 launch with n_tok columns (woq_b200_tc_plan; no GPU needed)."""
     out = (ctypes.c_int32 * 5)()
     _check(lib().woq_b200_tc_plan(n_tok, out))
     return {"kbs": out[0], "stages": out[1], "w_ring": out[2], "a_col0": out[3], "smem_bytes": out[4]}
