@@ -624,7 +624,7 @@ def run_ours(args):
         tf = flops / n_launch / (kernel_ms * 1e-3) / 1e12
         roofline = {"bound": "tensor", "achieved": tf, "peak": tf_peak_r, "unit": "TFLOP/s",
                     "frac": tf / tf_peak_r if tf_peak_r else None, "traffic": None,
-                    "kernel": "woq_int4_tc_kernel", "peak_source": peak_src, "avg_launch_us": kernel_ms * 1e3,
+                    "kernel": "woq_pair_kernel", "peak_source": peak_src, "avg_launch_us": kernel_ms * 1e3,
                     "algorithmic_flops_per_launch": flops / n_launch}
     else:
         roofline = {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
@@ -664,7 +664,7 @@ def run_ours(args):
         e2e_ops = e2e_through_ops(torch, quant, m, device)
         log(f"e2e through the ops: {e2e_ops}")
 
-    # ---- prefill side of the metric: the tcgen05 kernel on one gate_up-sized layer ----------
+    # ---- prefill side of the metric: the CTA-pair kernel on one gate_up-sized layer ---------
     prefill = None
     if p == 1 and not args.no_prefill:
         pm = 512
@@ -693,7 +693,7 @@ def run_ours(args):
         _, tf_peak, _ = peaks()
         tflops = 2.0 * pm * 2 * FFN * HIDDEN / pt / 1e12
         prefill = {"tflops": tflops, "m": pm, "shape": f"{2 * FFN}x{HIDDEN} INT4 g128", "us_per_linear": pt * 1e6,
-                   "kernel": "woq_int4_tc_kernel", "bound": "tensor", "peak": tf_peak, "unit": "TFLOP/s",
+                   "kernel": "woq_pair_kernel", "bound": "tensor", "peak": tf_peak, "unit": "TFLOP/s",
                    "frac": tflops / tf_peak if tf_peak else None}
         del pctx, px, py, pws
 
