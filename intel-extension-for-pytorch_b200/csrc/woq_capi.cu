@@ -991,16 +991,14 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 static EncodeTiledFn encode_tiled_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
+  // (looked up by the first caller; others wait for it)
+  static const EncodeTiledFn fn = [] {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  }
+    const bool ok = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+                    q == cudaDriverEntryPointSuccess;
+    return ok ? reinterpret_cast<EncodeTiledFn>(p) : nullptr;
+  }();
   return fn;
 }
 
@@ -1402,11 +1400,10 @@ static int run_int8(const woq_b200_ctx* c, const void* x, int64_t m, int64_t ldx
 }
 
 static bool use_tc_path(const woq_b200_ctx* c, int64_t m) {
-  static int env = -1;
-  if (env < 0) {
+  static const int env = [] {
     const char* e = getenv("WOQ_B200_KERNEL_HINT");
-    env = e ? atoi(e) : 0;
-  }
+    return e ? atoi(e) : 0;
+  }();
   if (!c->wq_tc) return false;  // context packed for the streaming kernel only
   if (!c->wq) return true;      // context packed for the tensor-core kernel only
   const int own = c->desc.kernel_hint & 0xff, hint = own ? own : env;

@@ -1,5 +1,8 @@
 """Host threads that run linears of different token counts at the same time, each on its own stream and workspace:
 every launch succeeds and gives what it gives alone."""
+import os
+import subprocess
+import sys
 import threading
 
 import pytest
@@ -72,3 +75,36 @@ def test_two_threads(capi, route, tokens):
     assert not errors, errors
     for out, ref in zip(outs, refs):
         assert len(out) == 4 and all(torch.equal(y, ref) for y in out)
+
+
+FIRST_CALLS = """
+import threading, torch
+from ipex_b200 import _capi as C
+n, k, m = 256, 512, 32
+ctxs = [C.WoqContext(torch.zeros((n, k // 2), dtype=torch.uint8, device="cuda"), torch.ones((n, 4), device="cuda"), None,
+                     None, n, k, C.DTYPE_INT4, 128, C.LOWP_BF16) for _ in range(16)]
+x, outs = torch.ones((m, k), device="cuda").bfloat16(), [torch.empty((m, n), device="cuda").bfloat16() for _ in ctxs]
+ws = [C.Workspace(c.workspace_bytes(m), "cuda") for c in ctxs]
+torch.cuda.synchronize()
+start, codes, call = threading.Barrier(16), [], C.lib().woq_b200_linear
+def work(i):
+    args = (ctxs[i].handle, x.data_ptr(), m, k, 0, None, 0, outs[i].data_ptr(), n, ws[i].buf.data_ptr(), ws[i].nbytes,
+            torch.cuda.Stream().cuda_stream)
+    start.wait()
+    codes.append(call(*args))
+threads = [threading.Thread(target=work, args=(i,)) for i in range(16)]
+[t.start() for t in threads]
+[t.join() for t in threads]
+torch.cuda.synchronize()
+assert codes == [0] * 16, codes
+assert all(bool((o == -8 * k).all()) for o in outs)
+"""
+
+
+def test_first_calls_of_a_process_from_many_threads():
+    """What the library looks up once (driver entry points, capacities of the device) is there for every caller."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([root, os.path.join(root, "intel-extension-for-pytorch_b200")]))
+    for _ in range(3):
+        out = subprocess.run([sys.executable, "-c", FIRST_CALLS], env=env, capture_output=True, text=True, timeout=300)
+        assert out.returncode == 0, out.stderr[-2000:]
