@@ -1062,7 +1062,8 @@ int run_i8block_tc(const woq_b200_ctx* c, const I8BlockWs& L, const __nv_bfloat1
   int32_t* zpa = reinterpret_cast<int32_t*>(w8 + L.zpa);
   float* sat = reinterpret_cast<float*>(w8 + L.sat);
   if (mode == WOQ_B200_ACT_PER_M_K_BLOCK_SYM) {
-    CUDA_TRY(woq::launch_act_block128_quant(x, ldx, (int)m, c->kc, w8 + L.qa, sa, zpa, sat, L.n_tok, stream));
+    CUDA_TRY(woq::launch_act_block128_quant(x, ldx, (int)m, c->kc, w8 + L.qa, sa, zpa,
+                                             reinterpret_cast<int32_t*>(w8 + L.sumqa), sat, L.n_tok, stream));
   } else {
     CUDA_TRY(woq::launch_act_block_quant(x, ldx, (int)m, (int)c->desc.k, 128, mode, 0, w8 + L.qa, sa, zpa,
                                          reinterpret_cast<int32_t*>(w8 + L.sumqa), reinterpret_cast<float*>(w8 + L.range),
@@ -1075,6 +1076,34 @@ int run_i8block_tc(const woq_b200_ctx* c, const I8BlockWs& L, const __nv_bfloat1
   if (sa_out) CUDA_TRY(cudaMemcpyAsync(sa_out, sa, mk * 4, cudaMemcpyDeviceToDevice, stream));
   if (zpa_out) CUDA_TRY(cudaMemcpyAsync(zpa_out, zpa, mk * 4, cudaMemcpyDeviceToDevice, stream));
   if (!y && !acc_out) return WOQ_B200_OK;
+  if (woq::i8_block_tc_few_tokens(m, c->desc.n, c->kc)) {
+    woq::I8BlockParams q{};
+    q.w = c->wq_tc;
+    q.sw = c->btc_sw;
+    q.zw = c->btc_zw;
+    q.qa = w8 + L.qa;
+    q.sa = sa;
+    q.zpa = zpa;
+    q.sumqa = reinterpret_cast<int32_t*>(w8 + L.sumqa);
+    q.bias = c->bias;
+    q.y = static_cast<__nv_bfloat16*>(y);
+    q.other0 = static_cast<const __nv_bfloat16*>(o0);
+    q.other1 = static_cast<const __nv_bfloat16*>(o1);
+    q.acc_out = acc_out;
+    q.ldy = ldy;
+    q.m = (int)m;
+    q.n = (int)c->desc.n;
+    q.k = (int)c->desc.k;
+    q.kb = 128;
+    q.kc = c->kc;
+    q.group = c->g_group;
+    q.groups = c->groups;
+    q.fusion = fusion;
+    q.w4 = 1;
+    CUDA_TRY(woq::launch_i8_block(q, stream));
+    woq::count_launch();
+    return WOQ_B200_OK;
+  }
   woq::I8BlockTcParams p{};
   p.w = c->wq_tc;
   p.zw = c->btc_zw;

@@ -440,8 +440,8 @@ __global__ void __launch_bounds__(kBtcThreads, 1)
 // Per-token, per-block symmetric codes (the qconfig factory's default mode): one warp per (token, 128-wide
 // block) holds its 128 elements in registers, so range and codes are one pass and one launch instead of two.
 __global__ void __launch_bounds__(256) act_block128_quant_kernel(const __nv_bfloat16* x, int64_t ldx, int m, int kc,
-                                                                 uint8_t* qa, float* sa, int32_t* zpa, float* sat,
-                                                                 int n_tok) {
+                                                                 uint8_t* qa, float* sa, int32_t* zpa, int32_t* sumqa,
+                                                                 float* sat, int n_tok) {
   grid_launch_dependents();  // the GEMM's weight loads need nothing from here
   const int item = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (item >= m * kc) return;
@@ -457,16 +457,20 @@ __global__ void __launch_bounds__(256) act_block128_quant_kernel(const __nv_bflo
   }
   const float scale = __fdiv_rn(fmaxf(fabsf(hi), fabsf(lo)), 127.0f);
   uint32_t word = 0;
+  int sum = 0;
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
     float q = 0.f;
     if (scale > 0.f) q = fminf(fmaxf(rintf(__fdiv_rn(f[e], scale)), -128.f), 127.f);
+    sum += static_cast<int>(q);
     word |= (static_cast<uint32_t>(static_cast<int>(q)) & 0xffu) << (8 * e);
   }
   reinterpret_cast<uint32_t*>(qa + static_cast<size_t>(tok) * kc * 128 + c * 128)[lane] = word;
+  sum = __reduce_add_sync(0xffffffffu, sum);
   if (lane == 0) {
     sa[item] = scale;
     zpa[item] = 0;
+    sumqa[item] = sum;
     sat[(static_cast<size_t>(tok / n_tok) * kc + c) * n_tok + tok % n_tok] = scale;
   }
 }
@@ -545,6 +549,16 @@ int i8_block_tc_columns(int64_t m) {
   return best;
 }
 
+// Up to 8 tokens the kernel of 16 rows x 8 tokens per CTA (mma.sync, woq_int8_block.cu) is quicker: nothing waits for a
+// tile's other parts and nothing is drained through tensor memory.  9 to 16 tokens are two CTAs that read the weights
+// twice: quicker where the second time comes from L2, so up to half of its 126 MB.  That kernel / this one, us: one
+// token, 1024 x 2048 5.1 / 12.7, 4096 x 4096 7.4 / 16.1, 4096 x 14336 17.2 / 27.2, 28672 x 4096 16.7 / 41.3, 57344 x 8192
+// 71.5 / 131, 512 x 16384 18.8 / 21.4; 16 tokens, 4096 x 4096 9.5 / 18.2, 28672 x 4096 (59 MB) 34.9 / 44.8, but
+// 8192 x 28672 (117 MB) 92.4 / 74.8, 57344 x 8192 (235 MB) 141 / 137.
+bool i8_block_tc_few_tokens(int64_t m, int64_t n, int kc) {
+  return m <= 8 || (m <= 16 && n * kc * 64 <= (64ll << 20));
+}
+
 size_t i8_block_tc_partial_bytes(int num_sms, int part_tok) {
   return static_cast<size_t>(num_sms) * 2 * part_tok * kTcTileN * sizeof(float);
 }
@@ -583,9 +597,9 @@ cudaError_t launch_i8_block_tc(I8BlockTcParams p, const CUtensorMap& qamap, int 
 }
 
 cudaError_t launch_act_block128_quant(const __nv_bfloat16* x, int64_t ldx, int m, int kc, uint8_t* qa, float* sa,
-                                      int32_t* zpa, float* sat, int n_tok, cudaStream_t stream) {
+                                      int32_t* zpa, int32_t* sumqa, float* sat, int n_tok, cudaStream_t stream) {
   const unsigned blocks = static_cast<unsigned>(ceil_div(static_cast<int64_t>(m) * kc, 8));
-  act_block128_quant_kernel<<<blocks, 256, 0, stream>>>(x, ldx, m, kc, qa, sa, zpa, sat, n_tok);
+  act_block128_quant_kernel<<<blocks, 256, 0, stream>>>(x, ldx, m, kc, qa, sa, zpa, sumqa, sat, n_tok);
   return cudaGetLastError();
 }
 

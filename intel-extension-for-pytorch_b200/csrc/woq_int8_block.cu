@@ -20,7 +20,8 @@
 // A CTA owns 16 output rows and 8 tokens; its four warps take every fourth K block and their
 // fp32 sums are added in warp order at the end (nothing depends on timing).  Larger token counts
 // are further CTAs that read the weights again (from L2): this route is built for decode-sized
-// batches; the tcgen05 kernel of woq_int8.cu keeps INT8 weights with whole-K activation ranges.
+// batches.  INT8 weights with whole-K activation ranges have their own kernel (woq_i8_pair.cu); INT4 weights with
+// symmetric codes and K blocks of 128 come here for a few tokens only, in the layout of woq_i8_block_tc.cu.
 #include "woq_kernels.h"
 
 namespace woq {
@@ -179,7 +180,9 @@ __device__ __forceinline__ void mma_i8(int (&d)[4], uint32_t a0, uint32_t a1, ui
 
 constexpr int kI8Warps = 4;
 
-template <bool W4, bool ASYM>
+// TILED: 4-bit weights, scales and zero points in the layout of the tcgen05 kernel (K blocks of 128): a word's low
+// nibbles are four neighbouring k and its high nibbles the next four, so the codes come in natural order.
+template <bool W4, bool ASYM, bool TILED = false>
 __global__ void __launch_bounds__(kI8Warps * 32) woq_i8_block_kernel(const I8BlockParams p) {
   __shared__ float red[kI8Warps][16][9];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -194,34 +197,17 @@ __global__ void __launch_bounds__(kI8Warps * 32) woq_i8_block_kernel(const I8Blo
   const size_t row_bytes = W4 ? p.k / 2 : p.k;
   const uint8_t* w0 = p.w + r0 * row_bytes;
   const uint8_t* w1 = p.w + r1 * row_bytes;
+  const size_t tile = r0 / kTcTileN;  // (row 0, in place of a row outside the problem, is never used for a result)
+  const int in0 = r0 % kTcTileN, in1 = row_hi < p.n ? in0 + 8 : in0;
+  if (TILED) {
+    w0 = p.w + tile * p.kc * (kTcTileN * 64) + in0 * 16;
+    w1 = w0 + (in1 - in0) * 16;
+  }
   const uint8_t* qb = p.qa + static_cast<size_t>(tok_b) * p.k;
   float c[4] = {0.f, 0.f, 0.f, 0.f};  // (row_lo, tc0) (row_lo, tc1) (row_hi, tc0) (row_hi, tc1)
 
-  for (int blk = warp; blk < p.kc; blk += kI8Warps) {
-    int acc[4] = {0, 0, 0, 0};
-    const int k0 = blk * p.kb;
-    for (int kk = 0; kk < p.kb; kk += 64) {
-      const int kq = k0 + kk + 16 * t;  // this lane's 16 k of the 64
-      const uint4 bv = *reinterpret_cast<const uint4*>(qb + kq);
-      if (W4) {
-        const uint2 a = *reinterpret_cast<const uint2*>(w0 + (kq >> 1));
-        const uint2 b = *reinterpret_cast<const uint2*>(w1 + (kq >> 1));
-        mma_i8<true, ASYM>(acc, a.x & 0x0f0f0f0fu, b.x & 0x0f0f0f0fu, (a.x >> 4) & 0x0f0f0f0fu,
-                           (b.x >> 4) & 0x0f0f0f0fu, bv.x, bv.y);
-        mma_i8<true, ASYM>(acc, a.y & 0x0f0f0f0fu, b.y & 0x0f0f0f0fu, (a.y >> 4) & 0x0f0f0f0fu,
-                           (b.y >> 4) & 0x0f0f0f0fu, bv.z, bv.w);
-      } else {
-        const uint4 a = *reinterpret_cast<const uint4*>(w0 + kq);
-        const uint4 b = *reinterpret_cast<const uint4*>(w1 + kq);
-        mma_i8<false, ASYM>(acc, a.x, b.x, a.y, b.y, bv.x, bv.y);
-        mma_i8<false, ASYM>(acc, a.z, b.z, a.w, b.w, bv.z, bv.w);
-      }
-    }
-    // the block's part of C
-    const int grp = p.group >= p.k ? 0 : k0 / p.group;
-    const float s0 = p.sw[static_cast<size_t>(r0) * p.groups + grp], s1 = p.sw[static_cast<size_t>(r1) * p.groups + grp];
-    const int z0 = static_cast<int>(p.zpw ? p.zpw[static_cast<size_t>(r0) * p.groups + grp] : p.default_zp);
-    const int z1 = static_cast<int>(p.zpw ? p.zpw[static_cast<size_t>(r1) * p.groups + grp] : p.default_zp);
+  // a block's part of C
+  auto drain = [&](int blk, const int (&acc)[4], float s0, float s1, int z0, int z1) {
     const int ia = ta * p.kc + blk, ib = tb * p.kc + blk;
     const int sqa = p.sumqa[ia], sqb = p.sumqa[ib];
     int v[4] = {acc[0] - z0 * sqa, acc[1] - z0 * sqb, acc[2] - z1 * sqa, acc[3] - z1 * sqb};
@@ -245,6 +231,72 @@ __global__ void __launch_bounds__(kI8Warps * 32) woq_i8_block_kernel(const I8Blo
     c[1] += (static_cast<float>(v[1]) * sa_b) * s0;
     c[2] += (static_cast<float>(v[2]) * sa_a) * s1;
     c[3] += (static_cast<float>(v[3]) * sa_b) * s1;
+  };
+  auto mma_w4 = [&](int (&acc)[4], const uint2& a, const uint2& b, const uint4& bv) {
+    mma_i8<true, ASYM>(acc, a.x & 0x0f0f0f0fu, b.x & 0x0f0f0f0fu, (a.x >> 4) & 0x0f0f0f0fu, (b.x >> 4) & 0x0f0f0f0fu,
+                       bv.x, bv.y);
+    mma_i8<true, ASYM>(acc, a.y & 0x0f0f0f0fu, b.y & 0x0f0f0f0fu, (a.y >> 4) & 0x0f0f0f0fu, (b.y >> 4) & 0x0f0f0f0fu,
+                       bv.z, bv.w);
+  };
+
+  if constexpr (TILED) {
+    // The loads of U K blocks are in flight together: a trip to memory per block is most of a block's time (28672 x
+    // 4096, one token: 26.6 us a block at a time, 16.7 with two, 18.8 with four and 128 registers).
+    constexpr int U = 2;
+    for (int blk0 = warp; blk0 < p.kc; blk0 += kI8Warps * U) {
+      uint2 a[U][2], b[U][2];
+      uint4 bv[U][2];
+      float s0[U], s1[U];
+      uint32_t z0[U], z1[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int blk = min(blk0 + u * kI8Warps, p.kc - 1);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          // [K block][quarter of 32 k][row][16 bytes]: this lane's two words of a quarter
+          const size_t off = (static_cast<size_t>(blk) * 4 + h * 2 + (t >> 1)) * (kTcTileN * 16) + (t & 1) * 8;
+          a[u][h] = *reinterpret_cast<const uint2*>(w0 + off);
+          b[u][h] = *reinterpret_cast<const uint2*>(w1 + off);
+          bv[u][h] = *reinterpret_cast<const uint4*>(qb + blk * 128 + h * 64 + 16 * t);
+        }
+        const size_t i0 = (tile * p.groups + (p.group >= p.k ? 0 : blk * 128 / p.group)) * kTcTileN + in0;
+        const size_t i1 = i0 + (in1 - in0);
+        s0[u] = p.sw[i0];
+        s1[u] = p.sw[i1];
+        z0[u] = p.zw[i0];
+        z1[u] = p.zw[i1];
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int blk = blk0 + u * kI8Warps;
+        if (blk >= p.kc) break;
+        int acc[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) mma_w4(acc, a[u][h], b[u][h], bv[u][h]);
+        drain(blk, acc, s0[u], s1[u], static_cast<int>(z0[u] & 0xffu), static_cast<int>(z1[u] & 0xffu));
+      }
+    }
+  } else {
+    for (int blk = warp; blk < p.kc; blk += kI8Warps) {
+      int acc[4] = {0, 0, 0, 0};
+      const int k0 = blk * p.kb;
+      for (int kk = 0; kk < p.kb; kk += 64) {
+        const int kq = k0 + kk + 16 * t;  // this lane's 16 k of the 64
+        const uint4 bv = *reinterpret_cast<const uint4*>(qb + kq);
+        if (W4) {
+          mma_w4(acc, *reinterpret_cast<const uint2*>(w0 + (kq >> 1)), *reinterpret_cast<const uint2*>(w1 + (kq >> 1)), bv);
+        } else {
+          const uint4 a = *reinterpret_cast<const uint4*>(w0 + kq);
+          const uint4 b = *reinterpret_cast<const uint4*>(w1 + kq);
+          mma_i8<false, ASYM>(acc, a.x, b.x, a.y, b.y, bv.x, bv.y);
+          mma_i8<false, ASYM>(acc, a.z, b.z, a.w, b.w, bv.z, bv.w);
+        }
+      }
+      const int grp = p.group >= p.k ? 0 : k0 / p.group;
+      const size_t i0 = static_cast<size_t>(r0) * p.groups + grp, i1 = static_cast<size_t>(r1) * p.groups + grp;
+      drain(blk, acc, p.sw[i0], p.sw[i1], static_cast<int>(p.zpw ? p.zpw[i0] : p.default_zp),
+            static_cast<int>(p.zpw ? p.zpw[i1] : p.default_zp));
+    }
   }
   red[warp][g][2 * t] = c[0];
   red[warp][g][2 * t + 1] = c[1];
@@ -503,6 +555,7 @@ cudaError_t launch_weight_block_sum(const uint8_t* w, const float* zpw, int n, i
 
 cudaError_t launch_i8_block(const I8BlockParams& p, cudaStream_t stream) {
   if (p.m > 16) {
+    if (p.zw) return cudaErrorInvalidValue;
     // 64 rows x 64 tokens per CTA
     const dim3 wgrid(static_cast<unsigned>((p.n + 63) / 64), static_cast<unsigned>((p.m + kWideTok - 1) / kWideTok));
     if (wgrid.y > 65535) return cudaErrorInvalidConfiguration;
@@ -520,8 +573,9 @@ cudaError_t launch_i8_block(const I8BlockParams& p, cudaStream_t stream) {
     return cudaGetLastError();
   }
   const dim3 grid(static_cast<unsigned>((p.n + 15) / 16), static_cast<unsigned>((p.m + 7) / 8));
-  if (grid.y > 65535) return cudaErrorInvalidConfiguration;
-  if (p.w4) {
+  if (p.zw) {
+    woq_i8_block_kernel<true, false, true><<<grid, kI8Warps * 32, 0, stream>>>(p);
+  } else if (p.w4) {
     if (p.asym)
       woq_i8_block_kernel<true, true><<<grid, kI8Warps * 32, 0, stream>>>(p);
     else

@@ -244,6 +244,7 @@ struct I8BlockParams {
   const uint8_t* w;      // plain [n][k/2] nibbles (w4) or [n][k] s8
   const float* sw;       // [n][groups] weight scales
   const float* zpw;      // [n][groups] weight zero points or null (default_zp)
+  const uint32_t* zw;    // not null: w, sw and zw in the layout of I8BlockTcParams, natural code order, m <= 16
   const int32_t* comp;   // [n][kc] sums of (qw - zp_w) per K block (asymmetric activations)
   const uint8_t* qa;     // [m][k] activation codes (w4: even / odd interleaved inside every 8)
   const float* sa;       // [m][kc]
@@ -289,7 +290,9 @@ int i8_block_tc_columns(int64_t m);
 size_t i8_block_tc_partial_bytes(int num_sms, int part_tok);
 cudaError_t launch_i8_block_tc(I8BlockTcParams p, const CUtensorMap& qamap, int num_sms, cudaStream_t stream);
 cudaError_t launch_act_block128_quant(const __nv_bfloat16* x, int64_t ldx, int m, int kc, uint8_t* qa, float* sa,
-                                      int32_t* zpa, float* sat, int n_tok, cudaStream_t stream);
+                                      int32_t* zpa, int32_t* sumqa, float* sat, int n_tok, cudaStream_t stream);
+// whether a call of m tokens on n x (kc * 128) weights runs on woq_i8_block_kernel instead
+bool i8_block_tc_few_tokens(int64_t m, int64_t n, int kc);
 cudaError_t launch_transpose_scales(const float* sa, int m, int kc, float* sat, int n_tok, cudaStream_t stream);
 cudaError_t launch_btc_pack(const uint8_t* plain, uint8_t* packed, int n, int k, cudaStream_t stream);
 cudaError_t launch_btc_unpack(const uint8_t* packed, uint8_t* plain, int n, int k, cudaStream_t stream);

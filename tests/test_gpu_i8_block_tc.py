@@ -50,6 +50,32 @@ def test_tile_edges(capi, m, n, k, g, mode):
     assert mx <= O.MAX_ABS_TOL and mr < 2e-4, (mx, mr)
 
 
+@pytest.mark.parametrize("m", [1, 7, 8, 9, 16, 17])
+@pytest.mark.parametrize("n,k,g,mode", [(331, 640, 128, 7), (331, 1152, 128, 7), (200, 4096, 256, 4), (137, 8320, -1, 7)])
+def test_few_tokens(capi, m, n, k, g, mode):
+    """Both sides of the line between the kernel of few tokens and the tcgen05 kernel, on one layout; numbers of K
+    blocks that are no multiple of the eight its warps take at a time, rows that fill no tile."""
+    test_tile_edges(capi, m, n, k, g, mode)
+
+
+@pytest.mark.parametrize("m", [8, 9])
+def test_few_tokens_on_large_weights(capi, m):
+    """9 tokens on more than 64 MB of weights are the tcgen05 kernel's; the results of the same rows agree."""
+    n, k = 28800, 4736
+    gen = torch.Generator(device="cuda").manual_seed(0)
+    qw = torch.randint(0, 256, (n, k // 2), dtype=torch.uint8, device="cuda", generator=gen)
+    s = torch.rand((n, k // 128), device="cuda", generator=gen) * 0.004 + 0.001
+    z = torch.randint(0, 128, (n, k // 128), device="cuda", generator=gen).float()
+    make = lambda rows: capi.WoqContext(qw[rows].contiguous(), s[rows].contiguous(), z[rows].contiguous(), None,  # noqa: E731
+                                        len(range(n)[rows]), k, O.WOQ_DTYPE_INT4, 128, capi.LOWP_INT8, act_quant_mode=7)
+    whole, part = make(slice(0, n)), make(slice(n - 300, n))
+    x = bf16_tensor(make_acts(m, k, seed=m), "cuda")
+    assert torch.equal(whole.int8_block_internals(x)[3][:, :, n - 300:], part.int8_block_internals(x)[3])
+    mx, mr = O.parity_metrics(bf16_numpy(whole.linear(x))[:, n - 300:], bf16_numpy(part.linear(x)))
+    # the same block accumulators; another order of the fp32 sum over 37 blocks
+    assert mx <= O.MAX_ABS_TOL and mr < 2e-4, (mx, mr)
+
+
 @pytest.mark.parametrize("m", [9, 70])
 def test_zero_points_out_of_range_stay_on_the_other_kernels(capi, m):
     n, k = 96, 512
