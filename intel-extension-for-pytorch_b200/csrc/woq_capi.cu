@@ -1061,22 +1061,26 @@ int run_i8block_tc(const woq_b200_ctx* c, const I8BlockWs& L, const __nv_bfloat1
   float* sa = reinterpret_cast<float*>(w8 + L.sa);
   int32_t* zpa = reinterpret_cast<int32_t*>(w8 + L.zpa);
   float* sat = reinterpret_cast<float*>(w8 + L.sat);
+  const bool few_tokens = woq::i8_block_tc_few_tokens(m, c->desc.n, c->kc);
   if (mode == WOQ_B200_ACT_PER_M_K_BLOCK_SYM) {
     CUDA_TRY(woq::launch_act_block128_quant(x, ldx, (int)m, c->kc, w8 + L.qa, sa, zpa,
-                                             reinterpret_cast<int32_t*>(w8 + L.sumqa), sat, L.n_tok, stream));
+                                             few_tokens ? reinterpret_cast<int32_t*>(w8 + L.sumqa) : nullptr, sat,
+                                             L.n_tok, stream));
   } else {
     CUDA_TRY(woq::launch_act_block_quant(x, ldx, (int)m, (int)c->desc.k, 128, mode, 0, w8 + L.qa, sa, zpa,
                                          reinterpret_cast<int32_t*>(w8 + L.sumqa), reinterpret_cast<float*>(w8 + L.range),
                                          reinterpret_cast<float*>(w8 + L.folded), stream));
-    CUDA_TRY(woq::launch_transpose_scales(sa, (int)m, c->kc, sat, L.n_tok, stream));
-    woq::count_launch();
+    if (!few_tokens) {
+      CUDA_TRY(woq::launch_transpose_scales(sa, (int)m, c->kc, sat, L.n_tok, stream));
+      woq::count_launch();
+    }
   }
   woq::count_launch();
   const size_t mk = static_cast<size_t>(m) * c->kc;
   if (sa_out) CUDA_TRY(cudaMemcpyAsync(sa_out, sa, mk * 4, cudaMemcpyDeviceToDevice, stream));
   if (zpa_out) CUDA_TRY(cudaMemcpyAsync(zpa_out, zpa, mk * 4, cudaMemcpyDeviceToDevice, stream));
   if (!y && !acc_out) return WOQ_B200_OK;
-  if (woq::i8_block_tc_few_tokens(m, c->desc.n, c->kc)) {
+  if (few_tokens) {
     woq::I8BlockParams q{};
     q.w = c->wq_tc;
     q.sw = c->btc_sw;

@@ -3,7 +3,7 @@
 // (csrc/cpu/aten/utils/woq.h:962-1126), the sum as int32 by tcgen05.mma kind::i8, exact.
 //
 // A CTA owns 128 output rows x up to 128 tokens of a share of the (row tile, token tile, K block) sequence
-// (equal contiguous shares; tiles that several CTAs share are summed in k order through the workspace by
+// (equal contiguous shares, or whole tiles where that is quicker; tiles that several CTAs share are summed in k order through the workspace by
 // whoever arrives last, so nobody waits and the order does not depend on timing).
 //
 //   warp 0       producer: packed weights + zero points, two K blocks per stage
@@ -466,11 +466,13 @@ __global__ void __launch_bounds__(256) act_block128_quant_kernel(const __nv_bflo
     word |= (static_cast<uint32_t>(static_cast<int>(q)) & 0xffu) << (8 * e);
   }
   reinterpret_cast<uint32_t*>(qa + static_cast<size_t>(tok) * kc * 128 + c * 128)[lane] = word;
-  sum = __reduce_add_sync(0xffffffffu, sum);
+  if (sumqa) {  // (for the kernel of few tokens)
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) sumqa[item] = sum;
+  }
   if (lane == 0) {
     sa[item] = scale;
     zpa[item] = 0;
-    sumqa[item] = sum;
     sat[(static_cast<size_t>(tok / n_tok) * kc + c) * n_tok + tok % n_tok] = scale;
   }
 }
@@ -570,8 +572,17 @@ cudaError_t launch_i8_block_tc(I8BlockTcParams p, const CUtensorMap& qamap, int 
   if (p.w_ring < 2) return cudaErrorInvalidConfiguration;
   const size_t smem = fixed + static_cast<size_t>(p.w_ring) * kWStage;
   const int64_t total = static_cast<int64_t>(p.tiles) * p.tok_tiles * p.kc;
-  // shares in whole stages where they are long enough for the rounding not to matter
-  p.unit = p.kc % 2 == 0 && total >= static_cast<int64_t>(num_sms) * 16 ? 2 : 1;
+  // Shares in whole stages where they are long enough for the rounding not to matter, or whole tiles: the parts of a
+  // shared tile are added one after another and behind its last K block.  In us, for c = columns / 32: a K block 0.54 +
+  // 0.085 c, a tile's end 3 c, a shared tile's 5.2 c + 0.31 c for each part (fitted to 512 x 512 .. 4096 x 4096).
+  // Shared / whole: 512 x 512, 128 tokens 29.2 / 18.7, 1024 x 2048, 128 tokens 46.0 / 28.8, 4096 x 4096, 512 tokens
+  // 56.3 / 47.5, but 1024 x 4096, 33 tokens 26.4 / 30.4.
+  const int64_t items = static_cast<int64_t>(p.tiles) * p.tok_tiles, ctas = total < num_sms ? total : num_sms;
+  const int64_t parts = items >= ctas ? 2 : ceil_div(ctas, items) + 1;
+  const double c = p.n_tok / 32, step = 0.54 + 0.085 * c;
+  const double shares = step * ceil_div(total, ctas) + c * (5.2 + 0.31 * (parts < p.kc ? parts : p.kc));
+  const double whole = step * p.kc * ceil_div(items, num_sms) + 3 * c;
+  p.unit = whole <= shares ? p.kc : p.kc % 2 == 0 && total >= static_cast<int64_t>(num_sms) * 16 ? 2 : 1;
   void (*kern)(const I8BlockTcParams, const CUtensorMap) = nullptr;
   switch (p.n_tok) {
     case 32: kern = woq_i8_block_tc_kernel<1>; break;
@@ -582,7 +593,8 @@ cudaError_t launch_i8_block_tc(I8BlockTcParams p, const CUtensorMap& qamap, int 
   cudaError_t e = allow_max_smem(kern);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(total < num_sms ? total : num_sms));
+  const int64_t units = total / p.unit;
+  cfg.gridDim = dim3(static_cast<unsigned>(units < num_sms ? units : num_sms));
   cfg.blockDim = dim3(kBtcThreads);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;

@@ -283,7 +283,7 @@ struct I8BlockTcParams {
   int64_t ldy;
   int m, n, kc, groups, bpg;  // bpg: K blocks per weight group (a large number: one group)
   int n_tok, tok_tiles, tiles, part_tok;
-  int w_ring, unit;           // slots of the packed-weight ring; shares are multiples of `unit` K blocks
+  int w_ring, unit;           // slots of the packed-weight ring; shares are multiples of `unit` K blocks (kc: whole tiles)
   int fusion;
 };
 int i8_block_tc_columns(int64_t m);
