@@ -135,7 +135,8 @@ extern "C" {
  * columns per tile (a multiple of 32 up to 256; 0: chosen) and deals its tiles in a fixed way, where the library
  * otherwise chooses by its estimate of the time.  `cut`: 0 chosen (with `columns`: equal shares), 1 equal shares of the
  * k sequence (shared tiles are summed through the workspace), 2 whole tiles, 3 .. 5 clusters of 2 .. 4 pairs that
- * split k (K of at least four k steps per pair; a k step is 64, INT8 compute 128).  Results differ in the order of the
+ * split k (K of at least four k steps per pair; a k step is 64, INT8 compute 128).  The K-block kernel of INT4 weights
+ * with INT8 compute knows cuts 1 and 2 (columns 0).  Results differ in the order of the
  * fp32 sums only. */
 #define WOQ_B200_HINT_PAIR(columns, cut) (((columns) << 16) | ((cut) << 8))
 

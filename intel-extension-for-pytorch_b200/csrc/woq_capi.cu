@@ -1129,6 +1129,7 @@ int run_i8block_tc(const woq_b200_ctx* c, const I8BlockWs& L, const __nv_bfloat1
   p.bpg = c->g_group >= c->desc.k ? 1 << 30 : c->g_group / 128;
   p.n_tok = L.n_tok;
   p.tok_tiles = L.tok_tiles;
+  p.cut = (c->desc.kernel_hint >> 8) & 3;
   p.part_tok = L.part_tok;
   p.tiles = c->tiles_tc;
   p.fusion = fusion;

@@ -582,7 +582,7 @@ cudaError_t launch_i8_block_tc(I8BlockTcParams p, const CUtensorMap& qamap, int 
   const double c = p.n_tok / 32, step = 0.54 + 0.085 * c;
   const double shares = step * ceil_div(total, ctas) + c * (5.2 + 0.31 * (parts < p.kc ? parts : p.kc));
   const double whole = step * p.kc * ceil_div(items, num_sms) + 3 * c;
-  p.unit = whole <= shares ? p.kc : p.kc % 2 == 0 && total >= static_cast<int64_t>(num_sms) * 16 ? 2 : 1;
+  p.unit = (p.cut ? p.cut == 2 : whole <= shares) ? p.kc : p.kc % 2 == 0 && total >= static_cast<int64_t>(num_sms) * 16 ? 2 : 1;
   void (*kern)(const I8BlockTcParams, const CUtensorMap) = nullptr;
   switch (p.n_tok) {
     case 32: kern = woq_i8_block_tc_kernel<1>; break;

@@ -284,6 +284,7 @@ struct I8BlockTcParams {
   int m, n, kc, groups, bpg;  // bpg: K blocks per weight group (a large number: one group)
   int n_tok, tok_tiles, tiles, part_tok;
   int w_ring, unit;           // slots of the packed-weight ring; shares are multiples of `unit` K blocks (kc: whole tiles)
+  int cut;                    // 0: by estimate, 1: shares, 2: whole tiles
   int fusion;
 };
 int i8_block_tc_columns(int64_t m);

@@ -76,6 +76,38 @@ def test_few_tokens_on_large_weights(capi, m):
     assert mx <= O.MAX_ABS_TOL and mr < 2e-4, (mx, mr)
 
 
+@pytest.mark.parametrize("m", [20, 31, 33, 65, 129, 290])
+@pytest.mark.parametrize("n,k,g", [(331, 640, 128), (200, 1536, 256), (1152, 2304, -1), (129, 4224, 128)])
+def test_both_cuts(capi, m, n, k, g):
+    """Whole tiles, and shares of the K blocks whose tiles are summed through the workspace: the same accumulators,
+    outputs in another order of the fp32 sum; the counters are left at zero."""
+    rng = np.random.default_rng(n + k + m)
+    w = (rng.standard_normal((n, k)) * 0.02).astype(np.float32)
+    if g > 0:
+        qw, s, z = O.quantize_per_block(w, O.WOQ_DTYPE_INT4, g, False)
+    else:
+        qw, s, z = O.quantize_per_channel(w, O.WOQ_DTYPE_INT4, False)
+        s, z = s[:, None], z[:, None]
+    bias = np.linspace(-1, 1, n).astype(np.float32) if n % 2 else None
+    t = lambda a: None if a is None else torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    x = O.rne_bf16(make_acts(m, k, seed=m))
+    resid = make_acts(m, n, seed=m + 1)
+    xb, rb = bf16_tensor(x, "cuda"), bf16_tensor(resid, "cuda")
+    y_ref, blocks, *_ = O.woq_linear_int8_blocks(x, qw, O.WOQ_DTYPE_INT4, s, z, bias, g, 7, return_blocks=True)
+    y_ref = O.rne_bf16(y_ref + resid)
+    for cut in (capi.PAIR_CUT_SHARES, capi.PAIR_CUT_WHOLE):
+        ctx = capi.WoqContext(t(qw), t(s), t(z), t(bias), n, k, O.WOQ_DTYPE_INT4, g, capi.LOWP_INT8, act_quant_mode=7,
+                              kernel_hint=capi.HINT_PAIR(0, cut))
+        np.testing.assert_array_equal(ctx.int8_block_internals(xb)[3].cpu().numpy(), blocks)
+        first = ctx.linear(xb, capi.FUSE_ADD, [rb])
+        for _ in range(3):
+            assert torch.equal(ctx.linear(xb, capi.FUSE_ADD, [rb]), first)
+        ctx.workspace(m).status()
+        mx, mr = O.parity_metrics(bf16_numpy(first), y_ref)
+        # the operand's rounding after a sum that may round to the neighbouring bf16 value
+        assert mx <= O.MAX_ABS_TOL and mr < 4e-4, (cut, mx, mr)
+
+
 @pytest.mark.parametrize("m", [9, 70])
 def test_zero_points_out_of_range_stay_on_the_other_kernels(capi, m):
     n, k = 96, 512
